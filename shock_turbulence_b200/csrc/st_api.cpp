@@ -18,6 +18,15 @@ int fail(st_ctx *c, int code, const std::string &msg) {
     return code;
 }
 
+int sync_stream(st_ctx *c) {
+    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (c->wait_flag && *(volatile int *)c->wait_flag) {
+        *c->wait_flag = 0;
+        return fail(c, ST_E_CUDA, "a line kernel's wait for its tile ran out");
+    }
+    return ST_OK;
+}
+
 struct OomError : std::runtime_error {
     OomError() : std::runtime_error("device scratch allocation failed") {}
 };
@@ -95,7 +104,13 @@ class Args {
     // returns the device pointer to use for p (nf fields of N^3)
     double *map(const double *p, int nf, bool in, bool out) {
         for (auto &a : v_)
-            if (a.host == p) { a.in |= in; a.out |= out; return a.dev; }
+            if (a.host == p) {
+                if (in && !a.in && a.staged &&
+                    cudaMemcpyAsync(a.dev, p, bytes(a.nf), cudaMemcpyDefault, c_->stream) != cudaSuccess)
+                    err_ = true;
+                a.in |= in; a.out |= out;
+                return a.dev;
+            }
         Arg a{p, nullptr, nf, in, out, false};
         cudaPointerAttributes at{};
         bool dev = false;
@@ -103,12 +118,15 @@ class Args {
             (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged))
             dev = at.device == c_->dev;
         cudaGetLastError();
-        if (dev) {
+        // device fields are used in place where the kernels' 16-byte transfers
+        // can reach them, and copied otherwise (a field that starts at an odd
+        // element of another array)
+        if (dev && !(reinterpret_cast<uintptr_t>(p) & 15)) {
             a.dev = const_cast<double *>(p);
         } else {
             a.dev = scratch(c_, nf);
             a.staged = true;
-            if (in && cudaMemcpyAsync(a.dev, p, bytes(nf), cudaMemcpyHostToDevice, c_->stream) != cudaSuccess)
+            if (in && cudaMemcpyAsync(a.dev, p, bytes(nf), cudaMemcpyDefault, c_->stream) != cudaSuccess)
                 err_ = true;
         }
         v_.push_back(a);
@@ -118,13 +136,11 @@ class Args {
     int finish() {
         for (auto &a : v_)
             if (a.staged && a.out)
-                if (cudaMemcpyAsync(const_cast<double *>(a.host), a.dev, bytes(a.nf), cudaMemcpyDeviceToHost,
+                if (cudaMemcpyAsync(const_cast<double *>(a.host), a.dev, bytes(a.nf), cudaMemcpyDefault,
                                     c_->stream) != cudaSuccess)
                     err_ = true;
-        cudaError_t e = cudaStreamSynchronize(c_->stream);
-        if (err_ || e != cudaSuccess)
-            return fail(c_, ST_E_CUDA, std::string("argument transfer: ") + cudaGetErrorString(
-                                                                                 e != cudaSuccess ? e : cudaErrorInvalidValue));
+        ST_TRY(sync_stream(c_));
+        if (err_) return fail(c_, ST_E_CUDA, std::string("argument transfer: ") + cudaGetErrorString(cudaErrorInvalidValue));
         return ST_OK;
     }
 
@@ -296,9 +312,13 @@ int st_create_batch(const st_params *p, int ncase, st_ctx **out) {
     c->dm.n3 = (size_t)p->nx * p->ny * p->nz;
     c->nb = c->na = ncase;
     c->fs = (size_t)ncase * c->dm.n3;
-    for (int d = 0; d < 3; d++) c->seg[d] = choose_seg(n[d]);
+    for (int d = 0; d < 3; d++) { c->seg[d] = choose_seg(n[d]); c->segf[d] = choose_seg_f(n[d]); }
     auto bail = [&](int code, const char *m) { c->err = m; st_destroy(c); return code; };
     if (cudaSetDevice(c->dev) != cudaSuccess) return bail(ST_E_CUDA, "cudaSetDevice");
+    if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c->smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c->smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev) != cudaSuccess)
+        return bail(ST_E_CUDA, "device attributes");
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(ST_E_CUDA, "cudaStreamCreate");
     c->stream = c->own_stream;
@@ -346,7 +366,12 @@ int st_create_batch(const st_params *p, int ncase, st_ctx **out) {
     }
     const size_t sb = (size_t)ncase * kScal * sizeof(double);
     ok = ok && cudaMalloc((void **)&c->dscal, sb) == cudaSuccess && cudaMemset(c->dscal, 0, sb) == cudaSuccess &&
-         cudaMallocHost((void **)&c->hpinned, sb) == cudaSuccess;
+         cudaMallocHost((void **)&c->hpinned, sb + sizeof(double)) == cudaSuccess;
+    if (ok) {   // behind the scalars' mirror
+        c->wait_flag = reinterpret_cast<int *>(c->hpinned + (size_t)ncase * kScal);
+        *c->wait_flag = 0;
+        ok = cudaHostGetDevicePointer((void **)&c->wait_flag_dev, c->wait_flag, 0) == cudaSuccess;
+    }
     if (!ok) { cudaGetLastError(); return bail(ST_E_NOMEM, "device allocation of the COMMON blocks failed"); }
     if (p->family == ST_FAMILY_PERIODIC) {
         if (dev_fill(c, c->gamma_eff, c->fs, p->gamma1) != ST_OK || dev_fill(c, c->Y, c->fs, 1.0) != ST_OK ||
@@ -385,7 +410,7 @@ int st_destroy(st_ctx *c) {
 
 int st_sync(st_ctx *c) {
     API_BEGIN(c)
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -410,7 +435,7 @@ int st_set_state(st_ctx *c, const double *Q, const double *Y) {
     }
     ST_CUDA(c, cudaMemsetAsync(c->rYW, 0, b, c->stream));
     ST_CUDA(c, cudaMemsetAsync(c->dscal + 7, 0, sizeof(double), c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -421,7 +446,7 @@ int st_get_state(st_ctx *c, double *Q, double *Y) {
     const size_t b = c->dm.n3 * 8;
     if (Q) ST_CUDA(c, cudaMemcpyAsync(Q, c->Q, 5 * b, cudaMemcpyDefault, c->stream));
     if (Y) ST_CUDA(c, cudaMemcpyAsync(Y, c->Y, b, cudaMemcpyDefault, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -432,7 +457,7 @@ int st_set_tstep(st_ctx *c, double t) {
     c->Tstep = t;
     c->hpinned[6] = t;
     ST_CUDA(c, cudaMemcpyAsync(c->dscal + 6, c->hpinned + 6, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -442,7 +467,7 @@ int st_get_tstep(st_ctx *c, double *t) {
     if (!t) return ST_E_ARG;
     API_BEGIN(c)
     ST_CUDA(c, cudaMemcpyAsync(c->hpinned + 6, c->dscal + 6, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     c->Tstep = c->hpinned[6];
     *t = c->Tstep;
     return ST_OK;
@@ -479,11 +504,11 @@ int st_get_common(st_ctx *c, const char *name, double *out) {
         Scratch t(c, nf);
         ST_TRY(dev_to_double(c, pf, t, nf * c->dm.n3));
         ST_CUDA(c, cudaMemcpyAsync(out, t, nf * c->dm.n3 * 8, cudaMemcpyDefault, c->stream));
-        ST_CUDA(c, cudaStreamSynchronize(c->stream));
+        ST_TRY(sync_stream(c));
         return ST_OK;
     }
     ST_CUDA(c, cudaMemcpyAsync(out, p, nf * c->dm.n3 * 8, cudaMemcpyDefault, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -500,11 +525,11 @@ int st_set_common(st_ctx *c, const char *name, const double *in) {
         Scratch t(c, nf);
         ST_CUDA(c, cudaMemcpyAsync(t, in, nf * c->dm.n3 * 8, cudaMemcpyDefault, c->stream));
         ST_TRY(dev_to_float(c, t, pf, nf * c->dm.n3));
-        ST_CUDA(c, cudaStreamSynchronize(c->stream));
+        ST_TRY(sync_stream(c));
         return ST_OK;
     }
     ST_CUDA(c, cudaMemcpyAsync(p, in, nf * c->dm.n3 * 8, cudaMemcpyDefault, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -831,7 +856,7 @@ int st_compute_tstep(st_ctx *c, const double *Q, const double *Y, double cfl_res
 // ---- time integration ------------------------------------------------------------
 static int read_time(st_ctx *c, double *time) {
     ST_CUDA(c, cudaMemcpyAsync(c->hpinned + 7, c->dscal + 7, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     if (time) *time = c->hpinned[7];
     return ST_OK;
 }
@@ -955,7 +980,7 @@ int st_case_start(st_ctx *c, int k, const double *Q, const double *Y, double tim
     // the set-up before the main loop, src/main_mf.f:100-101 (src/main.f:100)
     if (c->p.family != ST_FAMILY_PERIODIC) ST_TRY(dev_compute_gamma(c, c->Y));
     ST_TRY(dev_compute_hyper(c, c->Q, c->Y));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -971,7 +996,7 @@ int st_case_get(st_ctx *c, int k, double *Q, double *Y, double *time, int *step)
     if (Y) ST_CUDA(c, cudaMemcpyAsync(Y, c->Y + off, b, cudaMemcpyDefault, c->stream));
     ST_CUDA(c, cudaMemcpyAsync(c->hpinned, c->dscal + (size_t)k * kScal, kScal * sizeof(double),
                                cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     if (time) *time = c->hpinned[SC_TIME];
     if (step) *step = (int)c->hpinned[SC_STEP];
     return ST_OK;
@@ -1001,7 +1026,7 @@ int st_case_move(st_ctx *c, int src, int dst) {
     for (int h = 0; h < 4; h++) { ST_TRY(mv(c->hyp[h], 1)); ST_TRY(mv(c->hypf[h], 1)); }
     ST_CUDA(c, cudaMemcpyAsync(c->dscal + (size_t)dst * kScal, c->dscal + (size_t)src * kScal,
                                kScal * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -1049,7 +1074,7 @@ int st_set_time(st_ctx *c, double time) {
     API_BEGIN(c)
     c->hpinned[7] = time;
     ST_CUDA(c, cudaMemcpyAsync(c->dscal + 7, c->hpinned + 7, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     return ST_OK;
     API_END(c)
 }
@@ -1077,7 +1102,7 @@ int st_query(st_ctx *c) {
 
 int st_set_stream(st_ctx *c, void *stream) {
     API_BEGIN(c)
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     c->stream = stream ? (cudaStream_t)stream : c->own_stream;
     return ST_OK;
     API_END(c)
@@ -1104,7 +1129,7 @@ int st_launch_count(st_ctx *c, long long *count) {
 int st_profile_report(st_ctx *c, char *buf, int buflen) {
     if (!buf || buflen < 3) return ST_E_ARG;
     API_BEGIN(c)
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     struct Agg { long long n = 0; double ms = 0, bytes = 0; };
     std::vector<std::pair<std::string, Agg>> agg;
     for (auto &r : c->prec) {
@@ -1228,7 +1253,7 @@ int st_get_monitors(st_ctx *c, double out[10]) {
     API_BEGIN(c)
     ST_TRY(dev_monitors(c));
     ST_CUDA(c, cudaMemcpyAsync(c->hpinned, c->dscal, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     std::memcpy(out, c->mon, 8 * sizeof(double));
     out[8] = c->hpinned[1];
     out[9] = c->hpinned[6];

@@ -224,7 +224,7 @@ __global__ void k_shock(const double *b, double thr, Grid g, int My, int Mz, siz
 int fetch_sums(st_ctx *c, const double *part, int nv, double *out) {
     std::vector<double> h((size_t)nv * kRG);
     ST_CUDA(c, cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     for (int v = 0; v < nv; v++) {
         double s = 0.0;
         for (int b = 0; b < kRG; b++) s += h[(size_t)v * kRG + b];
@@ -235,7 +235,7 @@ int fetch_sums(st_ctx *c, const double *part, int nv, double *out) {
 int fetch_max(st_ctx *c, const double *part, double *out) {
     std::vector<double> h(kRG);
     ST_CUDA(c, cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     double m = -INFINITY;
     for (double v : h) m = std::fmax(m, v);
     *out = m;
@@ -323,7 +323,7 @@ int dev_compute_srm_stats(st_ctx *c, double *hmix, double *tke_total, double *ur
     std::vector<unsigned long long> hcnt(na);
     ST_CUDA(c, cudaMemcpyAsync(hsum.data(), d_sum, 2 * na * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     ST_CUDA(c, cudaMemcpyAsync(hcnt.data(), d_cnt, na * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     std::vector<double> ura(na), ya(na);
     for (int M = 0; M < na; M++) {
         ura[M] = hsum[M] / (double)hcnt[M];

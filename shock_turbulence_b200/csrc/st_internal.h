@@ -14,16 +14,16 @@
 
 namespace st {
 
-constexpr int kMaxSeg = 32;       // max segments per line (warps per CTA)
-constexpr int kLanes = 16;        // lines per CTA (half a warp; a warp holds two segments)
+constexpr int kMaxSeg = 32;       // max segments per line
+constexpr int kLanes = 16;        // columns of a line-kernel CTA (half a warp; a warp holds two segments)
 constexpr int kLineThreads = kLanes * kMaxSeg;     // threads of a line-kernel CTA at most
-constexpr int kLineCtasPerSm = 32 / kLanes;        // resident CTAs per SM at 64 registers a thread
-constexpr int kScanSteps = 5;     // log2(kMaxSeg): steps of a scan over the segments
+constexpr int kMaxRows = 16;      // max rows per segment
 
-// A line of n rows is split into P = n/S segments of S rows; thread t of a CTA
-// works on line t%16 and segment t/16 of 16 neighbouring lines, so a warp
-// holds two adjacent segments of the same 16 lines.  Supported S.
+// A line of n rows is split into P = n/S <= kMaxSeg segments of S rows (8 or
+// 16); 0 where n has no such split.
 int choose_seg(int n);
+// the same for the FP32 mode's float solves (2, 3, 4, 6, 8, 12 or 16 rows)
+int choose_seg_f(int n);
 
 // Row tables of a constant-coefficient tridiagonal system, factorised as the
 // reference's tridiagonal_serial does (src/tridiagonal.f90:264-287), plus the
@@ -43,11 +43,15 @@ struct TriTabT {
     // Away from the line ends the factorisation reaches a fixed point: in
     // segments slo <= s < shi every row's l, up, id equal (bitwise) cl, cup,
     // cid, which the solve then keeps in registers instead of loading per row.
+    // The carry responses g and h of such a segment's rows are cg and ch.
     int slo, shi;
     A cl, cup, cid;
-    // scan factors [kScanSteps][kMaxSeg]: sf[k][s] = B_s B_{s-1} ... B_{s-2^k+1}
-    // (B_s: response of segment s's last forward value to its carry-in) and
-    // sb[k][s] = G_s ... G_{s+2^k-1} (G_s: of its first backward value)
+    A cg[kMaxRows], ch[kMaxRows];
+    int clo, chi;  // segments clo <= s < chi need no corner correction
+    // float solves: scan factors [5][kMaxSeg], sf[k][s] = B_s B_{s-1} ...
+    // B_{s-2^k+1} (B_s: response of segment s's last forward value to its
+    // carry-in) and sb[k][s] = G_s ... G_{s+2^k-1} (G_s: of its first backward
+    // value)
     const A *sf, *sb;
 };
 using TriTab = TriTabT<double>;
@@ -63,14 +67,17 @@ struct PenTab {
     const double *h1, *h2;   // backward carry responses (carry = (x_{b+1}, x_{b+2}))
     const double *cyc;       // periodic family: [n][4] corner correction, else null
     // segments slo <= s < shi: every row's p1, p2, q1, q2, id equal (bitwise)
-    // the constants below (the factorisation's interior fixed point)
+    // the constants below (the factorisation's interior fixed point), and the
+    // carry responses of the rows are cg1, cg2, ch1, ch2
     int slo, shi;
     double cp1, cp2, cq1, cq2, cid;
-    // Scan factors [kScanSteps][kMaxSeg][4]: products of 2^k consecutive
-    // segment transfer matrices, sf[k][s] = M_s M_{s-1} ... M_{s-2^k+1}
-    // (M_s: response of segment s's last two forward values to its carry-in)
-    // and sb[k][s] = N_s ... N_{s+2^k-1} (N_s: of its first two backward values)
+    double cg1[kMaxRows], cg2[kMaxRows], ch1[kMaxRows], ch2[kMaxRows];
+    int clo, chi;            // segments clo <= s < chi need no corner correction
+    // segment transfer matrices [P][4]: sf[s] the response of segment s's last
+    // two forward values to its carry-in, sb[s] of its first two backward
+    // ones; FP32 mode: [5][kMaxSeg][4], the products of 2^k consecutive ones
     const double *sf, *sb;
+    double cm[4], cn[4];     // of the segments slo <= s < shi
 };
 
 enum TriKind { K_D1S = 0, K_D1A = 1, K_D2S = 2, K_D2A = 3 };
@@ -94,6 +101,7 @@ enum ProdOp {
     PR_MULMUL,       // c*(a*b)
     PR_SPEC,         // a*b*c + a*c*k0*k1             (Species_RHS flux)
     PR_SPECT,        // (k0*d)*(a*b*c + a*c*k0b*k1)    (its energy counterpart)
+    PR_HMULADD,      // a*b/2 + c        (half a momentum flux plus the pressure: one derivative for both)
 };
 template <class T>
 struct ProdT {
@@ -130,7 +138,9 @@ struct st_ctx {
     size_t fs = 0;     // field stride: nb * dm.n3
     size_t ncell() const { return (size_t)na * dm.n3; }   // cells the kernels process
     int seg[3];        // rows per segment along x, y, z
+    int segf[3];       // of the float solves
     int dev = 0;
+    int sms = 0, smem_sm = 0, smem_cta = 0;   // SMs; shared memory of an SM and of a CTA at most
     cudaStream_t stream = nullptr;
     std::string err;
     // derived scalars
@@ -168,6 +178,9 @@ struct st_ctx {
     // device scalars (reductions, dt)
     double *dscal = nullptr;     // [nb][kScal]
     double *hpinned = nullptr;   // pinned host mirror [nb][kScal]
+    // set by a line kernel whose wait for a tile ran out (mapped host memory,
+    // read at the synchronising calls)
+    int *wait_flag = nullptr, *wait_flag_dev = nullptr;
     // host<->device staging for the per-operator entry points
     std::vector<double *> stage;
     cudaStream_t own_stream = nullptr;
@@ -200,6 +213,9 @@ int fail(st_ctx *c, int code, const std::string &msg);
         int r_ = (expr);             \
         if (r_ != ST_OK) return r_;  \
     } while (0)
+
+// waits for the context's stream; an error if a line kernel gave up a wait
+int sync_stream(st_ctx *c);
 
 // launch instrumentation: every kernel launch is bracketed by these
 int prof_start(st_ctx *c, const char *name, double bytes);
@@ -262,13 +278,10 @@ int dev_dfd_f(st_ctx *c, int dir, int asym, const float *F, float *dF, int iadd,
 int dev_dfd_prod_f(st_ctx *c, int dir, int asym, const ProdF &F, float *dF, int iadd, double cadd);
 int dev_d2fd2_f(st_ctx *c, int dir, int asym, const float *F, float *dF, float *d2F, int iadd);
 int dev_gauss_f(st_ctx *c, int dir, const float *F, float *Fg);
-// last pass of a Laplacian: out = (derivative + E1) + E2 (x and z lines)
-int dev_dfd_sum(st_ctx *c, int dir, int asym, const double *F, double *dF, const double *E1, const double *E2);
-int dev_d2fd2_sum(st_ctx *c, int dir, int asym, const double *F, double *d2F, const double *E1,
-                  const double *E2);
-int dev_dfd_sum_f(st_ctx *c, int dir, int asym, const float *F, float *dF, const float *E1, const float *E2);
-int dev_d2fd2_sum_f(st_ctx *c, int dir, int asym, const float *F, float *d2F, const float *E1,
-                    const float *E2);
+// one direction of a Laplacian: out (=|+=) d(dF/ds)/ds (a symmetric field,
+// whose first derivative is antisymmetric) or, second, d2F/ds2
+int dev_lap(st_ctx *c, int dir, const double *F, double *out, int iadd, bool second);
+int dev_lap_f(st_ctx *c, int dir, const float *F, float *out, int iadd, bool second);
 int dev_d2fd2(st_ctx *c, int dir, int asym, const double *F, double *dF, double *d2F, int iadd);
 int dev_filter(st_ctx *c, int dir, int asym, const double *F, double *F0);
 int dev_gauss(st_ctx *c, int dir, const double *F, double *Fg);

@@ -1,216 +1,220 @@
 // st_kernels.cu - compact derivative, compact filter and Gaussian filter line
 // operators (bounded-line instantiations and the entry points of both
 // families), and the general (per-line coefficient) tri/pentadiagonal solvers.
+#include <initializer_list>
 #include "st_linekern.cuh"
 
 namespace st {
 
-static int launch_line(st_ctx *c, OpKind op, const LineArgs &a) {
-    return a.cyc ? launch_line_cyc(c, op, a) : launch_line_t<false, double>(c, op, a);
-}
-static int launch_line(st_ctx *c, OpKind op, const LineArgsF &a) {
-    return a.cyc ? launch_line_cyc_f32(c, op, a) : launch_line_f32(c, op, a);
+int launch_rec(st_ctx *c, RecId id, LineArgs &a, const double *const *in, double *const *out) {
+    return launch_rec_t<false, double>(c, id, a, in, out);
 }
 
-template <class T = double>
-static LineArgsT<T> make_args(st_ctx *c, int dir) {
-    LineArgsT<T> a{};
-    a.geo.dir = dir;
-    a.geo.n = c->dm.n[dir];
-    a.geo.My = c->dm.n[1];
-    a.geo.Mz = c->dm.n[2];
-    a.S = c->seg[dir];
-    a.P = a.geo.n / a.S;
-    a.K = c->k;
-    a.cyc = c->p.family == ST_FAMILY_PERIODIC;
-    return a;
+// the context's family and the field type pick the instantiation
+static int launch(st_ctx *c, RecId id, LineArgs &a, const double *const *in, double *const *out) {
+    return c->p.family == ST_FAMILY_PERIODIC ? launch_rec_cyc(c, id, a, in, out) : launch_rec(c, id, a, in, out);
+}
+static int launch(st_ctx *c, RecId id, LineArgsF &a, const float *const *in, float *const *out) {
+    return c->p.family == ST_FAMILY_PERIODIC ? launch_rec_cyc_f32(c, id, a, in, out) : launch_rec_f32(c, id, a, in, out);
 }
 
-static Prod plain(const double *F) {
-    Prod p{};
-    p.op = PR_A;
-    p.a = F;
-    return p;
+// cuTensorMapEncodeTiled through the runtime (the library does not link libcuda)
+typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (EncodeTiled)f;
+    }();
+    return fn;
 }
 
-int dev_dfd(st_ctx *c, int dir, int asym, const double *F, double *dF, int iadd, double cadd) {
-    return dev_dfd_prod(c, dir, asym, plain(F), dF, iadd, cadd);
-}
-
-int dev_dfd_prod(st_ctx *c, int dir, int asym, const Prod &F, double *dF, int iadd, double cadd) {
-    LineArgs a = make_args(c, dir);
-    a.F = F; a.O1 = dF; a.asym = asym; a.iadd = iadd;
-    a.fac1 = cadd * c->s1[dir] * (double)(a.geo.n - 1);           // src/derivCDopt6_sym_tri.f:424
-    a.t1 = c->tri[dir][asym ? K_D1A : K_D1S];
-    return launch_line(c, OP_D1, a);
-}
-
-int dev_d2fd2(st_ctx *c, int dir, int asym, const double *F, double *dF, double *d2F, int iadd) {
-    LineArgs a = make_args(c, dir);
-    a.F = plain(F); a.O1 = dF; a.O2 = d2F; a.asym = asym; a.iadd = iadd;
-    a.fac1 = 1.0 * c->s1[dir] * (double)(a.geo.n - 1);
-    a.fac2 = ((double)((a.geo.n - 1) * (a.geo.n - 1))) * c->s2[dir];   // src/derivCDopt6_sym_tri.f:554
-    a.t1 = c->tri[dir][asym ? K_D1A : K_D1S];
-    a.t2 = c->tri[dir][asym ? K_D2A : K_D2S];
-    return launch_line(c, OP_D2, a);
-}
-
-// The last pass of a Laplacian with the sum of the three directions fused into
-// its store: out = (d(F)/ds + E1) + E2 (first derivative, cadd = 1) or
-// (d2(F)/ds2 + E1) + E2; x and z lines only.
-int dev_dfd_sum(st_ctx *c, int dir, int asym, const double *F, double *dF, const double *E1, const double *E2) {
-    if (dir == 1) return fail(c, ST_E_ARG, "fused sum: x or z lines only");
-    LineArgs a = make_args(c, dir);
-    a.F = plain(F); a.O1 = dF; a.asym = asym; a.iadd = 0; a.E1 = E1; a.E2 = E2;
-    a.fac1 = 1.0 * c->s1[dir] * (double)(a.geo.n - 1);
-    a.t1 = c->tri[dir][asym ? K_D1A : K_D1S];
-    return launch_line(c, OP_D1, a);
-}
-
-int dev_d2fd2_sum(st_ctx *c, int dir, int asym, const double *F, double *d2F, const double *E1,
-                  const double *E2) {
-    if (dir == 1) return fail(c, ST_E_ARG, "fused sum: x or z lines only");
-    LineArgs a = make_args(c, dir);
-    a.F = plain(F); a.O2 = d2F; a.asym = asym; a.iadd = 0; a.E1 = E1; a.E2 = E2;
-    a.fac2 = ((double)((a.geo.n - 1) * (a.geo.n - 1))) * c->s2[dir];
-    a.t2 = c->tri[dir][asym ? K_D2A : K_D2S];
-    return launch_line(c, OP_D2, a);
-}
-
-int dev_filter(st_ctx *c, int dir, int asym, const double *F, double *F0) {
-    LineArgs a = make_args(c, dir);
-    a.F = plain(F); a.O1 = F0; a.asym = asym;
-    a.p = c->pen[dir][asym ? K_FA : K_FS];
-    return launch_line(c, OP_FILTER, a);
-}
-
-int dev_gauss(st_ctx *c, int dir, const double *F, double *Fg) {
-    LineArgs a = make_args(c, dir);
-    a.F = plain(F); a.O1 = Fg;
-    return launch_line(c, OP_GAUSS, a);
-}
-
-// ---- FP32 mode (float fields and arithmetic, two lines per thread) ----------
-static ProdF plain_f(const float *F) {
-    ProdF p{};
-    p.op = PR_A;
-    p.a = F;
-    return p;
-}
-
-// the kernels access a thread's two lines with one 8-byte load or store
-static int check_f2(st_ctx *c, const ProdF &F, const float *O1, const float *O2) {
-    const void *ptrs[6] = {F.a, F.b, F.c, F.d, O1, O2};
-    for (const void *p : ptrs)
-        if (reinterpret_cast<uintptr_t>(p) & 7)
-            return fail(c, ST_E_ARG, "FP32 line operators need 8-byte aligned fields");
+// Encoded anew for every launch (0.05 us on the host); L2 promotion to 256
+// bytes: neighbouring CTAs read the other half (2 % on x and z lines).
+int line_map(st_ctx *c, CUtensorMap *m, const void *p, bool f32, int dir, int nl, int box) {
+    const EncodeTiled enc = encode_tiled();
+    if (!enc) return fail(c, ST_E_CUDA, "cuTensorMapEncodeTiled is not available");
+    const cuuint64_t es = f32 ? 4 : 8, my = c->dm.n[1], mz = c->dm.n[2], mx = c->dm.n[0], na = (cuuint64_t)c->na;
+    cuuint64_t dims[4] = {my, mz, mx, na}, str[3] = {my * es, my * mz * es, (cuuint64_t)c->dm.n3 * es};
+    cuuint32_t b[4] = {(cuuint32_t)nl, dir == 0 ? 1u : (cuuint32_t)box, dir == 0 ? (cuuint32_t)box : 1u, 1u};
+    if (dir == 1) {   // the lines of all cases follow one another
+        const cuuint64_t rc = 128 / es, ch = my / rc;
+        dims[0] = rc; dims[1] = mz * mx * na; dims[2] = ch; dims[3] = 1;
+        str[1] = 128; str[2] = my * es * dims[1];
+        b[0] = (cuuint32_t)rc; b[1] = (cuuint32_t)nl; b[2] = (cuuint32_t)ch;
+    }
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    const CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void *>(p),
+                           dims, str, b, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           dir == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(c, ST_E_CUDA, "cuTensorMapEncodeTiled failed (field not 16-byte aligned?)");
     return ST_OK;
 }
 
-int dev_dfd_prod_f(st_ctx *c, int dir, int asym, const ProdF &F, float *dF, int iadd, double cadd) {
-    ST_TRY(check_f2(c, F, dF, nullptr));
-    LineArgsF a = make_args<float>(c, dir);
-    a.F = F; a.O1 = dF; a.asym = asym; a.iadd = iadd;
-    a.fac1 = cadd * c->s1[dir] * (double)(a.geo.n - 1);
-    a.t1 = c->trif[dir][asym ? K_D1A : K_D1S];
-    return launch_line(c, OP_D1, a);
+template <class T>
+static LineArgsT<T> make_args(st_ctx *c, int dir) {
+    LineArgsT<T> a{};
+    a.dir = dir;
+    a.n = c->dm.n[dir];
+    a.c = c->k;
+    return a;
+}
+template <class T>
+static const TriTabT<T> &tri_tab(st_ctx *c, int dir, int kind) {
+    if constexpr (sizeof(T) == 8) return c->tri[dir][kind];
+    else return c->trif[dir][kind];
+}
+// bulk copies and tensor maps need 16-byte aligned fields
+static int aligned(st_ctx *c, const void *p) {
+    if (reinterpret_cast<uintptr_t>(p) & 15) return fail(c, ST_E_ARG, "line operators need 16-byte aligned fields");
+    return ST_OK;
 }
 
-int dev_dfd_f(st_ctx *c, int dir, int asym, const float *F, float *dF, int iadd, double cadd) {
-    return dev_dfd_prod_f(c, dir, asym, plain_f(F), dF, iadd, cadd);
+// first-derivative arguments of operation k of a launch (its output, sign of
+// the symmetry, accumulation and factor), src/derivCDopt6_sym_tri.f:424
+template <class T>
+static void set_d1(st_ctx *c, LineArgsT<T> &a, int k, int asym, int iadd, double cadd) {
+    a.op[k].asym = asym;
+    a.op[k].fac1 = cadd * c->s1[a.dir] * (double)(a.n - 1);
+    a.op[k].t1 = tri_tab<T>(c, a.dir, asym ? K_D1A : K_D1S);
+    a.red[k] = iadd;
 }
+
+template <class T>
+static int dfd_t(st_ctx *c, int dir, int asym, const ProdT<T> &F, T *dF, int iadd, double cadd) {
+    static const RecId rec[] = {R_D1, R_MUL, R_ADDMUL, R_MULMUL, R_SPEC, R_SPECT, R_HMULADD};
+    static const int nin[] = {1, 2, 3, 3, 3, 4, 3};
+    LineArgsT<T> a = make_args<T>(c, dir);
+    set_d1(c, a, 0, asym, iadd, cadd);
+    a.k0 = F.k0; a.k1 = F.k1; a.k2 = F.k2;
+    // a*b/2 + c in the FP32 mode: the derivative of a*b with half the factor,
+    // plus that of c
+    if (F.op == PR_HMULADD && sizeof(T) == 4) { a.op[1] = a.op[0]; a.op[1].fac1 = 0.5 * a.op[0].fac1; }
+    const T *in[4] = {F.a, F.b, F.c, F.d};
+    for (int k = 0; k < nin[F.op]; k++) ST_TRY(aligned(c, in[k]));
+    ST_TRY(aligned(c, dF));
+    return launch(c, rec[F.op], a, in, &dF);
+}
+
+// D2F*2: d2F, and dF where given (iadd)
+template <class T>
+static int d2_t(st_ctx *c, int dir, int asym, const T *F, T *dF, T *d2F, int iadd, int red) {
+    LineArgsT<T> a = make_args<T>(c, dir);
+    a.op[0].asym = asym;
+    a.op[0].fac2 = ((double)((a.n - 1) * (a.n - 1))) * c->s2[dir];   // src/derivCDopt6_sym_tri.f:554
+    a.op[0].t2 = tri_tab<T>(c, dir, asym ? K_D2A : K_D2S);
+    a.red[0] = red;
+    ST_TRY(aligned(c, F)); ST_TRY(aligned(c, d2F));
+    if (iadd) { ST_TRY(aligned(c, dF)); set_d1(c, a, 1, asym, 0, 1.0); }
+    T *out[2] = {d2F, dF};
+    return launch(c, iadd ? R_D2D1 : R_D2, a, &F, out);
+}
+
+template <class T>
+static int lap_t(st_ctx *c, int dir, const T *F, T *out, int iadd, bool second) {
+    if (second) return d2_t<T>(c, dir, 0, F, (T *)nullptr, out, 0, iadd);
+    LineArgsT<T> a = make_args<T>(c, dir);
+    set_d1(c, a, 0, 0, iadd, 1.0);
+    a.op[0].t2 = tri_tab<T>(c, dir, K_D1A);
+    ST_TRY(aligned(c, F)); ST_TRY(aligned(c, out));
+    return launch(c, R_LAP, a, &F, &out);
+}
+
+template <class T>
+static int gauss_t(st_ctx *c, int dir, const T *F, T *Fg) {
+    LineArgsT<T> a = make_args<T>(c, dir);
+    ST_TRY(aligned(c, F)); ST_TRY(aligned(c, Fg));
+    return launch(c, R_GAUSS, a, &F, &Fg);
+}
+
+static Prod plain(const double *F) { Prod p{}; p.op = PR_A; p.a = F; return p; }
+static ProdF plain(const float *F) { ProdF p{}; p.op = PR_A; p.a = F; return p; }
+
+int dev_dfd(st_ctx *c, int dir, int asym, const double *F, double *dF, int iadd, double cadd) {
+    return dfd_t<double>(c, dir, asym, plain(F), dF, iadd, cadd);
+}
+int dev_dfd_prod(st_ctx *c, int dir, int asym, const Prod &F, double *dF, int iadd, double cadd) {
+    return dfd_t<double>(c, dir, asym, F, dF, iadd, cadd);
+}
+int dev_d2fd2(st_ctx *c, int dir, int asym, const double *F, double *dF, double *d2F, int iadd) {
+    return d2_t<double>(c, dir, asym, F, dF, d2F, iadd, 0);
+}
+int dev_lap(st_ctx *c, int dir, const double *F, double *out, int iadd, bool second) {
+    return lap_t<double>(c, dir, F, out, iadd, second);
+}
+int dev_filter(st_ctx *c, int dir, int asym, const double *F, double *F0) {
+    LineArgs a = make_args<double>(c, dir);
+    a.op[0].asym = asym;
+    a.p = c->pen[dir][asym ? K_FA : K_FS];
+    ST_TRY(aligned(c, F)); ST_TRY(aligned(c, F0));
+    return launch(c, R_FILTER, a, &F, &F0);
+}
+int dev_gauss(st_ctx *c, int dir, const double *F, double *Fg) { return gauss_t<double>(c, dir, F, Fg); }
+
+// FP32 mode (float fields and arithmetic, two lines per thread)
+int dev_dfd_f(st_ctx *c, int dir, int asym, const float *F, float *dF, int iadd, double cadd) {
+    return dfd_t<float>(c, dir, asym, plain(F), dF, iadd, cadd);
+}
+int dev_dfd_prod_f(st_ctx *c, int dir, int asym, const ProdF &F, float *dF, int iadd, double cadd) {
+    return dfd_t<float>(c, dir, asym, F, dF, iadd, cadd);
+}
+int dev_d2fd2_f(st_ctx *c, int dir, int asym, const float *F, float *dF, float *d2F, int iadd) {
+    return d2_t<float>(c, dir, asym, F, dF, d2F, iadd, 0);
+}
+int dev_lap_f(st_ctx *c, int dir, const float *F, float *out, int iadd, bool second) {
+    return lap_t<float>(c, dir, F, out, iadd, second);
+}
+int dev_gauss_f(st_ctx *c, int dir, const float *F, float *Fg) { return gauss_t<float>(c, dir, F, Fg); }
 
 // ---- two first derivatives along one direction, one launch ---------------------
-int launch_pair_f32(st_ctx *c, const D1PairT<float> &g, double bytes);
-
-// Two first derivatives of the bounded lines whose producers form a compiled
-// pair (kPairOps) run as one launch, in order; the periodic family and any
-// other pair run as two launches, with the same results.  The callers pair
-// operations that share fields (the second reads what the first reads, or
-// adds to what it wrote), which is where one launch saves DRAM traffic.
+// The pairs that the RHS routines form share operand fields, so that one
+// launch reads each field once:
+//   A  F, U F            B  a b, c (a b)            C  the species flux, its energy counterpart
+//   D  a u, (b + c) u    E  a u, b u
+// Each operation is the single one's arithmetic, so the results are those of
+// two launches.  Any other pair, and one whose operations add to the same
+// field, runs as two launches.
 template <class T>
 static int dfd_pair_t(st_ctx *c, int dir, const D1SpecT<T> *ops) {
-    const bool fuse = c->p.family != ST_FAMILY_PERIODIC && pair_kind(ops[0].F.op, ops[1].F.op) >= 0;
-    if (!fuse) {
-        for (int i = 0; i < 2; i++) {
-            if constexpr (sizeof(T) == 8)
-                ST_TRY(dev_dfd_prod(c, dir, ops[i].asym, ops[i].F, ops[i].dF, ops[i].iadd, ops[i].cadd));
-            else
-                ST_TRY(dev_dfd_prod_f(c, dir, ops[i].asym, ops[i].F, ops[i].dF, ops[i].iadd, ops[i].cadd));
-        }
+    const ProdT<T> &p = ops[0].F, &q = ops[1].F;
+    LineArgsT<T> a = make_args<T>(c, dir);
+    const T *in[4] = {nullptr, nullptr, nullptr, nullptr};
+    int id = -1, ni = 0;
+    auto use = [&](RecId r, std::initializer_list<const T *> f) { id = r; for (const T *x : f) in[ni++] = x; };
+    if (ops[0].dF != ops[1].dF) {
+        if (p.op == PR_A && q.op == PR_MUL && q.b == p.a) use(R_PAIRA, {p.a, q.a});
+        else if (p.op == PR_MUL && q.op == PR_MULMUL && q.a == p.a && q.b == p.b) use(R_PAIRB, {p.a, p.b, q.c});
+        else if (p.op == PR_SPEC && q.op == PR_SPECT && q.a == p.a && q.b == p.b && q.c == p.c &&
+                 c->p.family != ST_FAMILY_PERIODIC)
+            use(R_PAIRC, {p.a, p.b, p.c, q.d});
+        else if (p.op == PR_MUL && q.op == PR_ADDMUL && q.c == p.b) use(R_PAIRD, {p.a, p.b, q.a, q.b});
+        else if (p.op == PR_MUL && q.op == PR_MUL && q.b == p.b) use(R_PAIRE, {p.a, p.b, q.a});
+    }
+    if (id < 0) {
+        for (int i = 0; i < 2; i++) ST_TRY(dfd_t<T>(c, dir, ops[i].asym, ops[i].F, ops[i].dF, ops[i].iadd, ops[i].cadd));
         return ST_OK;
     }
-    D1PairT<T> g{};
-    g.a = make_args<T>(c, dir);
-    // algorithmic bytes per cell: each distinct field once (the producers'
-    // operands and accumulated outputs read, the outputs written)
-    const void *rd[10], *wr[2];
-    int nr = 0, nw = 0;
-    auto add_once = [](const void **v, int &n, const void *p) {
-        for (int k = 0; k < n; k++) if (v[k] == p) return;
-        v[n++] = p;
-    };
+    T *out[2];
     for (int i = 0; i < 2; i++) {
-        const D1SpecT<T> &o = ops[i];
-        if constexpr (sizeof(T) == 4) ST_TRY(check_f2(c, o.F, o.dF, nullptr));
-        D1OpT<T> &d = g.op[i];
-        d.F = o.F; d.O1 = o.dF; d.asym = o.asym; d.iadd = o.iadd;
-        d.fac1 = o.cadd * c->s1[dir] * (double)(g.a.geo.n - 1);           // src/derivCDopt6_sym_tri.f:424
-        if constexpr (sizeof(T) == 8) d.t1 = c->tri[dir][o.asym ? K_D1A : K_D1S];
-        else d.t1 = c->trif[dir][o.asym ? K_D1A : K_D1S];
-        const int op = o.F.op, ni = op == PR_A ? 1 : op == PR_MUL ? 2 : op == PR_SPECT ? 4 : 3;
-        const T *in[4] = {o.F.a, o.F.b, o.F.c, o.F.d};
-        for (int k = 0; k < ni; k++) add_once(rd, nr, in[k]);
-        // an accumulated output is read, unless the first operation wrote it
-        if (o.iadd && !(i == 1 && o.dF == ops[0].dF)) add_once(rd, nr, o.dF);
-        add_once(wr, nw, o.dF);
+        set_d1(c, a, i, ops[i].asym, ops[i].iadd, ops[i].cadd);
+        out[i] = ops[i].dF;
+        ST_TRY(aligned(c, out[i]));
     }
-    const double bytes = (double)sizeof(T) * (double)(nr + nw);
-    if constexpr (sizeof(T) == 8) return launch_pair_t<double>(c, g, bytes);
-    else return launch_pair_f32(c, g, bytes);
+    for (int k = 0; k < ni; k++) ST_TRY(aligned(c, in[k]));
+    a.k0 = q.k0; a.k1 = q.k1; a.k2 = q.k2;
+    return launch(c, (RecId)id, a, in, out);
 }
 
 int dev_dfd_pair(st_ctx *c, int dir, const D1SpecT<double> *ops) { return dfd_pair_t(c, dir, ops); }
 int dev_dfd_pair_f(st_ctx *c, int dir, const D1SpecT<float> *ops) { return dfd_pair_t(c, dir, ops); }
-
-int dev_d2fd2_f(st_ctx *c, int dir, int asym, const float *F, float *dF, float *d2F, int iadd) {
-    LineArgsF a = make_args<float>(c, dir);
-    a.F = plain_f(F); a.O1 = dF; a.O2 = d2F; a.asym = asym; a.iadd = iadd;
-    ST_TRY(check_f2(c, a.F, dF, d2F));
-    a.fac1 = 1.0 * c->s1[dir] * (double)(a.geo.n - 1);
-    a.fac2 = ((double)((a.geo.n - 1) * (a.geo.n - 1))) * c->s2[dir];
-    a.t1 = c->trif[dir][asym ? K_D1A : K_D1S];
-    a.t2 = c->trif[dir][asym ? K_D2A : K_D2S];
-    return launch_line(c, OP_D2, a);
-}
-
-int dev_dfd_sum_f(st_ctx *c, int dir, int asym, const float *F, float *dF, const float *E1, const float *E2) {
-    if (dir == 1) return fail(c, ST_E_ARG, "fused sum: x or z lines only");
-    ST_TRY(check_f2(c, plain_f(F), dF, E1) == ST_OK ? check_f2(c, plain_f(E2), nullptr, nullptr) : ST_E_ARG);
-    LineArgsF a = make_args<float>(c, dir);
-    a.F = plain_f(F); a.O1 = dF; a.asym = asym; a.iadd = 0; a.E1 = E1; a.E2 = E2;
-    a.fac1 = 1.0 * c->s1[dir] * (double)(a.geo.n - 1);
-    a.t1 = c->trif[dir][asym ? K_D1A : K_D1S];
-    return launch_line(c, OP_D1, a);
-}
-
-int dev_d2fd2_sum_f(st_ctx *c, int dir, int asym, const float *F, float *d2F, const float *E1,
-                    const float *E2) {
-    if (dir == 1) return fail(c, ST_E_ARG, "fused sum: x or z lines only");
-    ST_TRY(check_f2(c, plain_f(F), d2F, E1) == ST_OK ? check_f2(c, plain_f(E2), nullptr, nullptr) : ST_E_ARG);
-    LineArgsF a = make_args<float>(c, dir);
-    a.F = plain_f(F); a.O2 = d2F; a.asym = asym; a.iadd = 0; a.E1 = E1; a.E2 = E2;
-    a.fac2 = ((double)((a.geo.n - 1) * (a.geo.n - 1))) * c->s2[dir];
-    a.t2 = c->trif[dir][asym ? K_D2A : K_D2S];
-    return launch_line(c, OP_D2, a);
-}
-
-int dev_gauss_f(st_ctx *c, int dir, const float *F, float *Fg) {
-    ST_TRY(check_f2(c, plain_f(F), Fg, nullptr));
-    LineArgsF a = make_args<float>(c, dir);
-    a.F = plain_f(F); a.O1 = Fg;
-    return launch_line(c, OP_GAUSS, a);
-}
 
 // ---- general solvers (per-line coefficients), thread per line ---------------
 // tridiagonal_serial / tridiagonal_periodic_serial, src/tridiagonal.f90:197-287.

@@ -4,6 +4,8 @@
 
 namespace st {
 
-int launch_line_cyc(st_ctx *c, OpKind op, const LineArgs &a) { return launch_line_t<true, double>(c, op, a); }
+int launch_rec_cyc(st_ctx *c, RecId id, LineArgs &a, const double *const *in, double *const *out) {
+    return launch_rec_t<true, double>(c, id, a, in, out);
+}
 
 }  // namespace st

@@ -4,6 +4,8 @@
 
 namespace st {
 
-int launch_line_cyc_f32(st_ctx *c, OpKind op, const LineArgsF &a) { return launch_line_t<true, float>(c, op, a); }
+int launch_rec_cyc_f32(st_ctx *c, RecId id, LineArgsF &a, const float *const *in, float *const *out) {
+    return launch_rec_t<true, float>(c, id, a, in, out);
+}
 
 }  // namespace st

@@ -1,263 +1,359 @@
-// st_linekern.cuh - the line-operator kernels (compact derivatives, compact
-// filter, Gaussian filter) and their launch dispatch, templated on the family:
+// st_linekern.cuh - the line-operator kernel (compact derivatives, compact
+// filter, Gaussian filter) and its launch dispatch, templated on the family:
 // CYC = false for the _mf family's bounded lines, CYC = true for periodic
 // lines (wrapped halos and the corner correction after the banded solve).
-// The two families are instantiated in separate translation units
-// (st_kernels.cu, st_kernels_cyc.cu) so that the bounded-line kernels keep
-// their register allocation.
+//
+// One persistent kernel, k_lines, runs a compile-time list of operations
+// ("recipe") on each tile of lines.  A CTA keeps a ring of K slots in shared
+// memory; a slot holds the tiles of a recipe's input fields.  The TMA engine
+// fills a slot while the CTA's threads solve the slot before it in registers;
+// the results overwrite input tiles that no later operation reads and leave
+// by TMA stores, or by TMA reductions (cp.reduce, add) where the operation
+// accumulates, so the old value never comes to the SM.  Where only one slot
+// fits, its tiles are filled for the next lines one by one, as the operations
+// are done with them.
+//
+// What bounds it: at one field in and one out the TMA ring alone moves 5.5 to
+// 5.9 TB/s on 384^3 (x, z and y lines; 0.84 to 0.90 of a plain copy), and an
+// accumulation 5.8 to 6.3 TB/s of its 24 bytes per cell.  With the solve, FP64,
+// 384^3, against kernels that read the rows from global memory thread by
+// thread (about 85 instructions per cell, 512 threads of 64 registers):
+//   first derivative x, y, z   193, 172, 189 us (230, 290, 222)
+//   filter                     322, 309, 317 us (410, 437, 402)
+//   second with first          316, 300, 309 us (490)
+//   two first derivatives of Compute_Laplacian in one pass, accumulated
+//                              285, 258 us (480 as two passes)
+// The solve's latency is what is left: a solve costs about 130 us of a 384^3
+// pass, and is hidden only while another CTA of the SM is transferring.
 #pragma once
 #include <cfloat>
+#include <cuda.h>
+#include <type_traits>
+#include <utility>
 #include "st_line.cuh"
 
 namespace st {
 
-// T: element type of the fields read and written and of the arithmetic:
-// double, or float in the FP32 mode, whose kernels give each thread two
-// neighbouring lines (value type F2, 32 lines per CTA).
+enum OpKind { OP_D1, OP_D2, OP_FILTER, OP_GAUSS, OP_LAP, OP_D1ADD, OP_FILTERM };
+
+// One operation of a recipe: KIND applied to the operand SRC with arguments
+// op[ARG]; the result goes to tile OUT (OP_D1ADD: is added to what is there)
+// and from there to output field IO (none where IO < 0).
+template <int KIND_, class SRC_, int OUT_, int IO_, int ARG_ = IO_>
+struct Op {
+    static constexpr int KIND = KIND_, OUT = OUT_, IO = IO_, ARG = ARG_;
+    using SRC = SRC_;
+};
+// NIN input fields (tiles 0 .. NIN-1 of a slot), NT tiles of a slot
+template <int NIN_, int NT_, class... OPS>
+struct Recipe {
+    static constexpr int NIN = NIN_, NT = NT_, NOP = sizeof...(OPS);
+};
+
+// The recipes (operation order: an operation may overwrite only tiles that no
+// later one reads; outputs are indexed as the caller gives them)
+using RecD1 = Recipe<1, 1, Op<OP_D1, Src<PR_A, 0>, 0, 0>>;
+using RecMul = Recipe<2, 2, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, 0>>;
+using RecAddMul = Recipe<3, 3, Op<OP_D1, Src<PR_ADDMUL, 0, 1, 2>, 0, 0>>;
+using RecMulMul = Recipe<3, 3, Op<OP_D1, Src<PR_MULMUL, 0, 1, 2>, 0, 0>>;
+using RecHMulAdd = Recipe<3, 3, Op<OP_D1, Src<PR_HMULADD, 0, 1, 2>, 0, 0>>;
+// a b, plus c's derivative: the FP32 mode's form of RecHMulAdd, which would
+// round the sum to the pressure's magnitude before it is differenced
+using RecMulPlus = Recipe<3, 3, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, -1, 1>, Op<OP_D1ADD, Src<PR_A, 2>, 0, 0>>;
+using RecSpec = Recipe<3, 3, Op<OP_D1, Src<PR_SPEC, 0, 1, 2>, 0, 0>>;
+using RecSpecT = Recipe<4, 4, Op<OP_D1, Src<PR_SPECT, 0, 1, 2, 3>, 0, 0>>;
+using RecD2 = Recipe<1, 1, Op<OP_D2, Src<PR_A, 0>, 0, 0>>;
+using RecD2D1 = Recipe<1, 2, Op<OP_D2, Src<PR_A, 0>, 1, 0>, Op<OP_D1, Src<PR_A, 0>, 0, 1>>;
+using RecFilter = Recipe<1, 1, Op<OP_FILTER, Src<PR_A, 0>, 0, 0>>;
+using RecFilterM = Recipe<1, 1, Op<OP_FILTERM, Src<PR_A, 0>, 0, 0>>;   // the FP32 mode's
+using RecGauss = Recipe<1, 1, Op<OP_GAUSS, Src<PR_A, 0>, 0, 0>>;
+using RecLap = Recipe<1, 1, Op<OP_LAP, Src<PR_A, 0>, 0, 0>>;
+// pairs of first derivatives that share operand fields: outputs 0 and 1
+using RecPairA = Recipe<2, 2, Op<OP_D1, Src<PR_MUL, 1, 0>, 1, 1>, Op<OP_D1, Src<PR_A, 0>, 0, 0>>;              // F; U F
+using RecPairB = Recipe<3, 3, Op<OP_D1, Src<PR_MULMUL, 0, 1, 2>, 2, 1>, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, 0>>;  // a b; c (a b)
+using RecPairC = Recipe<4, 4, Op<OP_D1, Src<PR_SPECT, 0, 1, 2, 3>, 3, 1>, Op<OP_D1, Src<PR_SPEC, 0, 1, 2>, 0, 0>>;
+using RecPairD = Recipe<4, 4, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, 0>, Op<OP_D1, Src<PR_ADDMUL, 2, 3, 1>, 2, 1>>;  // a u; (b + c) u
+using RecPairE = Recipe<3, 3, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, 0>, Op<OP_D1, Src<PR_MUL, 2, 1>, 2, 1>>;        // a u; b u
+
 template <class T>
-struct LineArgsT {
-    ProdT<T> F;
-    T *O1, *O2;
-    LineGeo geo;
-    int S, P;
-    double fac1, fac2;
-    int asym, iadd;
-    const T *E1, *E2;   // x and z lines: O1 (k_dfd) / O2 (k_d2fd2) = (result + E1) + E2 when E1 is set
-    int cyc;            // periodic family: wrapped halos, corner correction (selects the CYC kernels)
-    TriTabT<T> t1, t2;
+struct OpArgT {
+    double fac1, fac2;       // first / second derivative factor
+    int asym;
+    TriTabT<T> t1, t2;       // first / second derivative tables (OP_LAP: t2 the antisymmetric first derivative's)
+};
+
+template <class T>
+struct alignas(64) LineArgsT {
+    CUtensorMap in[4], out[2];
+    int red[2];                   // output accumulates
+    int dir, n, P;
+    int jb;                       // x and z lines: tiles along y
+    int cblk, ntile;              // tiles per case, in all
+    int box;                      // rows of a TMA box (x and z lines)
+    int K;                        // slots
+    unsigned tb;                  // bytes of a tile
+    int *wait_flag;
+    OpArgT<T> op[2];
     PenTab p;
-    Consts K;
+    Consts c;
+    double k0, k1, k2;
 };
 using LineArgs = LineArgsT<double>;
 using LineArgsF = LineArgsT<float>;
 
-// Every line kernel is instantiated for x/z lines (YT = false: direct
-// coalesced row accesses) and for y lines (YT = true: staged through a
-// shared [32][n+1] tile).
-#define LINE_PROLOGUE                                                                  \
-    using V = typename Val<T>::V;                                                      \
-    using A = typename Val<T>::A;                                                      \
-    constexpr int W = Val<T>::W;                                                       \
-    __shared__ CarryBufT<V> cb;                                                        \
-    extern __shared__ __align__(16) unsigned char smem_raw[];                          \
-    A *tile = reinterpret_cast<A *>(smem_raw);                                         \
-    const int lane = threadIdx.x & (kLanes - 1), s = threadIdx.x / kLanes, n = a.geo.n, row0 = s * S; \
-    const ColMap m = a.geo.template map<W>(blockIdx.x);                                \
-    const RowReader<OP, T, V> rd = YT ? RowReader<OP, T, V>{tile + W * lane * (n + 1), nullptr, 0, 0, n + 1} \
-                                      : RowReader<OP, T, V>{nullptr, &a.F, m.base + (size_t)lane * W * m.lstride, \
-                                                            m.rstride, 0};
-
-// L2 prefetch of the rows the block kAhead blocks later will load (about one
-// wave of resident CTAs ahead: 2 per SM on 148 SMs), so that the next wave's
-// loads find their lines in L2 while this wave solves.
-constexpr unsigned kAhead = kLineCtasPerSm * 148;
-__device__ __forceinline__ void pf_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-template <int S, bool YT, int OP, class T>
-__device__ __forceinline__ void prefetch_next(const LineGeo &geo, const ProdT<T> &F, int lane, int row0) {
-    const unsigned nb = blockIdx.x + kAhead;
-    if (nb >= gridDim.x) return;
-    constexpr int W = Val<T>::W;
-    constexpr int NI = OP == PR_A ? 1 : OP == PR_MUL ? 2 : OP == PR_SPECT ? 4 : 3;   // fields the producer reads
-    const ColMap m = geo.template map<W>(nb);
-    const T *f[4] = {F.a, F.b, F.c, F.d};
-    if (YT) {
-        // the block's lines are one contiguous range: one 128-byte line per thread and pass
-        const size_t bytes = (size_t)kLanes * W * geo.n * sizeof(T);
-        for (size_t off = (size_t)threadIdx.x * 128; off < bytes; off += (size_t)blockDim.x * 128)
-#pragma unroll
-            for (int k = 0; k < NI; k++) pf_l2(reinterpret_cast<const char *>(f[k] + m.base) + off);
-    } else {
-        // a row of the block's lines is 128 contiguous bytes: lane 0 of each segment
-        if (lane != 0) return;
-#pragma unroll
-        for (int t = 0; t < S; t++)
-#pragma unroll
-            for (int k = 0; k < NI; k++) pf_l2(f[k] + m.base + (size_t)(row0 + t) * m.rstride);
+// ---- TMA and mbarrier instructions -----------------------------------------
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(unsigned bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase to complete, at most ~2e6 polls (a poll suspends the
+// thread for a while, so this is seconds); past that the flag is set and the
+// results are garbage, which the host reports at the next synchronising call.
+__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, int *flag) {
+    for (int i = 0; i < 2000000; i++) {
+        unsigned ok;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return;
     }
+    *reinterpret_cast<volatile int *>(flag) = 1;
 }
+__device__ __forceinline__ void tma_load(unsigned dst, const CUtensorMap *m, int c0, int c1, int c2, int c3, unsigned bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 ::"r"(dst), "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_store(const CUtensorMap *m, int c0, int c1, int c2, int c3, unsigned src, bool red) {
+    if (red)
+        asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                     ::"l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(src) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                     ::"l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(src) : "memory");
+}
+template <int N> __device__ __forceinline__ void wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-template <int S, int H, bool YT, int OP, class T, class V, class A>
-__device__ __forceinline__ void get_rows(V (&v)[S + 2 * H], const A *tile, const ProdT<T> &F,
-                                         const ColMap &m, int lane, int a, int n, int cyc) {
-    if (YT) ytile_rows<S, H>(v, tile, lane, a, n, cyc);
-    else load_rows<S, H, OP>(v, F, m, lane, a, n, cyc);
-}
-// SYNCED: a barrier since the last read of the tile (the solves' exchange)
-template <int S, bool YT, bool SYNCED, int N, class T, class V, class A>
-__device__ __forceinline__ void put_rows(const V (&v)[N], A *tile, T *O, const ColMap &m,
-                                         int lane, int a, int n, int add, const T *E1 = nullptr,
-                                         const T *E2 = nullptr) {
-    if (YT) {
-        if (!SYNCED) __syncthreads();    // every thread has finished reading the tile
-        ytile_put<S>(tile, v, lane, a, n);
-        __syncthreads();
-        ytile_store<T>(tile, O, m.base, n, add);
-    } else {
-        store_rows<S>(v, O, m, lane, a, add, E1, E2);
-    }
-}
+// ---- the kernel ------------------------------------------------------------
+// shared memory: K slots of NT tiles, the carry buffers, the slots' barriers
+constexpr int kSlotsMax = 4;
+template <class V, int L> __host__ __device__ constexpr unsigned corner_bytes() { return 4 * L * sizeof(V); }
+// bytes behind the tiles: the carry buffers (two of one value per segment and
+// column, or one of two values for the filter), the corner values, the
+// barriers, the filter's outer factors
+// (a scan of float carries needs one column more)
+template <class V, int L>
+__host__ __device__ inline unsigned carry_one(int P) { return (unsigned)(P + (std::is_same<V, F2>::value ? 1 : 0)) * L * (unsigned)sizeof(V); }
+template <class V, int L>
+__host__ __device__ inline unsigned carry_bytes(int P) { return 2u * carry_one<V, L>(P) + corner_bytes<V, L>() + 8u * kSlotsMax; }
 
-// DF*_sym/_asym and the periodic DF*: O1 (=|+=) cadd * dF/ds
-template <int S, bool YT, int OP, bool CYC, class T>
-__global__ void __launch_bounds__(kLineThreads, kLineCtasPerSm) k_dfd(LineArgsT<T> a) {
-    LINE_PROLOGUE
-    if (YT) { ytile_load<OP>(tile, a.F, m.base, n); prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0); __syncthreads(); }
-    V v[S + 4];
-    get_rows<S, 2, YT, OP>(v, tile, a.F, m, lane, row0, n, CYC);
-    if (!YT) prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0);
-    rhs_d1<S, 2>(v, row0, n, a.asym, CYC, a.fac1, a.K, rd);
-    tri_solve<S>(v, a.t1, s, a.P, lane, cb);
-    if constexpr (CYC) cyc_fix<S, S + 4, 2>(v, a.t1.cyc, s, a.P, lane, cb);
-    put_rows<S, YT, true>(v, tile, a.O1, m, lane, row0, n, a.iadd, a.E1, a.E2);
-}
-
-// D2F*2_sym/_asym and the periodic D2F*2: O2 = d2F/ds2; if iadd, O1 = dF/ds
-// (cadd = 1).  The first
-// derivative re-reads the rows (the CTA's lines are still in L2).
-template <int S, bool YT, bool CYC, class T>
-__global__ void __launch_bounds__(kLineThreads, kLineCtasPerSm) k_d2fd2(LineArgsT<T> a) {
-    constexpr int OP = PR_A;
-    LINE_PROLOGUE
-    {
-        if (YT) { ytile_load<OP>(tile, a.F, m.base, n); prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0); __syncthreads(); }
+template <int S, int M, int L, bool YT, bool CYC, class T, class OPD, class Mid>
+__device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o, const View<S, L, YT, T> &w, int s, int lane,
+                                       const CarryT<typename Val<T>::V, L> &cb, Mid mid) {
+    using V = typename Val<T>::V;
+    using SRC = typename OPD::SRC;
+    const int n = a.n, P = a.P, row0 = s * S;
+    auto rd = [&](int i) { return w.template row<SRC>(i); };
+    if constexpr (OPD::KIND == OP_D1 || OPD::KIND == OP_D1ADD || OPD::KIND == OP_LAP) {
         V v[S + 4];
-        get_rows<S, 2, YT, OP>(v, tile, a.F, m, lane, row0, n, CYC);
-        if (!YT) prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0);
-        rhs_d2<S, 2>(v, row0, n, a.asym, CYC, a.fac2, a.K, rd);
-        tri_solve<S>(v, a.t2, s, a.P, lane, cb);
-        if constexpr (CYC) cyc_fix<S, S + 4, 2>(v, a.t2.cyc, s, a.P, lane, cb);
-        put_rows<S, YT, true>(v, tile, a.O2, m, lane, row0, n, 0, a.E1, a.E2);
-    }
-    if (a.iadd) {
-        __syncthreads();   // carry buffers and tile are reused
-        if (YT) { ytile_load<OP>(tile, a.F, m.base, n); __syncthreads(); }
+        w.template load<SRC, 2>(v);
+        rhs_d1<S, CYC>(v, row0, n, o.asym, o.fac1, a.c, rd);
+        tri<S, M, L>(v, o.t1, s, P, lane, cb, mid);
+        if constexpr (CYC) cyc_fix<S, L, 2>(v, o.t1.cyc, o.t1.clo, o.t1.chi, s, P, lane, cb);
+        w.template store<OPD::KIND == OP_D1ADD>(v, OPD::OUT);
+        if constexpr (OPD::KIND == OP_LAP) {
+            // the derivative (in the tile now) of a symmetric field is
+            // antisymmetric; both passes of Compute_Laplacian in one
+            __syncthreads();
+            using D = Src<PR_A, OPD::OUT>;
+            auto rd2 = [&](int i) { return w.template row<D>(i); };
+            w.template load<D, 2>(v);
+            rhs_d1<S, CYC>(v, row0, n, 1, o.fac1, a.c, rd2);
+            tri<S, M, L>(v, o.t2, s, P, lane, cb, [] {});
+            if constexpr (CYC) cyc_fix<S, L, 2>(v, o.t2.cyc, o.t2.clo, o.t2.chi, s, P, lane, cb);
+            w.store(v, OPD::OUT);
+        }
+    } else if constexpr (OPD::KIND == OP_D2) {
         V v[S + 4];
-        get_rows<S, 2, YT, OP>(v, tile, a.F, m, lane, row0, n, CYC);
-        rhs_d1<S, 2>(v, row0, n, a.asym, CYC, a.fac1, a.K, rd);
-        tri_solve<S>(v, a.t1, s, a.P, lane, cb);
-        if constexpr (CYC) cyc_fix<S, S + 4, 2>(v, a.t1.cyc, s, a.P, lane, cb);
-        put_rows<S, YT, true>(v, tile, a.O1, m, lane, row0, n, 0);
+        w.template load<SRC, 2>(v);
+        rhs_d2<S, CYC>(v, row0, n, o.asym, o.fac2, a.c, rd);
+        tri<S, M, L>(v, o.t2, s, P, lane, cb, mid);
+        if constexpr (CYC) cyc_fix<S, L, 2>(v, o.t2.cyc, o.t2.clo, o.t2.chi, s, P, lane, cb);
+        w.store(v, OPD::OUT);
+    } else if constexpr (OPD::KIND == OP_FILTER || OPD::KIND == OP_FILTERM) {
+        V v[S + 8];
+        w.template load<SRC, 4>(v);
+        rhs_filter<S, CYC>(v, row0, n, o.asym, a.c, rd);
+        if constexpr (OPD::KIND == OP_FILTER) pen_solve<S, L>(v, a.p, s, P, lane, cb, mid);
+        else pen_solve_m<S / M, M, L>(v, a.p, s, P, lane, cb, mid);
+        if constexpr (CYC) cyc_fix<S, L, 4>(v, a.p.cyc, a.p.clo, a.p.chi, s, P, lane, cb);
+        w.store(v, OPD::OUT);
+    } else {
+        V v[S + 8];
+        w.template load<SRC, 4>(v);
+        rhs_gauss<S, CYC>(v, row0, n, a.c, rd);
+        __syncthreads();                       // every thread has read its rows
+        if (threadIdx.x == 0) mid();
+        w.store(v, OPD::OUT);
     }
+    proxy_fence();                             // the tile's new values, for the TMA store
 }
 
-// Compact_Filter_*_sym/_asym and the periodic Compact_Filter_*: O1 = filtered
-// F.  O1 may alias F: every read of
-// F (including the boundary re-reads) happens before the solve's first
-// barrier and every write after its last one.
-template <int S, bool YT, bool CYC, class T>
-__global__ void __launch_bounds__(kLineThreads, kLineCtasPerSm) k_filter(LineArgsT<T> a) {
-    constexpr int OP = PR_A;
-    LINE_PROLOGUE
-    if (YT) { ytile_load<OP>(tile, a.F, m.base, n); prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0); __syncthreads(); }
-    double v[S + 8];
-    get_rows<S, 4, YT, OP>(v, tile, a.F, m, lane, row0, n, CYC);
-    if (!YT) prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0);
-    rhs_filter<S, 4>(v, row0, n, a.asym, CYC, a.K, rd);
-    pen_solve<S>(v, a.p, s, a.P, lane, cb);
-    if constexpr (CYC) cyc_fix<S, S + 8, 4>(v, a.p.cyc, s, a.P, lane, cb);
-    put_rows<S, YT, true>(v, tile, a.O1, m, lane, row0, n, 0);
-}
-
-// Gaussian_Filter_X/Y/Z (both families): O1 = explicit 9-point Gaussian of F
-// (O1 != F)
-template <int S, bool YT, bool CYC, class T>
-__global__ void __launch_bounds__(kLineThreads, kLineCtasPerSm) k_gauss(LineArgsT<T> a) {
-    constexpr int OP = PR_A;
-    LINE_PROLOGUE
-    (void)cb;
-    if (YT) { ytile_load<OP>(tile, a.F, m.base, n); prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0); __syncthreads(); }
-    V v[S + 8];
-    get_rows<S, 4, YT, OP>(v, tile, a.F, m, lane, row0, n, CYC);
-    if (!YT) prefetch_next<S, YT, OP>(a.geo, a.F, lane, row0);
-    rhs_gauss<S, 4>(v, row0, n, CYC, a.K, rd);
-    put_rows<S, YT, false>(v, tile, a.O1, m, lane, row0, n, 0);
-}
-
-// ---- two first derivatives along one direction in one launch ------------
-// Hyper_RHS (src/hyper_rhs_sym_mf.f) differentiates, in each direction, a
-// viscous flux and then its product with a velocity component (v_h S_12 and
-// then v_h S_12 u, or tau_xx and then u tau_xx); Species_RHS
-// (src/species_rhs_sym.f) the diffusive flux of Y and then its energy
-// counterpart, and Y and then rho u_i Y.  The second operand set contains
-// the first, so one CTA runs both on its own lines: the second
-// operation finds the shared rows in L2, as the first derivative of
-// D2F*2 with iadd does.  (An accumulated output, the pressure-gradient case
-// below, is re-read by the thread that wrote it, with plain loads, so it is
-// coherent without a barrier.)  The convective fluxes of RHS pair up the same way
-// where two adjacent ones share the velocity factor, or where the second
-// adds the pressure gradient to what the first wrote.  Each operation is
-// exactly the k_dfd of its arguments, so the results are bitwise those of
-// two launches.
-template <class T>
-struct D1OpT {
-    ProdT<T> F;
-    T *O1;
-    double fac1;
-    int asym, iadd;
-    TriTabT<T> t1;
-};
-template <class T>
-struct D1PairT {
-    LineArgsT<T> a;      // geometry, segmentation and scheme constants (its F, O1, t1 unused)
-    D1OpT<T> op[2];
+// What thread 0 needs to know of a recipe: per operation its output tile and
+// field, and the input tiles that are free once the operation has read its
+// rows (read by no later operation and not written).
+template <class R> struct RecipeInfo;
+template <int NIN, int NT, class... OPS>
+struct RecipeInfo<Recipe<NIN, NT, OPS...>> {
+    static constexpr int N = sizeof...(OPS);
+    template <class O> __host__ __device__ static constexpr unsigned reads() {
+        const int t[4] = {O::SRC::T0, O::SRC::T1, O::SRC::T2, O::SRC::T3};
+        unsigned m = 0;
+        for (int k = 0; k < O::SRC::n; k++) m |= 1u << t[k];
+        return m;
+    }
+    __host__ __device__ static constexpr int out(int op) { const int o[N] = {OPS::OUT...}; return o[op]; }
+    __host__ __device__ static constexpr int io(int op) { const int o[N] = {OPS::IO...}; return o[op]; }
+    // TMA store groups of a tile of lines
+    __host__ __device__ static constexpr int stores() { int m = 0; for (int k = 0; k < N; k++) m += io(k) >= 0; return m; }
+    __host__ __device__ static constexpr unsigned freed(int op) {
+        const unsigned rd[N] = {reads<OPS>()...};
+        unsigned keep = 0;
+        for (int k = 0; k < N; k++) keep |= (k > op ? rd[k] : 0u) | 1u << out(k);
+        return rd[op] & ~keep;
+    }
 };
 
-// block and thread index read so that the compiler keeps nothing derived
-// from them live from the first operation to the second
-__device__ __forceinline__ unsigned opaque_ctaid() {
-    unsigned v;
-    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(v));
-    return v;
-}
-__device__ __forceinline__ unsigned opaque_tid() {
-    unsigned v;
-    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(v));
-    return v;
-}
-
-// one operation; PF: the L2 prefetch of the next wave's rows of the first
-// operation (OPF, producer FN), issued with the second operation
-template <int S, bool YT, int OP, bool PF, int OPF, class T>
-__device__ __forceinline__ void pair_d1(const LineArgsT<T> &a, const D1OpT<T> &o, const ProdT<T> &FN,
-                                        CarryBufT<typename Val<T>::V> &cb, typename Val<T>::A *tile) {
-    using V = typename Val<T>::V;
-    constexpr int W = Val<T>::W;
-    const unsigned tid = opaque_tid();
-    const int lane = tid & (kLanes - 1), s = tid / kLanes, row0 = s * S, n = a.geo.n;
-    const ColMap m = a.geo.template map<W>(opaque_ctaid());
-    const RowReader<OP, T, V> rd = YT ? RowReader<OP, T, V>{tile + W * lane * (n + 1), nullptr, 0, 0, n + 1}
-                                      : RowReader<OP, T, V>{nullptr, &o.F, m.base + (size_t)lane * W * m.lstride,
-                                                            m.rstride, 0};
-    if (YT) {
-        ytile_load<OP>(tile, o.F, m.base, n);
-        if (PF) prefetch_next<S, YT, OPF>(a.geo, FN, lane, row0);
-        __syncthreads();
+template <class R> struct RecipeRun;
+template <int NIN, int NT, class... OPS>
+struct RecipeRun<Recipe<NIN, NT, OPS...>> {
+    // the operations in turn; hook(op) runs in thread 0 behind the first
+    // barrier of each
+    template <int S, int M, int L, bool YT, bool CYC, class T, class Hook, size_t... Q>
+    __device__ __forceinline__ static void run(const LineArgsT<T> &a, const View<S, L, YT, T> &w, int s, int lane,
+                                               const CarryT<typename Val<T>::V, L> &cb, Hook hook, std::index_sequence<Q...>) {
+        (run_op<S, M, L, YT, CYC, T, OPS>(a, a.op[OPS::ARG], w, s, lane, cb, [&] { hook(std::integral_constant<int, (int)Q>()); }), ...);
     }
-    V v[S + 4];
-    get_rows<S, 2, YT, OP>(v, tile, o.F, m, lane, row0, n, 0);
-    if (!YT && PF) prefetch_next<S, YT, OPF>(a.geo, FN, lane, row0);
-    rhs_d1<S, 2>(v, row0, n, o.asym, 0, o.fac1, a.K, rd);
-    tri_solve<S>(v, o.t1, s, a.P, lane, cb);
-    put_rows<S, YT, true>(v, tile, o.O1, m, lane, row0, n, o.iadd);
-}
+};
 
-template <int S, bool YT, class T, int OP0, int OP1>
-__global__ void __launch_bounds__(kLineThreads, kLineCtasPerSm) k_dfd_pair(D1PairT<T> g) {
+template <class R, int S, int M, int L, bool YT, bool CYC, class T>
+__global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) {
     using V = typename Val<T>::V;
-    using A = typename Val<T>::A;
-    __shared__ CarryBufT<V> cb;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    A *tile = reinterpret_cast<A *>(smem_raw);
-    pair_d1<S, YT, OP0, false, OP0>(g.a, g.op[0], g.op[0].F, cb, tile);
-    __syncthreads();                     // tile and carry buffers are reused
-    pair_d1<S, YT, OP1, true, OP0>(g.a, g.op[1], g.op[0].F, cb, tile);
+    using I = RecipeInfo<R>;
+    constexpr int W = Val<T>::W, NL = L * W;         // lines of a tile
+    constexpr bool PENM = std::is_same<R, RecFilterM>::value, PEN = PENM || std::is_same<R, RecFilter>::value;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const unsigned tb = a.tb, slot_b = R::NT * tb;
+    const int n = a.n, P = a.P, K = a.K, G = gridDim.x;
+    const int tid = threadIdx.x, lane = tid % L, s = tid / L;
+    unsigned char *tail = smem + K * slot_b;
+    const unsigned cbb = (PENM ? 2u : 1u) * carry_one<V, L>(P * M);
+    unsigned char *tab = tail + 2 * cbb + corner_bytes<V, L>() + 8 * kSlotsMax;
+    const CarryT<V, L> cb{reinterpret_cast<V *>(tail), reinterpret_cast<V *>(tail + cbb), reinterpret_cast<V *>(tail + 2 * cbb),
+                          reinterpret_cast<const V *>(tab)};
+    const unsigned bars = smem_u32(tail + 2 * cbb + corner_bytes<V, L>());
+    if constexpr (PEN) pen_fill(reinterpret_cast<double *>(tab), a.p, P * M, S / M, !PENM);
+
+    // thread 0: transfers of one tile of lines.  x lines: (y, z) at c0, c1
+    // and rows along the third coordinate; z lines: (y, x) and rows along the
+    // second; y lines: (row in the chunk, line, chunk)
+    auto place = [&](int tile, int &c0, int &m, int &cs) {
+        if constexpr (YT) { c0 = 0; m = tile * NL; cs = 0; return; }
+        cs = tile / a.cblk;
+        const int b = tile - cs * a.cblk;
+        m = b / a.jb;
+        c0 = (b - m * a.jb) * NL;
+    };
+    auto load_tiles = [&](int tile, int k, unsigned mask) {
+        int c0, m, cs;
+        place(tile, c0, m, cs);
+        const unsigned bar = bars + 8 * k, dst = smem_u32(smem + k * slot_b);
+#pragma unroll
+        for (int f = 0; f < R::NIN; f++) {
+            if (!(mask >> f & 1)) continue;
+            if constexpr (YT) tma_load(dst + f * tb, &a.in[f], 0, m, 0, 0, bar);
+            else
+                for (int r = 0; r < n; r += a.box)
+                    tma_load(dst + f * tb + r * 8 * L, &a.in[f], c0, a.dir == 0 ? m : r, a.dir == 0 ? r : m, cs, bar);
+        }
+    };
+    auto expect = [&](int k) { bar_expect(bars + 8 * k, R::NIN * tb); };
+    auto store_out = [&](int tile, int k, int op) {
+        int c0, m, cs;
+        place(tile, c0, m, cs);
+        const int io = I::io(op);
+        const unsigned src = smem_u32(smem + k * slot_b + I::out(op) * tb);
+        if constexpr (YT) tma_store(&a.out[io], 0, m, 0, 0, src, a.red[io] != 0);
+        else
+            for (int r = 0; r < n; r += a.box)
+                tma_store(&a.out[io], c0, a.dir == 0 ? m : r, a.dir == 0 ? r : m, cs, src + r * 8 * L, a.red[io] != 0);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    };
+    constexpr unsigned ALL = (1u << R::NIN) - 1;
+
+    if (tid == 0) {
+        for (int k = 0; k < K; k++) bar_init(bars + 8 * k);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        proxy_fence();
+    }
+    __syncthreads();
+    if (tid == 0)
+        for (int k = 0; k < K; k++)
+            if ((int)blockIdx.x + k * G < a.ntile) { expect(k); load_tiles(blockIdx.x + k * G, k, ALL); }
+
+    View<S, L, YT, T> w;
+    w.tb = tb; w.lane = lane; w.n = n; w.a = s * S; w.mid = TileAcc<L, YT, T>::start(lane, s * S);
+    w.k0 = (typename Val<T>::A)a.k0; w.k1 = (typename Val<T>::A)a.k1; w.k2 = (typename Val<T>::A)a.k2;
+    int k = 0, kp = K - 1;          // slot of this tile and of the one before
+    unsigned par = 0;
+    for (int tile = blockIdx.x; tile < a.ntile; tile += G) {
+        bar_wait(bars + 8 * k, par, a.wait_flag);
+        w.sm = smem + k * slot_b;
+        const int next = tile + (K == 1 ? 1 : K - 1) * G;
+        const bool more = next < a.ntile;
+        RecipeRun<R>::template run<S, M, L, YT, CYC, T>(a, w, s, lane, cb, [&](auto q) {
+            constexpr int OP = decltype(q)::value;
+            // the result of the operation before leaves, and with one slot
+            // the tiles that are free are filled for the next tile of lines
+            if constexpr (OP > 0) {
+                if constexpr (I::io(OP > 0 ? OP - 1 : 0) >= 0) store_out(tile, k, OP - 1);
+            }
+            if (K == 1 && more) {
+                if constexpr (OP == 0) expect(0);
+                constexpr unsigned FREED = I::freed(OP);
+                if constexpr (FREED != 0) load_tiles(next, 0, FREED);
+            }
+        }, std::make_index_sequence<I::N>());
+        __syncthreads();
+        if (tid == 0) {
+            store_out(tile, k, I::N - 1);
+            if (K == 1) {
+                // the output tiles, as their stores have been read out
+                if constexpr (I::stores() == 2) {
+                    wait_read<1>();
+                    if (more) load_tiles(next, 0, 1u << I::out(0));
+                }
+                wait_read<0>();
+                if (more) load_tiles(next, 0, 1u << I::out(I::N - 1));
+            } else {
+                // the slot of the tile before, whose stores were issued a
+                // whole tile ago
+                wait_read<I::stores()>();
+                if (tile >= G && more) { expect(kp); load_tiles(next, kp, ALL); }
+            }
+        }
+        kp = k;
+        if (++k == K) { k = 0; par ^= 1; }
+    }
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-enum OpKind { OP_D1, OP_D2, OP_FILTER, OP_GAUSS };
+// ---- launch ------------------------------------------------------------------
+// Tensor map of a field whose boxes are (parts of) one tile of nl lines: 4-D
+// (y, z, x, case) for x and z lines; (row in a 128-byte chunk, line, chunk)
+// with the 128-byte swizzle for y lines
+int line_map(st_ctx *c, CUtensorMap *m, const void *p, bool f32, int dir, int nl, int box);
 
-// opt in to the dynamic shared memory a kernel needs on top of its static
-// carry buffers (the default cap is 48 KB in total); once per kernel and size
 template <auto Kern>
 static void set_smem(size_t bytes) {
     static size_t done = 0;   // one counter per kernel instantiation
@@ -267,124 +363,135 @@ static void set_smem(size_t bytes) {
     }
 }
 
-template <int S, bool YT, bool CYC, class T>
-static void launch_SY(st_ctx *c, OpKind op, const LineArgsT<T> &a0, cudaStream_t st) {
-    const size_t nlines = c->dm.n3 / (size_t)a0.geo.n;     // lines of one case
-    constexpr int NL = kLanes * Val<T>::W;
-    LineArgsT<T> a = a0;
-    a.geo.cblk = (unsigned)(nlines / NL);                  // CTAs per case
-    a.geo.cstride = c->dm.n3;
-    dim3 grid(a.geo.cblk * (unsigned)c->na), block(kLanes * a.P);
-    const size_t smem = YT ? (size_t)NL * (a.geo.n + 1) * sizeof(T) : 0;
-    // algorithmic bytes: every input and output field touched once
-    const double n3 = (double)c->ncell();
-    // inputs: 1 field, or every field a producer expression reads
-    static const int nin[6] = {1, 2, 3, 3, 3, 4};
-    const double es = (double)sizeof(T);
-    double b = es * nin[a.F.op] + es;              // + one output
-    if (op == OP_D1 && a.iadd) b += es;            // read-modify-write
-    if (op == OP_D2 && a.iadd) b += es;            // second output
-    if (a.E1) b += 2 * es;                         // epilogue addends
-    static const char *names[4] = {"k_dfd", "k_d2fd2", "k_filter", "k_gauss"};
-    int pi = prof_start(c, names[op], b * n3);
-    switch (op) {
-        case OP_D1:
-            switch (a.F.op) {
-#define PCASE(o_) case o_: set_smem<k_dfd<S, YT, o_, CYC, T>>(smem); k_dfd<S, YT, o_, CYC, T><<<grid, block, smem, st>>>(a); break;
-                PCASE(PR_A) PCASE(PR_MUL) PCASE(PR_ADDMUL) PCASE(PR_MULMUL) PCASE(PR_SPEC) PCASE(PR_SPECT)
-#undef PCASE
-            }
-            break;
-        case OP_D2: set_smem<k_d2fd2<S, YT, CYC, T>>(smem); k_d2fd2<S, YT, CYC, T><<<grid, block, smem, st>>>(a); break;
-        case OP_FILTER:
-            if constexpr (sizeof(T) == 8) {   // the compact filter acts on the FP64 state only
-                set_smem<k_filter<S, YT, CYC, T>>(smem); k_filter<S, YT, CYC, T><<<grid, block, smem, st>>>(a);
-            }
-            break;
-        case OP_GAUSS: set_smem<k_gauss<S, YT, CYC, T>>(smem); k_gauss<S, YT, CYC, T><<<grid, block, smem, st>>>(a); break;
+// One launch: fields in[0..NIN-1], outputs out[0..NOUT-1] (a.red set), the
+// operations' arguments in a.op; name and bytes for the timing report.
+template <class R, int S, int M, int L, bool YT, bool CYC, class T>
+static int launch_lines(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *const *out, const char *name) {
+    using V = typename Val<T>::V;
+    constexpr int NL = L * Val<T>::W;
+    const int n = a.n;
+    const size_t nlines = c->dm.n3 / (size_t)n;              // lines of one case
+    a.cblk = (int)(nlines / NL);
+    a.ntile = a.cblk * c->na;
+    a.jb = c->dm.n[1] / NL;
+    a.box = n <= 256 ? n : n / 2;
+    a.wait_flag = c->wait_flag_dev;
+    a.tb = (unsigned)n * 8 * L;
+    using I = RecipeInfo<R>;
+    double fields = R::NIN;
+    for (int k = 0; k < R::NIN; k++) {
+        ST_TRY(line_map(c, &a.in[k], in[k], sizeof(T) == 4, a.dir, NL, a.box));
     }
+    for (int k = 0; k < I::stores(); k++) {
+        ST_TRY(line_map(c, &a.out[k], out[k], sizeof(T) == 4, a.dir, NL, a.box));
+        fields += a.red[k] ? 2 : 1;
+    }
+    // Slots and CTAs per SM: two slots or more per CTA, so that a tile's
+    // transfers overlap another's solve, in as many CTAs as the registers
+    // (80 a thread) and the shared memory hold; one slot in two CTAs where
+    // two slots do not fit.
+    const unsigned slot = R::NT * a.tb, tail = carry_bytes<V, L>(a.P * M) +
+                          (std::is_same<R, RecFilterM>::value ? 2u * carry_one<V, L>(a.P * M) : 0u) +
+                          (a.p.id ? pen_bytes(a.p, a.P * M, S / M) : 0u);
+    const int threads = L * a.P;
+    const int by_regs = 65536 / (80 * ((threads + 31) / 32 * 32));
+    auto fit = [&](int ctas) { return ((long)(c->smem_sm / ctas) - 1024 - (long)tail) / (long)slot; };   // slots
+    int ctas = 1, K = 1;
+    const int want = R::NT >= 3 ? 2 : 3;
+    for (int q = by_regs < 8 ? by_regs : 8; q >= 1; q--) {
+        const long f = fit(q);
+        if (f >= 2 || (q == 2 && f == 1 && fit(1) < 3) || q == 1) { ctas = q; K = f > want ? want : (int)f; break; }
+    }
+    if (K < 1) return fail(c, ST_E_UNSUPPORTED, "line tile does not fit in shared memory");
+    a.K = K;
+    const size_t smem = (size_t)K * slot + tail;
+    long grid = (long)c->sms * ctas;
+    if (grid > a.ntile) grid = a.ntile;
+    int pi = prof_start(c, name, fields * sizeof(T) * (double)c->ncell());
+    constexpr auto kern = k_lines<R, S, M, L, YT, CYC, T>;
+    set_smem<kern>(smem);
+    kern<<<(unsigned)grid, threads, smem, c->stream>>>(a);
     prof_stop(c, pi);
+    ST_CUDA(c, cudaGetLastError());
+    return ST_OK;
 }
 
-template <int S, bool CYC, class T>
-static void launch_S(st_ctx *c, OpKind op, const LineArgsT<T> &a, cudaStream_t st) {
-    if (a.geo.dir == 1) launch_SY<S, true, CYC, T>(c, op, a, st);
-    else launch_SY<S, false, CYC, T>(c, op, a, st);
+// 16 columns where the recipe's tiles fit, 8 otherwise (only recipes of four
+// tiles, on lines of more than 432 rows, which have segments of 16 rows)
+template <class R, int S, int M, bool CYC, class T>
+static int launch_lines_L(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *const *out, const char *name) {
+    a.P = a.n / S;
+    if constexpr (R::NT == 4 && S == 16 && M == 1) {
+        if (4L * 128 * a.n + carry_bytes<typename Val<T>::V, 16>(a.P) > c->smem_cta) {
+            if (a.dir == 1) return launch_lines<R, S, M, 8, true, CYC, T>(c, a, in, out, name);
+            return launch_lines<R, S, M, 8, false, CYC, T>(c, a, in, out, name);
+        }
+    }
+    if (a.dir == 1) return launch_lines<R, S, M, 16, true, CYC, T>(c, a, in, out, name);
+    return launch_lines<R, S, M, 16, false, CYC, T>(c, a, in, out, name);
 }
 
-// all line-operator launches of one family (CYC: periodic lines)
+// recipe by number
+enum RecId { R_D1, R_MUL, R_ADDMUL, R_MULMUL, R_HMULADD, R_SPEC, R_SPECT, R_D2, R_D2D1, R_FILTER, R_GAUSS, R_LAP,
+             R_PAIRA, R_PAIRB, R_PAIRC, R_PAIRD, R_PAIRE };
+
+template <int S, int M, bool CYC, class T>
+static int launch_rec_S(st_ctx *c, RecId id, LineArgsT<T> &a, const T *const *in, T *const *out) {
+    switch (id) {
+#define REC(id_, rec_, name_) case id_: return launch_lines_L<rec_, S, M, CYC, T>(c, a, in, out, name_);
+        REC(R_D1, RecD1, "k_dfd") REC(R_MUL, RecMul, "k_dfd") REC(R_ADDMUL, RecAddMul, "k_dfd")
+        REC(R_MULMUL, RecMulMul, "k_dfd")
+        case R_HMULADD:
+            return launch_lines_L<std::conditional_t<sizeof(T) == 8, RecHMulAdd, RecMulPlus>, S, M, CYC, T>(c, a, in, out, "k_dfd");
+        REC(R_D2, RecD2, "k_d2fd2") REC(R_D2D1, RecD2D1, "k_d2fd2") REC(R_GAUSS, RecGauss, "k_gauss")
+        REC(R_PAIRA, RecPairA, "k_dfd_pair") REC(R_PAIRB, RecPairB, "k_dfd_pair")
+        REC(R_PAIRD, RecPairD, "k_dfd_pair") REC(R_PAIRE, RecPairE, "k_dfd_pair")
+        case R_FILTER:
+            if constexpr (sizeof(T) == 8) return launch_lines_L<RecFilter, S, M, CYC, T>(c, a, in, out, "k_filter");
+            break;                    // the compact filter acts on the FP64 state only
+        // the species terms and the first-derivative Laplacian exist in the _mf family only
+        case R_SPEC: if constexpr (!CYC) return launch_lines_L<RecSpec, S, M, CYC, T>(c, a, in, out, "k_dfd"); break;
+        case R_SPECT: if constexpr (!CYC) return launch_lines_L<RecSpecT, S, M, CYC, T>(c, a, in, out, "k_dfd"); break;
+        case R_PAIRC: if constexpr (!CYC) return launch_lines_L<RecPairC, S, M, CYC, T>(c, a, in, out, "k_dfd_pair"); break;
+        case R_LAP: if constexpr (!CYC) return launch_lines_L<RecLap, S, M, CYC, T>(c, a, in, out, "k_lap"); break;
+#undef REC
+    }
+    return fail(c, ST_E_UNSUPPORTED, "line operation not available in this mode");
+}
+
+// all line-operator launches of one family and type: rows per thread from the
+// direction's segments (one per thread for doubles, up to four for floats)
 template <bool CYC, class T>
-static int launch_line_t(st_ctx *c, OpKind op, const LineArgsT<T> &a) {
-    switch (a.S) {
-#define CASE(s_) case s_: launch_S<s_, CYC, T>(c, op, a, c->stream); break;
-        CASE(2) CASE(3) CASE(4) CASE(6) CASE(8) CASE(12) CASE(16)
-#undef CASE
-        default: return fail(c, ST_E_UNSUPPORTED, "unsupported line segmentation");
-    }
-    ST_CUDA(c, cudaGetLastError());
-    return ST_OK;
-}
-
-
-// one launch of a pair (bounded lines), producers as in kPairOps;
-// bytes: algorithmic bytes per cell (every distinct field read or written once)
-template <int S, bool YT, class T, int OP0, int OP1>
-static void launch_pair_SY(st_ctx *c, const D1PairT<T> &g0, double bytes, cudaStream_t st) {
-    const size_t nlines = c->dm.n3 / (size_t)g0.a.geo.n;   // lines of one case
-    constexpr int NL = kLanes * Val<T>::W;
-    D1PairT<T> g = g0;
-    g.a.geo.cblk = (unsigned)(nlines / NL);                  // CTAs per case
-    g.a.geo.cstride = c->dm.n3;
-    dim3 grid(g.a.geo.cblk * (unsigned)c->na), block(kLanes * g.a.P);
-    const size_t smem = YT ? (size_t)NL * (g.a.geo.n + 1) * sizeof(T) : 0;
-    int pi = prof_start(c, "k_dfd_pair", bytes * (double)c->ncell());
-    set_smem<k_dfd_pair<S, YT, T, OP0, OP1>>(smem);
-    k_dfd_pair<S, YT, T, OP0, OP1><<<grid, block, smem, st>>>(g);
-    prof_stop(c, pi);
-}
-
-// the producer pairs compiled (first, second); pair_kind gives the index
-constexpr int kPairOps[][2] = {{PR_A, PR_MUL},   {PR_MUL, PR_MULMUL}, {PR_SPEC, PR_SPECT},
-                               {PR_MUL, PR_ADDMUL}, {PR_MUL, PR_A},    {PR_MUL, PR_MUL}};
-inline int pair_kind(int op0, int op1) {
-    for (int k = 0; k < (int)(sizeof(kPairOps) / sizeof(kPairOps[0])); k++)
-        if (kPairOps[k][0] == op0 && kPairOps[k][1] == op1) return k;
-    return -1;
-}
-
-template <int S, bool YT, class T>
-static void launch_pair_SYT(st_ctx *c, const D1PairT<T> &g, double bytes) {
-    switch (pair_kind(g.op[0].F.op, g.op[1].F.op)) {
-        case 0: launch_pair_SY<S, YT, T, PR_A, PR_MUL>(c, g, bytes, c->stream); break;
-        case 1: launch_pair_SY<S, YT, T, PR_MUL, PR_MULMUL>(c, g, bytes, c->stream); break;
-        case 2: launch_pair_SY<S, YT, T, PR_SPEC, PR_SPECT>(c, g, bytes, c->stream); break;
-        case 3: launch_pair_SY<S, YT, T, PR_MUL, PR_ADDMUL>(c, g, bytes, c->stream); break;
-        case 4: launch_pair_SY<S, YT, T, PR_MUL, PR_A>(c, g, bytes, c->stream); break;
-        default: launch_pair_SY<S, YT, T, PR_MUL, PR_MUL>(c, g, bytes, c->stream); break;
+static int launch_rec_t(st_ctx *c, RecId id, LineArgsT<T> &a, const T *const *in, T *const *out) {
+    if constexpr (sizeof(T) == 8) {
+        if (id == R_FILTER && fp32_mode(c)) {
+            switch (c->segf[a.dir]) {
+#define SEG(s_, st_, m_) case s_: return launch_lines_L<RecFilterM, st_, m_, CYC, T>(c, a, in, out, "k_filter");
+                SEG(2, 8, 4) SEG(3, 12, 4) SEG(4, 16, 4) SEG(6, 12, 2) SEG(8, 16, 2) SEG(12, 12, 1) SEG(16, 16, 1)
+#undef SEG
+            }
+            return fail(c, ST_E_UNSUPPORTED, "unsupported line segmentation");
+        }
+        return c->seg[a.dir] == 8 ? launch_rec_S<8, 1, CYC, T>(c, id, a, in, out) : launch_rec_S<16, 1, CYC, T>(c, id, a, in, out);
+    } else {
+        switch (c->segf[a.dir]) {
+            case 2: return launch_rec_S<8, 4, CYC, T>(c, id, a, in, out);
+            case 3: return launch_rec_S<12, 4, CYC, T>(c, id, a, in, out);
+            case 4: return launch_rec_S<16, 4, CYC, T>(c, id, a, in, out);
+            case 6: return launch_rec_S<12, 2, CYC, T>(c, id, a, in, out);
+            case 8: return launch_rec_S<16, 2, CYC, T>(c, id, a, in, out);
+            case 12: return launch_rec_S<12, 1, CYC, T>(c, id, a, in, out);
+            default: return launch_rec_S<16, 1, CYC, T>(c, id, a, in, out);
+        }
     }
 }
 
-template <class T>
-static int launch_pair_t(st_ctx *c, const D1PairT<T> &g, double bytes) {
-    switch (g.a.S) {
-#define CASE(s_)                                                       \
-    case s_:                                                           \
-        if (g.a.geo.dir == 1) launch_pair_SYT<s_, true, T>(c, g, bytes); \
-        else launch_pair_SYT<s_, false, T>(c, g, bytes);                 \
-        break;
-        CASE(2) CASE(3) CASE(4) CASE(6) CASE(8) CASE(12) CASE(16)
-#undef CASE
-        default: return fail(c, ST_E_UNSUPPORTED, "unsupported line segmentation");
-    }
-    ST_CUDA(c, cudaGetLastError());
-    return ST_OK;
-}
-
-// launches of the other instantiations, each in its own translation unit:
-// periodic lines (st_kernels_cyc.cu), FP32 fields (st_kernels_f32.cu) and
-// both (st_kernels_cyc_f32.cu)
-int launch_line_cyc(st_ctx *c, OpKind op, const LineArgs &a);
-int launch_line_f32(st_ctx *c, OpKind op, const LineArgsF &a);
-int launch_line_cyc_f32(st_ctx *c, OpKind op, const LineArgsF &a);
+// the instantiations, each in its own translation unit: bounded lines
+// (st_kernels.cu), periodic lines (st_kernels_cyc.cu), FP32 fields
+// (st_kernels_f32.cu) and both (st_kernels_cyc_f32.cu)
+int launch_rec(st_ctx *c, RecId id, LineArgs &a, const double *const *in, double *const *out);
+int launch_rec_cyc(st_ctx *c, RecId id, LineArgs &a, const double *const *in, double *const *out);
+int launch_rec_f32(st_ctx *c, RecId id, LineArgsF &a, const float *const *in, float *const *out);
+int launch_rec_cyc_f32(st_ctx *c, RecId id, LineArgsF &a, const float *const *in, float *const *out);
 
 }  // namespace st

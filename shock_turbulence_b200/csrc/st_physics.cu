@@ -55,6 +55,12 @@ template <class R>
 static ProdT<R> pr_mulmul(const R *a, const R *b, const R *c) {
     ProdT<R> p{}; p.op = PR_MULMUL; p.a = a; p.b = b; p.c = c; return p;
 }
+// a*b/2 + c: a momentum flux taken with the factor -1/2 and the pressure taken
+// with -1 along the same direction are one derivative (with -1) of this sum
+template <class R>
+static ProdT<R> pr_hmuladd(const R *a, const R *b, const R *c) {
+    ProdT<R> p{}; p.op = PR_HMULADD; p.a = a; p.b = b; p.c = c; return p;
+}
 
 // Line operators by field type: double arrays, or float arrays in the FP32
 // mode (the kernels compute in double either way; only storage differs).
@@ -76,20 +82,11 @@ static int d2fd2(st_ctx *c, int dir, int asym, const double *F, double *dF, doub
 static int d2fd2(st_ctx *c, int dir, int asym, const float *F, float *dF, float *d2F, int iadd) {
     return dev_d2fd2_f(c, dir, asym, F, dF, d2F, iadd);
 }
-static int dfd_sum(st_ctx *c, int dir, int asym, const double *F, double *dF, const double *E1,
-                   const double *E2) {
-    return dev_dfd_sum(c, dir, asym, F, dF, E1, E2);
+static int lap(st_ctx *c, int dir, const double *F, double *out, int iadd, bool second) {
+    return dev_lap(c, dir, F, out, iadd, second);
 }
-static int dfd_sum(st_ctx *c, int dir, int asym, const float *F, float *dF, const float *E1, const float *E2) {
-    return dev_dfd_sum_f(c, dir, asym, F, dF, E1, E2);
-}
-static int d2fd2_sum(st_ctx *c, int dir, int asym, const double *F, double *d2F, const double *E1,
-                     const double *E2) {
-    return dev_d2fd2_sum(c, dir, asym, F, d2F, E1, E2);
-}
-static int d2fd2_sum(st_ctx *c, int dir, int asym, const float *F, float *d2F, const float *E1,
-                     const float *E2) {
-    return dev_d2fd2_sum_f(c, dir, asym, F, d2F, E1, E2);
+static int lap(st_ctx *c, int dir, const float *F, float *out, int iadd, bool second) {
+    return dev_lap_f(c, dir, F, out, iadd, second);
 }
 // two first derivatives of one direction in order (producer, output, asym,
 // iadd[, cadd] of each; cadd 1 where not given), one launch where they share
@@ -248,12 +245,12 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
         mu[p] = m;
         dmu[p] = dm;
     });
-    // adjacent fluxes sharing u (or the second adding dP/dx to what the first
-    // wrote) run as pairs, in the reference's order
+    // adjacent fluxes sharing u run as pairs, in the reference's order; the
+    // flux that the pressure gradient adds to takes the pressure along
     const R *cu = u, *cv = v, *cw = w, *cP = P;
     ST_TRY(dfd_pair<R>(c, 0, pr_mul(q4r, cu), Qcx + 3 * n3, 1, 0, -1.0, pr_addmul(q5r, cP, cu), Qcx + 4 * n3, 1, 0,
                        -1.0));
-    ST_TRY(dfd_pair<R>(c, 0, pr_mul(q1r, cu), Qcx, 0, 0, -5.0e-1, pr_one(cP), Qcx, 0, 1, -1.0));
+    ST_TRY(dfd(c, 0, 0, pr_hmuladd(q1r, cu, cP), Qcx, 0, -1.0));
     ST_TRY(dfd_pair<R>(c, 0, pr_mul(q2r, cu), Qcx + n3, 1, 0, -5.0e-1, pr_mul(q3r, cu), Qcx + 2 * n3, 1, 0,
                        -5.0e-1));
     ST_TRY(dfd(c, 0, 1, q1r, FF, 0, 1.0));
@@ -302,12 +299,12 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
     // d(rho v)/dy and d(rho w)/dz with iadd=0, cadd=-1: Qconv(4) = 0 - d(.) exactly
     ST_TRY(dfd(c, 1, 1, q2r, Qcy + 3 * n3, 0, -1.0));
     ST_TRY(dfd(c, 1, 1, pr_mul(q1r, v), Qcy, 0, -5.0e-1));
-    ST_TRY(dfd_pair<R>(c, 1, pr_mul(q2r, cv), Qcy + n3, 0, 0, -5.0e-1, pr_one(cP), Qcy + n3, 0, 1, -1.0));
+    ST_TRY(dfd(c, 1, 0, pr_hmuladd(q2r, cv, cP), Qcy + n3, 0, -1.0));
     ST_TRY(dfd_pair<R>(c, 1, pr_mul(q3r, cv), Qcy + 2 * n3, 1, 0, -5.0e-1, pr_addmul(q5r, cP, cv), Qcy + 4 * n3, 1,
                        0, -1.0));
     ST_TRY(dfd(c, 2, 1, q3r, Qcz + 3 * n3, 0, -1.0));
     ST_TRY(dfd_pair<R>(c, 2, pr_mul(q1r, cw), Qcz, 1, 0, -5.0e-1, pr_mul(q2r, cw), Qcz + n3, 1, 0, -5.0e-1));
-    ST_TRY(dfd_pair<R>(c, 2, pr_mul(q3r, cw), Qcz + 2 * n3, 0, 0, -5.0e-1, pr_one(cP), Qcz + 2 * n3, 0, 1, -1.0));
+    ST_TRY(dfd(c, 2, 0, pr_hmuladd(q3r, cw, cP), Qcz + 2 * n3, 0, -1.0));
     ST_TRY(dfd(c, 2, 1, pr_addmul(q5r, P, w), Qcz + 4 * n3, 0, -1.0));
     R *d2Ty = dd[0], *d2Tz = dd[1], *d2uy = dd[2], *d2vy = dd[3], *d2wy = dd[4], *d2wz = dd[5];
     R *dGzz_y = dd[6], *d2uz = dd[7], *d2vz = dd[8], *dGxx_y = dd[9], *dGxx_z = dd[10], *dGyx_y = dd[11];
@@ -451,22 +448,14 @@ static int gaussian_filter_t(st_ctx *c, const R *F, R *Fg, int nvar) {
 // Compute_Laplacian src/hyper_dynamic_sym_mf.f:41-65
 template <class R>
 static int laplacian(st_ctx *c, const R *S, R *d2S) {
-    ScratchT<R> dS(c), t1(c), t2(c);
-    R *pt1 = t1, *pt2 = t2;
-    if (c->p.family == ST_FAMILY_PERIODIC) {
-        // Compute_Laplacian src/hyper_dynamic.f:41-58 (second derivatives)
-        ST_TRY(d2fd2(c, 0, 0, S, (R *)nullptr, (R *)t1, 0));
-        ST_TRY(d2fd2(c, 1, 0, S, (R *)nullptr, (R *)t2, 0));
-        // d2S = d2S + t1 + t2 in the z pass's store
-        return d2fd2_sum(c, 2, 0, S, d2S, (const R *)pt1, (const R *)pt2);
-    }
-    ST_TRY(dfd(c, 0, 0, S, (R *)dS, 0, 1.0));
-    ST_TRY(dfd(c, 0, 1, (const R *)dS, (R *)t1, 0, 1.0));
-    ST_TRY(dfd(c, 1, 0, S, (R *)dS, 0, 1.0));
-    ST_TRY(dfd(c, 1, 1, (const R *)dS, (R *)t2, 0, 1.0));
-    ST_TRY(dfd(c, 2, 0, S, (R *)dS, 0, 1.0));
-    // d2S = d2S + temp1 + temp2 (src/hyper_dynamic_sym_mf.f:61) in the z pass's store
-    return dfd_sum(c, 2, 1, (const R *)dS, d2S, (const R *)pt1, (const R *)pt2);
+    // each direction is one pass: both first derivatives of the _mf family,
+    // or the periodic family's second derivative (src/hyper_dynamic.f:41-58).
+    // d2S = d2S + temp1 + temp2 (z, x, y; src/hyper_dynamic_sym_mf.f:61) is
+    // accumulated by the passes in that order.
+    const bool second = c->p.family == ST_FAMILY_PERIODIC;
+    ST_TRY(lap(c, 2, S, d2S, 0, second));
+    ST_TRY(lap(c, 0, S, d2S, 1, second));
+    return lap(c, 1, S, d2S, 1, second);
 }
 
 // Compute_hyper src/hyper_dynamic_sym_mf.f:166-334 (+ Compute_coeff1 :79-158,
@@ -1110,7 +1099,7 @@ int dev_compute_cfl(st_ctx *c, const double *Q, bool to_host, double *stab, doub
     ST_CUDA(c, cudaGetLastError());
     if (to_host) {
         ST_CUDA(c, cudaMemcpyAsync(c->hpinned, c->dscal, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        ST_CUDA(c, cudaStreamSynchronize(c->stream));
+        ST_TRY(sync_stream(c));
         if (stab) *stab = c->hpinned[0];
         if (resv) *resv = c->hpinned[1];
         c->last_cfl_stab = c->hpinned[0];
@@ -1394,7 +1383,7 @@ int dev_monitors(st_ctx *c) {
     ST_CUDA(c, cudaGetLastError());
     std::vector<double> h(8 * nb);
     ST_CUDA(c, cudaMemcpyAsync(h.data(), part, 8 * nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(c, cudaStreamSynchronize(c->stream));
+    ST_TRY(sync_stream(c));
     double s[8] = {0};
     for (int k = 0; k < 8; k++) for (int b = 0; b < nb; b++) s[k] += h[(size_t)k * nb + b];
     const double N = (double)(c->dm.n[0] * c->dm.n[1] * c->dm.n[2]);

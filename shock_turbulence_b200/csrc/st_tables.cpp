@@ -26,6 +26,15 @@ namespace st {
 static const double kTiny = (double)FLT_MIN;   // tiny(1.0), src/tridiagonal.f90:275
 
 int choose_seg(int n) {
+    if (n < 2 * 8 || n % 16 != 0 || n > kMaxSeg * kMaxRows) return 0;
+    // Longer segments mean fewer halo rows and carries per row, shorter ones
+    // more threads and shorter chains.  Measured (256^3 and 64^3, filter /
+    // first / second derivative, us): 16 rows 102 / 76 / 131 and 22.8 / 23.6 /
+    // 26.8, 8 rows 192 / 87 / 136 and 23.1 / 22.9 / 25.2; they cross at 96.
+    return n < 96 ? 8 : 16;
+}
+
+int choose_seg_f(int n) {
     static const int sup[] = {2, 3, 4, 6, 8, 12, 16};
     for (int S : sup)
         if (n % S == 0 && n / S <= kMaxSeg) return S;
@@ -212,9 +221,8 @@ struct PenHost {
 };
 
 // The contiguous range [slo, shi) of segments around the middle one in which
-// every listed coefficient array holds, on every row, exactly (bitwise) its
-// value at the middle row; empty when the middle segment itself varies (the
-// antisymmetric filter's factorisation ends in a cycle, not a fixed point).
+// every listed coefficient array holds, on every row, its value at the middle
+// row (bitwise); empty when the middle segment itself varies.
 static void flat_segments(const std::vector<const std::vector<double> *> &arrs, int n, int S, int *slo,
                           int *shi) {
     const int P = n / S, mid = n / 2;
@@ -288,12 +296,12 @@ static TriHost tri_tables(const std::vector<double> &a, const std::vector<double
     t.kf = carry_span(t.wf, P, 1, true);
     t.kb = carry_span(t.wb, P, 1, false);
     flat_segments({&t.l, &t.up, &t.id}, n, S, &t.slo, &t.shi);
-    // scan factors: products of 2^k consecutive B ending at s and G starting
-    // at s; entries whose span leaves [0, P) stay 0 (never read)
-    t.sf.assign((size_t)kScanSteps * kMaxSeg, 0.0);
-    t.sb.assign((size_t)kScanSteps * kMaxSeg, 0.0);
+    // products of 2^k consecutive B ending at s and G starting at s; entries
+    // whose span leaves [0, P) stay 0 (never read)
+    t.sf.assign((size_t)5 * kMaxSeg, 0.0);
+    t.sb.assign((size_t)5 * kMaxSeg, 0.0);
     for (int s = 0; s < P; s++) { t.sf[s] = B[s]; t.sb[s] = G[s]; }
-    for (int k = 1, d = 1; k < kScanSteps; k++, d <<= 1)
+    for (int k = 1, d = 1; k < 5; k++, d <<= 1)
         for (int s = 0; s < P; s++) {
             if (s - d >= 0) t.sf[k * kMaxSeg + s] = t.sf[(k - 1) * kMaxSeg + s] * t.sf[(k - 1) * kMaxSeg + s - d];
             if (s + d < P) t.sb[k * kMaxSeg + s] = t.sb[(k - 1) * kMaxSeg + s] * t.sb[(k - 1) * kMaxSeg + s + d];
@@ -307,10 +315,17 @@ static void mat2mul(const double *A, const double *B, double *C) {  // C = A*B (
     std::memcpy(C, r, sizeof(r));
 }
 
-static PenHost pen_tables(std::vector<double> M[5], int n, int S) {
+// R: type of the factorisation.  This nearly singular system amplifies the
+// rounding of its factors, which in double need not settle on their interior
+// fixed point (and so on constants for the interior segments); in long double
+// they do.  The FP32 mode's filter takes the double factors, and (scan) the
+// products of 2^k consecutive segment matrices.
+template <class R>
+static PenHost pen_tables(std::vector<double> M[5], int n, int S, bool scan) {
     PenHost t;
-    std::vector<double> A = M[0], B = M[1], C = M[2], D = M[3], E = M[4];
-    std::vector<double> k1(n, 0.0), k2(n, 0.0);
+    std::vector<R> A(M[0].begin(), M[0].end()), B(M[1].begin(), M[1].end()), C(M[2].begin(), M[2].end()),
+        D(M[3].begin(), M[3].end()), E(M[4].begin(), M[4].end());
+    std::vector<R> k1(n, (R)0), k2(n, (R)0);
     for (int i = 0; i <= n - 3; i++) {
         k1[i] = B[i + 1] / (C[i] + kTiny);
         C[i + 1] = C[i + 1] - D[i] * k1[i];
@@ -319,16 +334,16 @@ static PenHost pen_tables(std::vector<double> M[5], int n, int S) {
         B[i + 2] = B[i + 2] - D[i] * k2[i];
         C[i + 2] = C[i + 2] - E[i] * k2[i];
     }
-    double k3 = B[n - 1] / (C[n - 2] + kTiny);
+    const R k3 = B[n - 1] / (C[n - 2] + kTiny);
     C[n - 1] = C[n - 1] - D[n - 2] * k3;
     t.p1.assign(n, 0.0); t.p2.assign(n, 0.0);
-    t.p1[1] = k1[0];
-    for (int i = 2; i <= n - 2; i++) { t.p1[i] = k1[i - 1]; t.p2[i] = k2[i - 2]; }
-    t.p1[n - 1] = k3; t.p2[n - 1] = k2[n - 3];
+    t.p1[1] = (double)k1[0];
+    for (int i = 2; i <= n - 2; i++) { t.p1[i] = (double)k1[i - 1]; t.p2[i] = (double)k2[i - 2]; }
+    t.p1[n - 1] = (double)k3; t.p2[n - 1] = (double)k2[n - 3];
     t.q1.assign(n, 0.0); t.q2.assign(n, 0.0); t.id.resize(n);
-    for (int i = 0; i <= n - 2; i++) t.q1[i] = D[i];
-    for (int i = 0; i <= n - 3; i++) t.q2[i] = E[i];
-    for (int i = 0; i < n; i++) t.id[i] = 1.0 / (C[i] + kTiny);
+    for (int i = 0; i <= n - 2; i++) t.q1[i] = (double)D[i];
+    for (int i = 0; i <= n - 3; i++) t.q2[i] = (double)E[i];
+    for (int i = 0; i < n; i++) t.id[i] = (double)((R)1.0 / (C[i] + kTiny));
     const int P = n / S;
     t.g1.assign(n, 0.0); t.g2.assign(n, 0.0); t.h1.assign(n, 0.0); t.h2.assign(n, 0.0);
     std::vector<double> Mseg(P * 4), Nseg(P * 4);
@@ -363,16 +378,15 @@ static PenHost pen_tables(std::vector<double> M[5], int n, int S) {
         }
     }
     flat_segments({&t.p1, &t.p2, &t.q1, &t.q2, &t.id}, n, S, &t.slo, &t.shi);
-    // scan factors: T_0(s) = M_s, T_{k+1}(s) = T_k(s) T_k(s-2^k);
-    // U_0(s) = N_s, U_{k+1}(s) = U_k(s) U_k(s+2^k); entries whose span leaves
-    // [0, P) stay 0 (never read)
-    t.sf.assign((size_t)kScanSteps * kMaxSeg * 4, 0.0);
-    t.sb.assign((size_t)kScanSteps * kMaxSeg * 4, 0.0);
-    for (int s = 0; s < P; s++) {
-        std::memcpy(&t.sf[(size_t)s * 4], &Mseg[s * 4], 32);
-        std::memcpy(&t.sb[(size_t)s * 4], &Nseg[s * 4], 32);
-    }
-    for (int k = 1, d = 1; k < kScanSteps; k++, d <<= 1)
+    t.sf = Mseg;
+    t.sb = Nseg;
+    if (!scan) return t;
+    // [5][kMaxSeg][4]: T_0(s) = M_s, T_{k+1}(s) = T_k(s) T_k(s-2^k); U_0(s) =
+    // N_s, U_{k+1}(s) = U_k(s) U_k(s+2^k); entries whose span leaves [0, P)
+    // stay 0 (never read)
+    t.sf.resize((size_t)5 * kMaxSeg * 4, 0.0);
+    t.sb.resize((size_t)5 * kMaxSeg * 4, 0.0);
+    for (int k = 1, d = 1; k < 5; k++, d <<= 1)
         for (int s = 0; s < P; s++) {
             if (s - d >= 0)
                 mat2mul(&t.sf[((size_t)(k - 1) * kMaxSeg + s) * 4], &t.sf[((size_t)(k - 1) * kMaxSeg + s - d) * 4],
@@ -382,6 +396,22 @@ static PenHost pen_tables(std::vector<double> M[5], int n, int S) {
                         &t.sb[((size_t)k * kMaxSeg + s) * 4]);
         }
     return t;
+}
+
+// The segments [clo, chi) around the middle one in which every weight of the
+// corner correction K ([n][k]) is below 1e-22, so that it cannot change a
+// result of the size of the solution.
+static void corner_range(const std::vector<double> &K, int k, int n, int S, int *clo, int *chi) {
+    const int P = n / S;
+    auto small = [&](int s) {
+        for (int q = s * S * k; q < (s + 1) * S * k; q++)
+            if (std::fabs(K[q]) >= 1e-22) return false;
+        return true;
+    };
+    int lo = P / 2, hi = P / 2;
+    while (lo > 0 && small(lo - 1)) lo--;
+    while (hi < P && small(hi)) hi++;
+    *clo = lo; *chi = hi;
 }
 
 static const double *upload(st_ctx *c, const std::vector<double> &v, int *err) {
@@ -403,31 +433,57 @@ static const float *upload_f(st_ctx *c, const std::vector<double> &v, int *err) 
     return (const float *)p;
 }
 
-// The FP32 mode's tridiagonal factors: the double tables rounded to float.
-// Carry weights below 1e-12 cannot change a float result of the size of the
-// solution (float epsilon 6e-8 times the few segment end values they scale).
-static void upload_tri(st_ctx *c, st::TriTab &t, st::TriTabT<float> &tf, const TriHost &h,
-                       const std::vector<double> *K, int P, int *err) {
+static void upload_tri(st_ctx *c, st::TriTab &t, const TriHost &h, const std::vector<double> *K, int P, int *err) {
+    const int n = (int)h.l.size(), S = n / P, mid = n / 2, row0 = mid / S * S;
     t.l = upload(c, h.l, err); t.g = upload(c, h.g, err); t.up = upload(c, h.up, err);
     t.id = upload(c, h.id, err); t.h = upload(c, h.h, err);
     t.wf = upload(c, h.wf, err); t.wb = upload(c, h.wb, err);
-    t.sf = upload(c, h.sf, err); t.sb = upload(c, h.sb, err);
+    t.sf = t.sb = nullptr;
     t.kf = h.kf; t.kb = h.kb;
     t.cyc = K ? upload(c, *K, err) : nullptr;
-    const int mid = (int)h.l.size() / 2;
+    if (K) corner_range(*K, 2, n, S, &t.clo, &t.chi);
     t.slo = h.slo; t.shi = h.shi;
     t.cl = h.l[mid]; t.cup = h.up[mid]; t.cid = h.id[mid];
-    tf = st::TriTabT<float>{};
-    tf.slo = h.slo; tf.shi = h.shi;
-    tf.cl = (float)t.cl; tf.cup = (float)t.cup; tf.cid = (float)t.cid;
-    if (c->p.precision != ST_PRECISION_FP32) return;
-    tf.l = upload_f(c, h.l, err); tf.g = upload_f(c, h.g, err); tf.up = upload_f(c, h.up, err);
-    tf.id = upload_f(c, h.id, err); tf.h = upload_f(c, h.h, err);
-    tf.wf = upload_f(c, h.wf, err); tf.wb = upload_f(c, h.wb, err);
-    tf.sf = upload_f(c, h.sf, err); tf.sb = upload_f(c, h.sb, err);
-    tf.kf = carry_span(h.wf, P, 1, true, 1e-12);
-    tf.kb = carry_span(h.wb, P, 1, false, 1e-12);
-    tf.cyc = K ? upload_f(c, *K, err) : nullptr;
+    for (int q = 0; q < S; q++) { t.cg[q] = h.g[row0 + q]; t.ch[q] = h.h[row0 + q]; }
+}
+// The FP32 mode's tridiagonal factors: the double ones rounded to float.
+// Carry weights below 1e-12 cannot change a float result of the size of the
+// solution (float epsilon 6e-8 times the few segment end values they scale).
+static void upload_tri(st_ctx *c, st::TriTabT<float> &t, const TriHost &h, const std::vector<double> *K, int P, int *err) {
+    const int n = (int)h.l.size(), S = n / P, mid = n / 2, row0 = mid / S * S;
+    t.l = upload_f(c, h.l, err); t.g = upload_f(c, h.g, err); t.up = upload_f(c, h.up, err);
+    t.id = upload_f(c, h.id, err); t.h = upload_f(c, h.h, err);
+    t.wf = upload_f(c, h.wf, err); t.wb = upload_f(c, h.wb, err);
+    t.sf = upload_f(c, h.sf, err); t.sb = upload_f(c, h.sb, err);
+    t.kf = carry_span(h.wf, P, 1, true, 1e-12);
+    t.kb = carry_span(h.wb, P, 1, false, 1e-12);
+    t.cyc = K ? upload_f(c, *K, err) : nullptr;
+    t.clo = t.chi = 0;      // every row is corrected
+    t.slo = h.slo; t.shi = h.shi;
+    t.cl = (float)h.l[mid]; t.cup = (float)h.up[mid]; t.cid = (float)h.id[mid];
+    for (int q = 0; q < S; q++) { t.cg[q] = (float)h.g[row0 + q]; t.ch[q] = (float)h.h[row0 + q]; }
+}
+
+static void upload_pen(st_ctx *c, st::PenTab &t, std::vector<double> M[5], const std::vector<double> *K, int n, int d, int *err) {
+    const bool f32 = c->p.precision == ST_PRECISION_FP32;
+    const int S = f32 ? c->segf[d] : c->seg[d];
+    const PenHost h = f32 ? pen_tables<double>(M, n, S, true) : pen_tables<long double>(M, n, S, false);
+    const int mid = n / 2, row0 = mid / S * S;
+    t.p1 = upload(c, h.p1, err); t.p2 = upload(c, h.p2, err);
+    t.g1 = upload(c, h.g1, err); t.g2 = upload(c, h.g2, err);
+    t.q1 = upload(c, h.q1, err); t.q2 = upload(c, h.q2, err);
+    t.id = upload(c, h.id, err); t.h1 = upload(c, h.h1, err); t.h2 = upload(c, h.h2, err);
+    t.sf = upload(c, h.sf, err); t.sb = upload(c, h.sb, err);
+    t.slo = h.slo; t.shi = h.shi;
+    t.cp1 = h.p1[mid]; t.cp2 = h.p2[mid]; t.cq1 = h.q1[mid]; t.cq2 = h.q2[mid]; t.cid = h.id[mid];
+    for (int q = 0; q < S; q++) {
+        t.cg1[q] = h.g1[row0 + q]; t.cg2[q] = h.g2[row0 + q];
+        t.ch1[q] = h.h1[row0 + q]; t.ch2[q] = h.h2[row0 + q];
+    }
+    for (int q = 0; q < 4; q++) { t.cm[q] = h.sf[mid / S * 4 + q]; t.cn[q] = h.sb[mid / S * 4 + q]; }
+    t.cyc = K ? upload(c, *K, err) : nullptr;
+    if (K && !f32) corner_range(*K, 4, n, S, &t.clo, &t.chi);
+    else t.clo = t.chi = 0;
 }
 
 // Periodic family: every derivative and filter kind of a direction gets the
@@ -447,26 +503,17 @@ static int build_tables_periodic(st_ctx *c) {
             std::vector<double> K = cyclic_correction(n, 0.0, al, 2);
             for (int asym = 0; asym < 2; asym++) {
                 const int kind = (order - 1) * 2 + asym;
-                upload_tri(c, c->tri[d][kind], c->trif[d][kind], h, &K, n / c->seg[d], &err);
+                upload_tri(c, c->tri[d][kind], h, &K, n / c->seg[d], &err);
+                if (c->p.precision == ST_PRECISION_FP32)
+                    upload_tri(c, c->trif[d][kind], tri_tables(M[1], M[2], M[3], n, c->segf[d]), &K, n / c->segf[d], &err);
             }
         }
         std::vector<double> M[5];
         band_rows(n, bf, af, M);
-        PenHost h = pen_tables(M, n, c->seg[d]);
         std::vector<double> K = cyclic_correction(n, bf, af, 4);
         for (int kind = 0; kind < 2; kind++) {
             PenTab &t = c->pen[d][kind];
-            t.p1 = upload(c, h.p1, &err); t.p2 = upload(c, h.p2, &err);
-            t.g1 = upload(c, h.g1, &err); t.g2 = upload(c, h.g2, &err);
-            t.q1 = upload(c, h.q1, &err); t.q2 = upload(c, h.q2, &err);
-            t.id = upload(c, h.id, &err); t.h1 = upload(c, h.h1, &err); t.h2 = upload(c, h.h2, &err);
-            t.sf = upload(c, h.sf, &err); t.sb = upload(c, h.sb, &err);
-            {
-                const int mid = n / 2;
-                t.slo = h.slo; t.shi = h.shi;
-                t.cp1 = h.p1[mid]; t.cp2 = h.p2[mid]; t.cq1 = h.q1[mid]; t.cq2 = h.q2[mid]; t.cid = h.id[mid];
-            }
-            t.cyc = upload(c, K, &err);
+            upload_pen(c, t, M, &K, n, d, &err);
         }
     }
     if (err) return fail(c, ST_E_NOMEM, "could not allocate or upload the LU tables");
@@ -482,24 +529,15 @@ int build_tables(st_ctx *c) {
             std::vector<double> a, b, cc;
             deriv_lhs(n, kind < 2 ? 1 : 2, kind & 1, a, b, cc);
             TriHost h = tri_tables(a, b, cc, n, c->seg[d]);
-            upload_tri(c, c->tri[d][kind], c->trif[d][kind], h, nullptr, n / c->seg[d], &err);
+            upload_tri(c, c->tri[d][kind], h, nullptr, n / c->seg[d], &err);
+            if (c->p.precision == ST_PRECISION_FP32)
+                upload_tri(c, c->trif[d][kind], tri_tables(a, b, cc, n, c->segf[d]), nullptr, n / c->segf[d], &err);
         }
         for (int kind = 0; kind < 2; kind++) {
             std::vector<double> M[5];
             filter_lhs(n, kind, M);
-            PenHost h = pen_tables(M, n, c->seg[d]);
-            PenTab &t = c->pen[d][kind];
-            t.p1 = upload(c, h.p1, &err); t.p2 = upload(c, h.p2, &err);
-            t.g1 = upload(c, h.g1, &err); t.g2 = upload(c, h.g2, &err);
-            t.q1 = upload(c, h.q1, &err); t.q2 = upload(c, h.q2, &err);
-            t.id = upload(c, h.id, &err); t.h1 = upload(c, h.h1, &err); t.h2 = upload(c, h.h2, &err);
-            t.sf = upload(c, h.sf, &err); t.sb = upload(c, h.sb, &err);
-            {
-                const int mid = n / 2;
-                t.slo = h.slo; t.shi = h.shi;
-                t.cp1 = h.p1[mid]; t.cp2 = h.p2[mid]; t.cq1 = h.q1[mid]; t.cq2 = h.q2[mid]; t.cid = h.id[mid];
-            }
-            t.cyc = nullptr;
+                PenTab &t = c->pen[d][kind];
+            upload_pen(c, t, M, nullptr, n, d, &err);
         }
     }
     if (err) return fail(c, ST_E_NOMEM, "could not allocate or upload the LU tables");
