@@ -402,6 +402,7 @@ int st_destroy(st_ctx *c) {
     for (float *a : c->hypf) if (a) cudaFree(a);
     for (float *a : c->dYdf) if (a) cudaFree(a);
     for (auto &e : c->pool) cudaFree(e.p);
+    if (c->solver_ws) cudaFree(c->solver_ws);
     if (c->hpinned) cudaFreeHost(c->hpinned);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
@@ -535,24 +536,48 @@ int st_set_common(st_ctx *c, const char *name, const double *in) {
 }
 
 // ---- line solvers --------------------------------------------------------------
+// Arrays on the context's device are used where they are; others, and a
+// right-hand side that overlaps a coefficient array (which the solve still
+// reads), go through the workspace.
+}  // extern "C"
+static int solve_lines(st_ctx *c, const double *const *co, int nco, double *R, int n, int lot, int nper) {
+    const bool pen = nco == 5;
+    const size_t N = (size_t)n * lot, bytes = N * 8;
+    bool move[6];
+    int fields = solver_fields(pen, nper);
+    for (int q = 0; q < nco; q++) fields += move[q] = !on_device(c, co[q]);
+    move[nco] = !on_device(c, R);
+    for (int q = 0; q < nco; q++)
+        if (!move[q] && co[q] < R + N && R < co[q] + N) move[nco] = true;
+    fields += move[nco];
+    double *ws = solver_workspace(c, (size_t)fields * bytes);
+    if (!ws) return fail(c, ST_E_NOMEM, "line solver workspace");
+    double *next = ws + (size_t)solver_fields(pen, nper) * N;
+    const double *a[6];
+    for (int q = 0; q <= nco; q++) {
+        const double *src = q < nco ? co[q] : R;
+        a[q] = src;
+        if (!move[q]) continue;
+        ST_CUDA(c, cudaMemcpyAsync(next, src, bytes, cudaMemcpyDefault, c->stream));
+        a[q] = next;
+        next += N;
+    }
+    double *Rd = const_cast<double *>(a[nco]);
+    const int rc = pen ? dev_pentadiagonal(c, a[0], a[1], a[2], a[3], a[4], Rd, ws, n, lot, nper)
+                       : dev_tridiagonal(c, a[0], a[1], a[2], Rd, ws, n, lot, nper);
+    if (rc == ST_OK && move[nco]) ST_CUDA(c, cudaMemcpyAsync(R, Rd, bytes, cudaMemcpyDefault, c->stream));
+    const int rs = sync_stream(c);
+    solver_workspace_trim(c);
+    return rc != ST_OK ? rc : rs;
+}
+extern "C" {
+
 int st_tridiagonal(st_ctx *c, const double *A, const double *B, const double *C, double *R, int n, int lot,
                    int nper) {
     if (!A || !B || !C || !R || n < 1 || lot < 1) return ST_E_ARG;
     API_BEGIN(c)
-    const size_t N = (size_t)n * lot, bytes = N * 8;
-    double *buf = nullptr;
-    ST_CUDA(c, cudaMalloc((void **)&buf, 4 * bytes));
-    double *dA = buf, *dB = buf + N, *dC = buf + 2 * N, *dR = buf + 3 * N;
-    const double *src[4] = {A, B, C, R};
-    double *dst[4] = {dA, dB, dC, dR};
-    for (int q = 0; q < 4; q++) cudaMemcpyAsync(dst[q], src[q], bytes, cudaMemcpyDefault, c->stream);
-    int rc = dev_tridiagonal(c, dA, dB, dC, dR, n, lot, nper);
-    if (rc == ST_OK) cudaMemcpyAsync(R, dR, bytes, cudaMemcpyDefault, c->stream);
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    cudaFree(buf);
-    if (rc != ST_OK) return rc;
-    if (e != cudaSuccess) return fail(c, ST_E_CUDA, cudaGetErrorString(e));
-    return ST_OK;
+    const double *co[3] = {A, B, C};
+    return solve_lines(c, co, 3, R, n, lot, nper);
     API_END(c)
 }
 
@@ -560,18 +585,8 @@ int st_pentadiagonal(st_ctx *c, const double *A, const double *B, const double *
                      const double *E, double *R, int n, int lot, int nper) {
     if (!A || !B || !C || !D || !E || !R || n < 1 || lot < 1) return ST_E_ARG;
     API_BEGIN(c)
-    const size_t N = (size_t)n * lot, bytes = N * 8;
-    double *buf = nullptr;
-    ST_CUDA(c, cudaMalloc((void **)&buf, 6 * bytes));
-    const double *src[6] = {A, B, C, D, E, R};
-    for (int q = 0; q < 6; q++) cudaMemcpyAsync(buf + q * N, src[q], bytes, cudaMemcpyDefault, c->stream);
-    int rc = dev_pentadiagonal(c, buf, buf + N, buf + 2 * N, buf + 3 * N, buf + 4 * N, buf + 5 * N, n, lot, nper);
-    if (rc == ST_OK) cudaMemcpyAsync(R, buf + 5 * N, bytes, cudaMemcpyDefault, c->stream);
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    cudaFree(buf);
-    if (rc != ST_OK) return rc;
-    if (e != cudaSuccess) return fail(c, ST_E_CUDA, cudaGetErrorString(e));
-    return ST_OK;
+    const double *co[5] = {A, B, C, D, E};
+    return solve_lines(c, co, 5, R, n, lot, nper);
     API_END(c)
 }
 

@@ -175,6 +175,8 @@ struct st_ctx {
     struct PoolEntry { void *p; size_t bytes; bool used; };
     std::vector<PoolEntry> pool;
     bool pool_oom = false;
+    void *solver_ws = nullptr;          // workspace of the general line solvers
+    size_t solver_ws_bytes = 0;
     // device scalars (reductions, dt)
     double *dscal = nullptr;     // [nb][kScal]
     double *hpinned = nullptr;   // pinned host mirror [nb][kScal]
@@ -288,10 +290,15 @@ int dev_gauss(st_ctx *c, int dir, const double *F, double *Fg);
 int dev_fill(st_ctx *c, double *x, size_t n, double v);
 int dev_to_float(st_ctx *c, const double *x, float *y, size_t n);
 int dev_to_double(st_ctx *c, const float *x, double *y, size_t n);
-int dev_tridiagonal(st_ctx *c, const double *A, const double *B, const double *C, double *R,
-                    int n, int lot, int nper);
-int dev_pentadiagonal(st_ctx *c, const double *A, const double *B, const double *C,
-                      const double *D, const double *E, double *R, int n, int lot, int nper);
+// general solvers (st_solvers.cu): coefficients read only, R solved in place,
+// ws: solver_fields() fields of n*lot values
+int solver_fields(bool pen, int nper);
+double *solver_workspace(st_ctx *c, size_t bytes);
+void solver_workspace_trim(st_ctx *c);
+int dev_tridiagonal(st_ctx *c, const double *A, const double *B, const double *C, double *R, double *ws, int n, int lot,
+                    int nper);
+int dev_pentadiagonal(st_ctx *c, const double *A, const double *B, const double *C, const double *D, const double *E, double *R,
+                      double *ws, int n, int lot, int nper);
 
 // physics on device arrays (st_physics.cu)
 int dev_compute_gamma(st_ctx *c, const double *Y);

@@ -1,6 +1,6 @@
 // st_kernels.cu - compact derivative, compact filter and Gaussian filter line
 // operators (bounded-line instantiations and the entry points of both
-// families), and the general (per-line coefficient) tri/pentadiagonal solvers.
+// families).
 #include <initializer_list>
 #include "st_linekern.cuh"
 
@@ -215,210 +215,5 @@ static int dfd_pair_t(st_ctx *c, int dir, const D1SpecT<T> *ops) {
 
 int dev_dfd_pair(st_ctx *c, int dir, const D1SpecT<double> *ops) { return dfd_pair_t(c, dir, ops); }
 int dev_dfd_pair_f(st_ctx *c, int dir, const D1SpecT<float> *ops) { return dfd_pair_t(c, dir, ops); }
-
-// ---- general solvers (per-line coefficients), thread per line ---------------
-// tridiagonal_serial / tridiagonal_periodic_serial, src/tridiagonal.f90:197-287.
-// Arrays (lot,n) with lot fastest; A,B,C are copied into scratch first (the
-// reference's A=A1; B=B1; C=C1).
-__global__ void k_tri_general(double *a, double *b, const double *cc, double *R, int n, int lot,
-                              int nper) {
-    int L = blockIdx.x * blockDim.x + threadIdx.x;
-    if (L >= lot) return;
-    const double tiny = (double)FLT_MIN;
-#define A_(i) a[(size_t)(i) * lot + L]
-#define B_(i) b[(size_t)(i) * lot + L]
-#define C_(i) cc[(size_t)(i) * lot + L]
-#define R_(i) R[(size_t)(i) * lot + L]
-    if (nper == 0) {
-        for (int i = 1; i < n; i++) {
-            double cs = A_(i) / (B_(i - 1) + tiny);
-            B_(i) = B_(i) - C_(i - 1) * cs;
-            R_(i) = R_(i) - R_(i - 1) * cs;
-        }
-        R_(n - 1) = R_(n - 1) / B_(n - 1);
-        for (int i = n - 2; i >= 0; i--) R_(i) = (R_(i) - C_(i) * R_(i + 1)) / (B_(i) + tiny);
-        return;
-    }
-    double c0 = C_(0);
-    if (n == 1) { R_(0) = R_(0) / (A_(0) + B_(0) + C_(0)); return; }
-    if (n == 2) {
-        c0 = C_(0) + A_(0);
-        A_(1) = A_(1) + C_(1);
-        double cs = A_(1) / B_(0);
-        B_(1) = B_(1) - c0 * cs;
-        R_(1) = R_(1) - R_(0) * cs;
-        R_(1) = R_(1) / B_(1);
-        R_(0) = (R_(0) - c0 * R_(1)) / B_(0);
-        return;
-    }
-    for (int i = 1; i <= n - 3; i++) {
-        double cs = A_(i) / B_(i - 1);
-        B_(i) = B_(i) - C_(i - 1) * cs;
-        R_(i) = R_(i) - R_(i - 1) * cs;
-        A_(i) = -A_(i - 1) * cs;
-    }
-    int i = n - 2;
-    double cs = A_(i) / B_(i - 1);
-    B_(i) = B_(i) - C_(i - 1) * cs;
-    R_(i) = R_(i) - R_(i - 1) * cs;
-    A_(i) = C_(i) - A_(i - 1) * cs;
-    i = n - 1;
-    cs = A_(i) / B_(i - 1);
-    R_(i) = R_(i) - R_(i - 1) * cs;
-    A_(i) = B_(i) - A_(i - 1) * cs;
-    for (i = n - 3; i >= 0; i--) {
-        cs = C_(i) / B_(i + 1);
-        R_(i) = R_(i) - R_(i + 1) * cs;
-        A_(i) = A_(i) - A_(i + 1) * cs;
-    }
-    cs = C_(n - 1) / B_(0);
-    R_(n - 1) = R_(n - 1) - R_(0) * cs;
-    A_(n - 1) = A_(n - 1) - A_(0) * cs;
-    R_(n - 1) = R_(n - 1) / A_(n - 1);
-    for (i = n - 2; i >= 0; i--) R_(i) = (R_(i) - A_(i) * R_(n - 1)) / B_(i);
-#undef A_
-#undef B_
-#undef C_
-#undef R_
-}
-
-// pentadiagonal_serial / pentadiagonal_periodic_serial,
-// src/pentadiagonal.f90:319-504 (n >= 5 for the periodic path)
-__global__ void k_pen_general(double *A, double *B, double *C, double *D, double *E, double *R,
-                              double *s1, double *s2, int n, int lot, int nper) {
-    int L = blockIdx.x * blockDim.x + threadIdx.x;
-    if (L >= lot) return;
-    const double tiny = (double)FLT_MIN;
-#define X_(arr, i) arr[(size_t)(i) * lot + L]
-    if (nper == 0) {
-        if (n == 1) { X_(R, 0) = X_(R, 0) / X_(C, 0); return; }
-        if (n == 2) {
-            double cs = X_(B, 1) / X_(C, 0);
-            X_(C, 1) = X_(C, 1) - X_(D, 0) * cs;
-            X_(R, 1) = X_(R, 1) - X_(R, 0) * cs;
-            X_(R, 1) = X_(R, 1) / X_(C, 1);
-            X_(R, 0) = (X_(R, 0) - X_(D, 0) * X_(R, 1)) / X_(C, 0);
-            return;
-        }
-        for (int i = 0; i <= n - 3; i++) {
-            double cs = X_(B, i + 1) / (X_(C, i) + tiny);
-            X_(C, i + 1) = X_(C, i + 1) - X_(D, i) * cs;
-            X_(D, i + 1) = X_(D, i + 1) - X_(E, i) * cs;
-            X_(R, i + 1) = X_(R, i + 1) - X_(R, i) * cs;
-            cs = X_(A, i + 2) / (X_(C, i) + tiny);
-            X_(B, i + 2) = X_(B, i + 2) - X_(D, i) * cs;
-            X_(C, i + 2) = X_(C, i + 2) - X_(E, i) * cs;
-            X_(R, i + 2) = X_(R, i + 2) - X_(R, i) * cs;
-        }
-        double cs = X_(B, n - 1) / (X_(C, n - 2) + tiny);
-        X_(C, n - 1) = X_(C, n - 1) - X_(D, n - 2) * cs;
-        X_(R, n - 1) = X_(R, n - 1) - X_(R, n - 2) * cs;
-        X_(R, n - 1) = X_(R, n - 1) / (X_(C, n - 1) + tiny);
-        X_(R, n - 2) = (X_(R, n - 2) - X_(D, n - 2) * X_(R, n - 1)) / (X_(C, n - 2) + tiny);
-        for (int i = n - 3; i >= 0; i--)
-            X_(R, i) = (X_(R, i) - X_(D, i) * X_(R, i + 1) - X_(E, i) * X_(R, i + 2)) / (X_(C, i) + tiny);
-        return;
-    }
-    for (int i = 0; i < n; i++) { X_(s1, i) = 0.0; X_(s2, i) = 0.0; }
-    if (n == 4) for (int i = 0; i < 4; i++) { X_(A, i) = X_(A, i) + X_(E, i); X_(E, i) = 0.0; }
-    X_(s1, 0) = X_(A, 0);
-    X_(s1, n - 4) = X_(s1, n - 4) + X_(E, n - 4);
-    X_(s1, n - 3) = X_(D, n - 3);
-    X_(s1, n - 2) = X_(C, n - 2);
-    X_(s1, n - 1) = X_(B, n - 1);
-    X_(s2, 0) = X_(B, 0);
-    X_(s2, 1) = X_(A, 1);
-    X_(s2, n - 3) = X_(s2, n - 3) + X_(E, n - 3);
-    X_(s2, n - 2) = X_(D, n - 2);
-    X_(s2, n - 1) = X_(C, n - 1);
-    for (int i = 0; i <= n - 3; i++) {
-        double cs = X_(B, i + 1) / X_(C, i);
-        X_(C, i + 1) = X_(C, i + 1) - X_(D, i) * cs;
-        X_(D, i + 1) = X_(D, i + 1) - X_(E, i) * cs;
-        X_(R, i + 1) = X_(R, i + 1) - X_(R, i) * cs;
-        X_(s1, i + 1) = X_(s1, i + 1) - X_(s1, i) * cs;
-        X_(s2, i + 1) = X_(s2, i + 1) - X_(s2, i) * cs;
-        cs = X_(A, i + 2) / X_(C, i);
-        X_(B, i + 2) = X_(B, i + 2) - X_(D, i) * cs;
-        X_(C, i + 2) = X_(C, i + 2) - X_(E, i) * cs;
-        X_(R, i + 2) = X_(R, i + 2) - X_(R, i) * cs;
-        X_(s1, i + 2) = X_(s1, i + 2) - X_(s1, i) * cs;
-        X_(s2, i + 2) = X_(s2, i + 2) - X_(s2, i) * cs;
-    }
-    for (int i = n - 3; i >= 2; i--) {
-        double cs = X_(D, i - 1) / X_(C, i);
-        X_(R, i - 1) = X_(R, i - 1) - X_(R, i) * cs;
-        X_(s1, i - 1) = X_(s1, i - 1) - X_(s1, i) * cs;
-        X_(s2, i - 1) = X_(s2, i - 1) - X_(s2, i) * cs;
-        cs = X_(E, i - 2) / X_(C, i);
-        X_(R, i - 2) = X_(R, i - 2) - X_(R, i) * cs;
-        X_(s1, i - 2) = X_(s1, i - 2) - X_(s1, i) * cs;
-        X_(s2, i - 2) = X_(s2, i - 2) - X_(s2, i) * cs;
-    }
-    {
-        double cs = X_(D, 0) / X_(C, 1);
-        X_(R, 0) = X_(R, 0) - X_(R, 1) * cs;
-        X_(s1, 0) = X_(s1, 0) - X_(s1, 1) * cs;
-        X_(s2, 0) = X_(s2, 0) - X_(s2, 1) * cs;
-    }
-    double cs = X_(E, n - 2) / X_(C, 0);
-    X_(R, n - 2) = X_(R, n - 2) - X_(R, 0) * cs;
-    X_(s1, n - 2) = X_(s1, n - 2) - X_(s1, 0) * cs;
-    X_(s2, n - 2) = X_(s2, n - 2) - X_(s2, 0) * cs;
-    cs = X_(D, n - 1) / X_(C, 0);
-    X_(R, n - 1) = X_(R, n - 1) - X_(R, 0) * cs;
-    X_(s1, n - 1) = X_(s1, n - 1) - X_(s1, 0) * cs;
-    X_(s2, n - 1) = X_(s2, n - 1) - X_(s2, 0) * cs;
-    cs = X_(E, n - 1) / X_(C, 1);
-    X_(R, n - 1) = X_(R, n - 1) - X_(R, 1) * cs;
-    X_(s1, n - 1) = X_(s1, n - 1) - X_(s1, 1) * cs;
-    X_(s2, n - 1) = X_(s2, n - 1) - X_(s2, 1) * cs;
-    cs = X_(s1, n - 1) / X_(s1, n - 2);
-    X_(R, n - 1) = X_(R, n - 1) - X_(R, n - 2) * cs;
-    X_(s2, n - 1) = X_(s2, n - 1) - X_(s2, n - 2) * cs;
-    X_(R, n - 1) = X_(R, n - 1) / X_(s2, n - 1);
-    X_(R, n - 2) = (X_(R, n - 2) - X_(s2, n - 2) * X_(R, n - 1)) / X_(s1, n - 2);
-    for (int i = n - 3; i >= 0; i--)
-        X_(R, i) = (X_(R, i) - X_(s1, i) * X_(R, n - 2) - X_(s2, i) * X_(R, n - 1)) / X_(C, i);
-#undef X_
-}
-
-int dev_tridiagonal(st_ctx *c, const double *A, const double *B, const double *C, double *R, int n,
-                    int lot, int nper) {
-    size_t N = (size_t)n * lot;
-    double *a = nullptr, *b = nullptr;
-    ST_CUDA(c, cudaMallocAsync(&a, 2 * N * sizeof(double), c->stream));
-    b = a + N;
-    ST_CUDA(c, cudaMemcpyAsync(a, A, N * 8, cudaMemcpyDeviceToDevice, c->stream));
-    ST_CUDA(c, cudaMemcpyAsync(b, B, N * 8, cudaMemcpyDeviceToDevice, c->stream));
-    int pi = prof_start(c, "k_tri_general", 32.0 * N);
-    k_tri_general<<<(lot + 127) / 128, 128, 0, c->stream>>>(a, b, C, R, n, lot, nper);
-    prof_stop(c, pi);
-    cudaError_t e = cudaGetLastError();
-    cudaFreeAsync(a, c->stream);
-    if (e != cudaSuccess) return fail(c, ST_E_CUDA, cudaGetErrorString(e));
-    return ST_OK;
-}
-
-int dev_pentadiagonal(st_ctx *c, const double *A, const double *B, const double *C, const double *D,
-                      const double *E, double *R, int n, int lot, int nper) {
-    if (nper && n < 5) return fail(c, ST_E_UNSUPPORTED, "periodic pentadiagonal needs n >= 5");
-    size_t N = (size_t)n * lot;
-    double *buf = nullptr;
-    ST_CUDA(c, cudaMallocAsync(&buf, 7 * N * sizeof(double), c->stream));
-    double *a = buf, *b = buf + N, *cc = buf + 2 * N, *d = buf + 3 * N, *e = buf + 4 * N;
-    double *s1 = buf + 5 * N, *s2 = buf + 6 * N;
-    const double *src[5] = {A, B, C, D, E};
-    double *dst[5] = {a, b, cc, d, e};
-    for (int q = 0; q < 5; q++)
-        ST_CUDA(c, cudaMemcpyAsync(dst[q], src[q], N * 8, cudaMemcpyDeviceToDevice, c->stream));
-    int pi = prof_start(c, "k_pen_general", 48.0 * N);
-    k_pen_general<<<(lot + 127) / 128, 128, 0, c->stream>>>(a, b, cc, d, e, R, s1, s2, n, lot, nper);
-    prof_stop(c, pi);
-    cudaError_t er = cudaGetLastError();
-    cudaFreeAsync(buf, c->stream);
-    if (er != cudaSuccess) return fail(c, ST_E_CUDA, cudaGetErrorString(er));
-    return ST_OK;
-}
 
 }  // namespace st

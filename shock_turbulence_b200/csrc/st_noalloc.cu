@@ -1,13 +1,14 @@
 // st_noalloc.cu - st_tridiagonal_noalloc: the general tridiagonal solve of
 // st_tridiagonal, for callers that must not allocate device memory.
 //
-// st_tridiagonal needs two working copies of A and B (the reference's
-// tridiagonal_serial overwrites its coefficients, src/tridiagonal.f90:274-284).
-// It gets them from cudaMalloc/cudaMallocAsync, and it stages host arrays
-// through more device buffers.  Some callers cannot allow that: a host program
+// st_tridiagonal needs room for what the elimination makes of B, and of A for
+// periodic lines (the reference's tridiagonal_serial overwrites its
+// coefficients, src/tridiagonal.f90:274-284).  It gets it from a workspace
+// that it allocates when a call needs more than the ones before, and it stages
+// host arrays there.  Some callers cannot allow that: a host program
 // that owns all device memory through its own pool and must not see a second
 // allocator touch the device, and code on a latency budget where an allocation
-// can block on the driver and stall the device's other work.  This entry point takes the working copies
+// can block on the driver and stall the device's other work.  This entry point takes the workspace
 // from a fixed array in the library's static device memory instead.
 //
 // Limits and rules:
@@ -18,8 +19,8 @@
 //  - The first call on each device looks up the scratch array's address with
 //    cudaGetSymbolAddress; the driver may load the library's device code at
 //    that moment.  Make that first call before any stream capture begins.
-//  - Nothing in the scratch has to start at zero: each call copies A and B
-//    into it in full before the solve reads it.
+//  - Nothing in the scratch has to start at zero: each call writes what it
+//    reads.
 //  - The scratch is one array per device, shared by every context on that
 //    device.  Calls whose GPU work overlaps (different streams, threads or
 //    contexts on one device) race on it.  Calls on one stream are ordered and
@@ -30,18 +31,13 @@
 
 namespace st {
 
-// defined in st_kernels.cu: tridiagonal_serial / tridiagonal_periodic_serial,
-// thread per line, arrays (lot,n) with lot fastest; a and b are overwritten.
-__global__ void k_tri_general(double *a, double *b, const double *cc, double *R, int n, int lot,
-                              int nper);
-
 namespace {
 
 constexpr size_t kNoAllocMaxElems = size_t(1) << 18;
 constexpr int kMaxDevices = 64;
 
-// working copies of A and B: a call with N = n*lot elements puts A's copy in
-// the first N entries and B's copy right after it, in entries N .. 2N-1
+// a call with N = n*lot elements uses the first N entries, or 2N for periodic
+// lines
 __device__ __align__(256) double g_tri_scratch[2 * kNoAllocMaxElems];
 
 std::mutex g_setup_mu;
@@ -98,12 +94,7 @@ static int tridiagonal_noalloc(st_ctx *c, const double *A, const double *B, cons
     double *a = nullptr;
     int rc = scratch_on(c, c->dev, &a);
     if (rc != ST_OK) return rc;
-    double *b = a + N;
-    ST_CUDA(c, cudaMemcpyAsync(a, A, N * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    ST_CUDA(c, cudaMemcpyAsync(b, B, N * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    c->launches++;
-    k_tri_general<<<(lot + 127) / 128, 128, 0, c->stream>>>(a, b, C, R, n, lot, nper);
-    ST_CUDA(c, cudaGetLastError());
+    ST_TRY(dev_tridiagonal(c, A, B, C, R, a, n, lot, nper));
     ST_CUDA(c, cudaStreamSynchronize(c->stream));
     return ST_OK;
 }
