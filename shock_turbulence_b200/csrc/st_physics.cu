@@ -15,20 +15,20 @@ namespace st {
 // largest passes (the fused RHS flux passes, 80 registers uncapped) spill
 // about 100 bytes but gain the occupancy; measured 10 % faster on the FP32
 // mode's pointwise family and 2 % on the FP64 one.
-template <class Fn>
-__global__ void __launch_bounds__(256, 4) k_pfor(size_t n, Fn fn) {
+template <int CTAS, class Fn>
+__global__ void __launch_bounds__(256, CTAS) k_pfor(size_t n, Fn fn) {
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
         fn(p);
 }
 // site: "k_pointwise@<source line>" for the per-launch timing report
 // bpe: algorithmic bytes per element (every array element the launch reads
 // or writes, once; an element both read and written counts twice)
-template <class Fn>
+template <int CTAS = 4, class Fn>
 static int pfor(st_ctx *c, size_t n, const char *site, double bpe, Fn fn) {
     size_t blocks = (n + 255) / 256;    // one element per thread
     if (blocks == 0) return ST_OK;
     int pi = prof_start(c, site, bpe * (double)n);
-    k_pfor<<<(unsigned)blocks, 256, 0, c->stream>>>(n, fn);
+    k_pfor<CTAS><<<(unsigned)blocks, 256, 0, c->stream>>>(n, fn);
     prof_stop(c, pi);
     ST_CUDA(c, cudaGetLastError());
     return ST_OK;
@@ -37,6 +37,9 @@ static int pfor(st_ctx *c, size_t n, const char *site, double bpe, Fn fn) {
 #define ST_STR(x) ST_STR2(x)
 #define PFOR(c, n, bpe, ...) \
     ST_TRY(pfor((c), (n), "k_pointwise@" ST_STR(__LINE__), (bpe), [=] __device__(size_t p) __VA_ARGS__))
+// the same with CTAS resident CTAs per SM
+#define PFOR_CTAS(c, ctas, n, bpe, ...) \
+    ST_TRY(pfor<ctas>((c), (n), "k_pointwise@" ST_STR(__LINE__), (bpe), [=] __device__(size_t p) __VA_ARGS__))
 // bytes of one element of each listed array (its element type's size), for
 // the algorithmic byte count of a pointwise launch
 template <class... P>
@@ -152,8 +155,13 @@ __device__ __forceinline__ void viscosity(const Phys &f, double T, double Y, dou
     double se = sqrt(f.eps);
     double num = f.Re1_inv * Y + f.Re2_inv * se * (1.0 - Y);
     double den = Y + se * (1.0 - Y);
-    mu = pow(fac1 * T, f.vis_exp) * num / den;
-    dmu = pow(fac1 * T, fac2) * num / den * f.vis_exp * fac1;
+    // x^(e-1) = x^e / x: a power costs some hundred FP64 operations, which
+    // bound the pass in the FP32 mode; taken directly where the quotient is
+    // not defined
+    const double x = fac1 * T, pw = pow(x, f.vis_exp);
+    const double pd = (pw > 0.0 && pw < INFINITY) ? pw / x : pow(x, fac2);
+    mu = pw * num / den;
+    dmu = pd * num / den * f.vis_exp * fac1;
 }
 
 // n separate scratch fields
@@ -178,15 +186,17 @@ int dev_to_double(st_ctx *c, const float *x, double *y, size_t n) {
     return ST_OK;
 }
 
+// Compute_gamma, src/lddrk4_nonperiodic_mf.f:342-372
+__device__ __forceinline__ double gamma_of(const Phys &f, double Y) {
+    double fac1 = f.g1 - 1.0, fac2 = f.g2 - 1.0;
+    double num = (Y * f.g1 / fac1) + (f.eps * (1.0 - Y) * f.g2 / fac2);
+    double den = (Y / fac1) + (f.eps * (1.0 - Y) / fac2);
+    return num / den;
+}
 int dev_compute_gamma(st_ctx *c, const double *Y) {
     Phys f = phys(c);
     double *ge = c->gamma_eff;
-    PFOR(c, c->ncell(), io(Y, ge), {
-        double fac1 = f.g1 - 1.0, fac2 = f.g2 - 1.0;
-        double num = (Y[p] * f.g1 / fac1) + (f.eps * (1.0 - Y[p]) * f.g2 / fac2);
-        double den = (Y[p] / fac1) + (f.eps * (1.0 - Y[p]) / fac2);
-        ge[p] = num / den;
-    });
+    PFOR(c, c->ncell(), io(Y, ge), { ge[p] = gamma_of(f, Y[p]); });
     return ST_OK;
 }
 
@@ -208,8 +218,9 @@ int dev_compute_gamma(st_ctx *c, const double *Y) {
 // R is the storage type of every field except the state: double, or float in
 // the FP32 mode.  Qr is the state in that type (Q itself in FP64); the
 // derivative operands come from Qr, the pointwise thermodynamics from Q.
+// gamma_from_Y: also Compute_gamma (gamma_eff of Y) in the first pass.
 template <class R>
-static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
+static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bool gamma_from_Y = false) {
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
     const Phys f = phys(c);
     // src/rhsv_periodic_sf.f:1381 adds Qvisc unconditionally
@@ -221,22 +232,24 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
     R *Gxy = G[G_DUX_DY], *Gyy = G[G_DUY_DY], *Gzy = G[G_DUZ_DY];
     R *Gxz = G[G_DUX_DZ], *Gyz = G[G_DUY_DZ], *Gzz = G[G_DUZ_DZ];
     R *GTx = G[G_DTDX], *GTy = G[G_DTDY], *GTz = G[G_DTDZ];
-    ScratchT<R> sQcx(c, 5), sQcy(c, 5), sQcz(c, 5), sQv(c, 5);
-    R *Qcx = sQcx, *Qcy = sQcy, *Qcz = sQcz, *Qv = sQv;   // Qv(:,:,:,4) is never formed
+    ScratchT<R> sQcx(c, 5), sQcy(c, 5), sQcz(c, 5);
+    R *Qcx = sQcx, *Qcy = sQcy, *Qcz = sQcz;
     ScratchNT<R> s(c, 8);
     R *P = s[0], *T = s[1], *u = s[2], *v = s[3], *w = s[4], *mu = s[5], *dmu = s[6], *FF = s[7];
-    // second derivatives and derivatives of /GRAD/ consumed by the two
-    // pointwise passes below (one field each, so that all of them can be
-    // formed before the pass that uses them)
-    ScratchNT<R> dd(c, 14);
-    const double *g = c->gamma_eff;
+    // second derivatives and derivatives of /GRAD/ (one field each: all of
+    // them are formed before the one pointwise pass that uses them)
+    ScratchNT<R> dd(c, 18);
+    double *g = c->gamma_eff;
 
     // ---- RHS_x (src/rhsv_sym_mf.f:37-481)
     // P, T, u, and (the same expressions the reference evaluates later from
     // the same inputs) v, w, mu, dmu/dT
     PFOR(c, nc, io(g, Y, Q1, Q2, Q3, Q4, Q5, P, T, u, v, w, mu, dmu), {
         double vs, pp, tt, m, dm;
-        thermo(f, g[p], Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], vs, pp, tt);
+        double ge;
+        if (gamma_from_Y) { ge = gamma_of(f, Y[p]); g[p] = ge; }
+        else ge = g[p];
+        thermo(f, ge, Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], vs, pp, tt);
         P[p] = pp; T[p] = tt;
         u[p] = Q1[p] * vs;
         v[p] = Q2[p] * vs;
@@ -254,7 +267,7 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
     ST_TRY(dfd_pair<R>(c, 0, pr_mul(q2r, cu), Qcx + n3, 1, 0, -5.0e-1, pr_mul(q3r, cu), Qcx + 2 * n3, 1, 0,
                        -5.0e-1));
     ST_TRY(dfd(c, 0, 1, q1r, FF, 0, 1.0));
-    R *dTx = dd[0], *duxx = dd[1], *dvxx = dd[2], *dwxx = dd[3];
+    R *dTx = dd[14], *duxx = dd[15], *dvxx = dd[16], *dwxx = dd[17];
     if (visc) {
         ST_TRY(d2fd2(c, 0, 0, (const R *)T, GTx, dTx, 1));
         ST_TRY(d2fd2(c, 0, 1, (const R *)u, Gxx, duxx, 1));
@@ -266,35 +279,6 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
         ST_TRY(dfd(c, 0, 0, (const R *)v, Gyx, 0, 1.0));
         ST_TRY(dfd(c, 0, 0, (const R *)w, Gzx, 0, 1.0));
     }
-    // convective terms -0.5*d(rho u)/dx*(u,v,w) and -0.5*rho*u*d(u,v,w)/dx,
-    // and the x part of Qvisc, in the reference's order of accumulation
-    {
-        const double Pri = f.Pr_inv, fac1 = 4.0 / 3.0 + f.bulk;
-        PFOR(c, nc, io(FF, u, v, w, Q4, Gxx, Gyx, Gzx) + 6 * io(Qcx) + (visc ? io(mu, dTx, dmu, GTx, duxx, dvxx, dwxx) + 4 * io(Qv) : 0.0), {
-            double fac2 = -5.0e-1 * FF[p];
-            double c1 = Qcx[p] + fac2 * u[p];
-            double c2 = Qcx[n3 + p] + fac2 * v[p];
-            double c3 = Qcx[2 * n3 + p] + fac2 * w[p];
-            if (visc) {
-                double q5 = Pri * (mu[p] * dTx[p] + dmu[p] * GTx[p] * GTx[p]);
-                double fx = fac1 * mu[p] * duxx[p];
-                q5 = q5 + u[p] * fx;
-                double fy = mu[p] * dvxx[p];
-                q5 = q5 + v[p] * fy;
-                double fz = mu[p] * dwxx[p];
-                q5 = q5 + w[p] * fz;
-                Qv[p] = fx;
-                Qv[n3 + p] = fy;
-                Qv[2 * n3 + p] = fz;
-                Qv[4 * n3 + p] = q5;
-            }
-            fac2 = -5.0e-1 * Q4[p] * u[p];
-            Qcx[p] = c1 + fac2 * Gxx[p];
-            Qcx[n3 + p] = c2 + fac2 * Gyx[p];
-            Qcx[2 * n3 + p] = c3 + fac2 * Gzx[p];
-        });
-    }
-
     // ---- RHS_yz (src/rhsv_sym_mf.f:492-1428)
     // d(rho v)/dy and d(rho w)/dz with iadd=0, cadd=-1: Qconv(4) = 0 - d(.) exactly
     ST_TRY(dfd(c, 1, 1, q2r, Qcy + 3 * n3, 0, -1.0));
@@ -336,17 +320,27 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
         ST_TRY(dfd(c, 2, 1, (const R *)Gzx, dGzx_z, 0, 1.0));
         ST_TRY(dfd(c, 1, 1, (const R *)Gyz, dGyz_y, 0, 1.0));
     }
-    // One pass for the rest of RHS_yz and the sum Qrhs = Qconvx + Qconvy +
-    // Qconvz + Qvisc: each accumulator receives its terms in the order the
-    // reference adds them (src/rhsv_sym_mf.f:992-1424), in registers.
+    // One pass for the pointwise terms of RHS_x and RHS_yz and the sum Qrhs =
+    // Qconvx + Qconvy + Qconvz + Qvisc: each accumulator receives its terms in
+    // the order the reference adds them (src/rhsv_sym_mf.f:312-481, 992-1424),
+    // in registers.  Two CTAs of up to 128 registers per SM instead of four of
+    // 64: a thread has its 55 loads in flight at once, and none spill.  384^3:
+    // 3.93 ms at 6.9 TB/s (x terms in a pass of their own that stored and
+    // reloaded seven fields, four CTAs: 1.70 + 4.79 ms).
     {
         const double Pri = f.Pr_inv;
         const double fb43 = f.bulk + 4.0 / 3.0, fb23 = f.bulk - 2.0 / 3.0, fb13 = f.bulk + 1.0 / 3.0;
         const bool fp64 = is_fp64<R>();
-        PFOR(c, nc, io(u, v, w, Q4, Gxx, Gyx, Gzx, Gxy, Gyy, Gzy, Gxz, Gyz, Gzz) + 5 * io(Qcx, Qcy, Qcz, Qrhs) + (fp64 ? io(Q1, Q2, Q3) : 0.0) + (visc ? io(mu, dmu, d2Ty, d2Tz, GTy, GTz, GTx, d2uy, d2vy, d2wy, dGzz_y, d2wz, d2uz, d2vz, dGyx_y, dGzx_z, dGxx_y, dGxx_z, dGyz_y) + 4 * io(Qv) : 0.0), {
+        const double fac43 = 4.0 / 3.0 + f.bulk;
+        PFOR_CTAS(c, 2, nc, io(FF, u, v, w, Q4, Gxx, Gyx, Gzx, Gxy, Gyy, Gzy, Gxz, Gyz, Gzz) + 5 * io(Qcx, Qcy, Qcz, Qrhs) + (fp64 ? io(Q1, Q2, Q3) : 0.0) + (visc ? io(mu, dmu, dTx, duxx, dvxx, dwxx, d2Ty, d2Tz, GTy, GTz, GTx, d2uy, d2vy, d2wy, dGzz_y, d2wz, d2uz, d2vz, dGyx_y, dGzx_z, dGxx_y, dGxx_z, dGyz_y) : 0.0), {
             const double uu = u[p], vv = v[p], ww = w[p], q4 = Q4[p];
+            // x: -0.5*d(rho u)/dx*(u,v,w).  The x sums are rounded to R where
+            // they stand alone (the FP32 mode's results do not depend on how
+            // the terms are split into passes).
+            double fac2 = -5.0e-1 * FF[p];
+            double cx1 = Qcx[p] + fac2 * uu, cx2 = Qcx[n3 + p] + fac2 * vv, cx3 = Qcx[2 * n3 + p] + fac2 * ww;
             // -0.5*d(rho v)/dy = 0.5*Qconvy(4) exactly (cadd flips only the sign)
-            double fac2 = -5.0e-1 * (-(double)Qcy[3 * n3 + p]);
+            fac2 = -5.0e-1 * (-(double)Qcy[3 * n3 + p]);
             double cy1 = Qcy[p] + fac2 * uu, cy2 = Qcy[n3 + p] + fac2 * vv, cy3 = Qcy[2 * n3 + p] + fac2 * ww;
             fac2 = -5.0e-1 * (-(double)Qcz[3 * n3 + p]);
             double cz1 = Qcz[p] + fac2 * uu, cz2 = Qcz[n3 + p] + fac2 * vv, cz3 = Qcz[2 * n3 + p] + fac2 * ww;
@@ -354,14 +348,27 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
             if (visc) {
                 m = mu[p];
                 const double dm = dmu[p];
-                v5 = Qv[4 * n3 + p] + Pri * (m * (d2Ty[p] + d2Tz[p]) +
-                                             dm * (GTy[p] * GTy[p] + GTz[p] * GTz[p]));
+                // x part of Qvisc
+                const R mr = mu[p], dmr = dmu[p];
+                double q5 = Pri * (mr * dTx[p] + dmr * GTx[p] * GTx[p]);
+                v1 = fac43 * mr * duxx[p];
+                q5 = q5 + uu * v1;
+                v2 = mr * dvxx[p];
+                q5 = q5 + vv * v2;
+                v3 = mr * dwxx[p];
+                q5 = q5 + ww * v3;
+                v1 = (R)v1; v2 = (R)v2; v3 = (R)v3;
+                v5 = (double)(R)q5 + Pri * (m * (d2Ty[p] + d2Tz[p]) + dm * (GTy[p] * GTy[p] + GTz[p] * GTz[p]));
                 U4 = dm * GTx[p];
                 Tdy = dm * GTy[p];
                 Tdz = dm * GTz[p];
             }
             const double gxx = Gxx[p], gyx = Gyx[p], gzx = Gzx[p], gxy = Gxy[p], gyy = Gyy[p], gzy = Gzy[p];
             const double gxz = Gxz[p], gyz = Gyz[p], gzz = Gzz[p];
+            fac2 = -5.0e-1 * q4 * uu;
+            cx1 = (R)(cx1 + fac2 * gxx);
+            cx2 = (R)(cx2 + fac2 * gyx);
+            cx3 = (R)(cx3 + fac2 * gzx);
             fac2 = -5.0e-1 * q4 * vv;
             cy1 = cy1 + fac2 * gxy;
             cy2 = cy2 + fac2 * gyy;
@@ -375,9 +382,9 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
                 double fX = m * d2uy[p];
                 double fY = fb43 * m * d2vy[p];
                 double fZ = m * d2wy[p];
-                v1 = Qv[p] + fX;
-                v2 = Qv[n3 + p] + fY;
-                v3 = Qv[2 * n3 + p] + fZ;
+                v1 = v1 + fX;
+                v2 = v2 + fY;
+                v3 = v3 + fZ;
                 v5 = v5 + uu * fX + vv * fY + ww * fZ;
                 // dilatation terms
                 double tmp1 = gxx;
@@ -416,12 +423,13 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y) {
                 Q2[p] = vv * q4;
                 Q3[p] = ww * q4;
             }
+            const double cx[5] = {cx1, cx2, cx3, Qcx[3 * n3 + p], Qcx[4 * n3 + p]};
             const double cy[5] = {cy1, cy2, cy3, Qcy[3 * n3 + p], Qcy[4 * n3 + p]};
             const double cz[5] = {cz1, cz2, cz3, Qcz[3 * n3 + p], Qcz[4 * n3 + p]};
             const double vq[5] = {v1, v2, v3, 0.0, v5};
             for (int l = 0; l < 5; l++) {
                 size_t q = l * n3 + p;
-                double r = Qcx[q] + cy[l] + cz[l];
+                double r = cx[l] + cy[l] + cz[l];
                 if (visc && l != 3) r = r + vq[l];   // Qvisc(:,:,:,4) stays zero
                 Qrhs[q] = r;
             }
@@ -1278,8 +1286,7 @@ static int lddrk4_mf(st_ctx *c) {
             double *Q = c->Q, *QW = c->QW, *Y = c->Y, *rYW = c->rYW;
             R *dQ = Store<R>::dQ(c), *drYi = Store<R>::drYi(c);
             if (!fresh) ST_TRY(refresh<R>(c, sc, Q, Y, true));
-            ST_TRY(dev_compute_gamma(c, Y));
-            ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, Y));
+            ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, Y, true));   // Compute_gamma and RHS
             ST_TRY(hyper_rhs_t<R>(c, Q, dQ, Y, sc.y(Y)));
             ST_TRY(species_rhs_t<R>(c, Q, sc.q(Q), dQ, Y, sc.y(Y), drYi));
             ST_TRY(bc_rhs_t<R>(c, Q, dQ, Y, drYi));
