@@ -890,26 +890,12 @@ int st_lddrk4(st_ctx *c, double *time, int *step) {
     API_END(c)
 }
 
-int st_step(st_ctx *c, double *time, int *step) {
-    SINGLE_CASE(c);
-    if (!time || !step) return ST_E_ARG;
-    API_BEGIN(c)
-    c->hpinned[7] = *time;
-    ST_CUDA(c, cudaMemcpyAsync(c->dscal + 7, c->hpinned + 7, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    ST_TRY(dev_compute_cfl(c, c->Q, false, nullptr, nullptr));
-    ST_TRY(dev_compute_tstep(c, c->Q, c->Y, *step, true, 0.0));
-    ST_TRY(dev_lddrk4(c, true));
-    ST_TRY(read_time(c, time));
-    *step = *step + 1;
-    return ST_OK;
-    API_END(c)
-}
-
 // the main-loop body without host synchronisation (dt and time stay on the device)
 static int enqueue_step(st_ctx *c, int step) {
     ST_TRY(dev_compute_cfl(c, c->Q, false, nullptr, nullptr));
     ST_TRY(dev_compute_tstep(c, c->Q, c->Y, step, true, 0.0));
     ST_TRY(dev_lddrk4(c, true));
+    c->step_warm = true;
     return ST_OK;
 }
 
@@ -944,18 +930,43 @@ static int capture_graph(st_ctx *c, cudaGraphExec_t *out, long long *nk, Fn fn) 
 
 extern "C" {
 
-int st_step_async(st_ctx *c, int step) {
-    if (step < 0) return ST_E_ARG;
-    if (c && c->nb > 1) return st_batch_step_async(c);
-    API_BEGIN(c)
-    // Compute_Tstep's branch depends on the step number only up to step 2;
-    // from then on every step is the same sequence of launches on the same
-    // buffers, captured once as a CUDA graph and replayed.
-    if (step < 2 || c->prof) return enqueue_step(c, step);
+// Compute_Tstep's branch depends on the step number only up to step 2; from
+// then on every step is the same sequence of launches on the same buffers,
+// captured once as a CUDA graph and replayed.  A step has run launch by launch
+// before (the scratch pool is sized), and the legacy stream cannot be captured.
+static int step_graph(st_ctx *c, int step) {
     if (!c->step_graph) ST_TRY(capture_graph(c, &c->step_graph, &c->graph_kernels, [&] { return enqueue_step(c, step); }));
     ST_CUDA(c, cudaGraphLaunch(c->step_graph, c->stream));
     c->launches += c->graph_kernels;
     return ST_OK;
+}
+
+// A step that the caller waits for takes the graph on grids whose launches
+// cost the host more than their kernels cost the GPU (64^3: 8.6 ms enqueued
+// launch by launch, @@ ms replayed; the two meet near 128^3, and larger grids
+// are spared the capture).
+constexpr size_t kGraphCells = (size_t)128 * 128 * 128;
+int st_step(st_ctx *c, double *time, int *step) {
+    SINGLE_CASE(c);
+    if (!time || !step) return ST_E_ARG;
+    API_BEGIN(c)
+    c->hpinned[7] = *time;
+    ST_CUDA(c, cudaMemcpyAsync(c->dscal + 7, c->hpinned + 7, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    if (*step >= 2 && !c->prof && c->step_warm && c->stream != cudaStreamLegacy && c->ncell() <= kGraphCells)
+        ST_TRY(step_graph(c, *step));
+    else ST_TRY(enqueue_step(c, *step));
+    ST_TRY(read_time(c, time));
+    *step = *step + 1;
+    return ST_OK;
+    API_END(c)
+}
+
+int st_step_async(st_ctx *c, int step) {
+    if (step < 0) return ST_E_ARG;
+    if (c && c->nb > 1) return st_batch_step_async(c);
+    API_BEGIN(c)
+    if (step < 2 || c->prof || !c->step_warm) return enqueue_step(c, step);
+    return step_graph(c, step);
     API_END(c)
 }
 

@@ -9,6 +9,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 #include "../../include/st_b200.h"
 
@@ -190,6 +191,7 @@ struct st_ctx {
     long long launches = 0;
     cudaGraphExec_t step_graph = nullptr;   // captured main-loop step (st_step_async)
     long long graph_kernels = 0;            // kernels in one replay of step_graph
+    bool step_warm = false;                 // a step has run launch by launch
     std::vector<cudaGraphExec_t> batch_graphs;   // batch step per active count (index na - 1)
     std::vector<long long> batch_graph_kernels;
     bool batch_warm = false;                     // a batch step has run eagerly (scratch pool sized)
@@ -222,6 +224,31 @@ int sync_stream(st_ctx *c);
 // launch instrumentation: every kernel launch is bracketed by these
 int prof_start(st_ctx *c, const char *name, double bytes);
 void prof_stop(st_ctx *c, int idx);
+
+// Launch that may begin while the kernel before it in the stream ends
+// (programmatic dependent launch): its blocks become resident as that one's
+// leave, run their prologue and stop at pdl_wait(), which returns when the
+// kernel before has completed.  Every kernel launched this way calls
+// pdl_wait() before it touches memory that another kernel writes or reads, and
+// pdl_next() behind it.  64^3 step, 1082 launches: @@.
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
 
 // tables
 int build_tables(st_ctx *c);

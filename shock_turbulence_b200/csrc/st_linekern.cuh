@@ -292,11 +292,16 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
     constexpr unsigned ALL = (1u << R::NIN) - 1;
 
     if (tid == 0) {
+#pragma unroll
+        for (int f = 0; f < R::NIN; f++) asm volatile("prefetch.tensormap [%0];" ::"l"(&a.in[f]) : "memory");
+#pragma unroll
+        for (int f = 0; f < I::stores(); f++) asm volatile("prefetch.tensormap [%0];" ::"l"(&a.out[f]) : "memory");
         for (int k = 0; k < K; k++) bar_init(bars + 8 * k);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         proxy_fence();
     }
     __syncthreads();
+    pdl_wait();
     if (tid == 0)
         for (int k = 0; k < K; k++)
             if ((int)blockIdx.x + k * G < a.ntile) { expect(k); load_tiles(blockIdx.x + k * G, k, ALL); }
@@ -345,6 +350,7 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
         kp = k;
         if (++k == K) { k = 0; par ^= 1; }
     }
+    pdl_next();
     if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
@@ -408,11 +414,11 @@ static int launch_lines(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *const
     long grid = (long)c->sms * ctas;
     if (grid > a.ntile) grid = a.ntile;
     int pi = prof_start(c, name, fields * sizeof(T) * (double)c->ncell());
-    constexpr auto kern = k_lines<R, S, M, L, YT, CYC, T>;
-    set_smem<kern>(smem);
-    kern<<<(unsigned)grid, threads, smem, c->stream>>>(a);
+    set_smem<k_lines<R, S, M, L, YT, CYC, T>>(smem);
+    void (*kern)(const LineArgsT<T>) = k_lines<R, S, M, L, YT, CYC, T>;
+    const cudaError_t e = launch_pdl(kern, dim3((unsigned)grid), dim3(threads), smem, c->stream, a);
     prof_stop(c, pi);
-    ST_CUDA(c, cudaGetLastError());
+    ST_CUDA(c, e);
     return ST_OK;
 }
 

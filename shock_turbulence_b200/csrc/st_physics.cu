@@ -17,8 +17,10 @@ namespace st {
 // mode's pointwise family and 2 % on the FP64 one.
 template <int CTAS, class Fn>
 __global__ void __launch_bounds__(256, CTAS) k_pfor(size_t n, Fn fn) {
+    pdl_wait();
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
         fn(p);
+    pdl_next();
 }
 // site: "k_pointwise@<source line>" for the per-launch timing report
 // bpe: algorithmic bytes per element (every array element the launch reads
@@ -28,9 +30,9 @@ static int pfor(st_ctx *c, size_t n, const char *site, double bpe, Fn fn) {
     size_t blocks = (n + 255) / 256;    // one element per thread
     if (blocks == 0) return ST_OK;
     int pi = prof_start(c, site, bpe * (double)n);
-    k_pfor<CTAS><<<(unsigned)blocks, 256, 0, c->stream>>>(n, fn);
+    const cudaError_t e = launch_pdl(k_pfor<CTAS, Fn>, dim3((unsigned)blocks), dim3(256), 0, c->stream, n, fn);
     prof_stop(c, pi);
-    ST_CUDA(c, cudaGetLastError());
+    ST_CUDA(c, e);
     return ST_OK;
 }
 #define ST_STR2(x) #x
