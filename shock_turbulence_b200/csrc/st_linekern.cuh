@@ -80,6 +80,7 @@ struct OpArgT {
     double fac1, fac2;       // first / second derivative factor
     int asym;
     TriTabT<T> t1, t2;       // first / second derivative tables (OP_LAP: t2 the antisymmetric first derivative's)
+    unsigned tab, tab2;      // where their copies start in shared memory, from the tables' start
 };
 
 template <class T>
@@ -148,8 +149,9 @@ template <class V, int L>
 __host__ __device__ inline unsigned carry_bytes(int P) { return 2u * carry_one<V, L>(P) + corner_bytes<V, L>() + 8u * kSlotsMax; }
 
 template <int S, int M, int L, bool YT, bool CYC, class T, class OPD, class Mid>
-__device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o, const View<S, L, YT, T> &w, int s, int lane,
-                                       const CarryT<typename Val<T>::V, L> &cb, Mid mid) {
+__device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o, const unsigned char *tabs,
+                                       const View<S, L, YT, T> &w, int s, int lane, const CarryT<typename Val<T>::V, L> &cb,
+                                       Mid mid) {
     using V = typename Val<T>::V;
     using SRC = typename OPD::SRC;
     const int n = a.n, P = a.P, row0 = s * S;
@@ -158,8 +160,8 @@ __device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o
         V v[S + 4];
         w.template load<SRC, 2>(v);
         rhs_d1<S, CYC>(v, row0, n, o.asym, o.fac1, a.c, rd);
-        tri<S, M, L>(v, o.t1, s, P, lane, cb, mid);
-        if constexpr (CYC) cyc_fix<S, L, 2>(v, o.t1.cyc, o.t1.clo, o.t1.chi, s, P, lane, cb);
+        const T *tab = reinterpret_cast<const T *>(tabs + o.tab);
+        tri<S, M, L, CYC>(v, o.t1, tab, s, P, lane, cb, mid);
         w.template store<OPD::KIND == OP_D1ADD>(v, OPD::OUT);
         if constexpr (OPD::KIND == OP_LAP) {
             // the derivative (in the tile now) of a symmetric field is
@@ -169,16 +171,14 @@ __device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o
             auto rd2 = [&](int i) { return w.template row<D>(i); };
             w.template load<D, 2>(v);
             rhs_d1<S, CYC>(v, row0, n, 1, o.fac1, a.c, rd2);
-            tri<S, M, L>(v, o.t2, s, P, lane, cb, [] {});
-            if constexpr (CYC) cyc_fix<S, L, 2>(v, o.t2.cyc, o.t2.clo, o.t2.chi, s, P, lane, cb);
+            tri<S, M, L, CYC>(v, o.t2, reinterpret_cast<const T *>(tabs + o.tab2), s, P, lane, cb, [] {});
             w.store(v, OPD::OUT);
         }
     } else if constexpr (OPD::KIND == OP_D2) {
         V v[S + 4];
         w.template load<SRC, 2>(v);
         rhs_d2<S, CYC>(v, row0, n, o.asym, o.fac2, a.c, rd);
-        tri<S, M, L>(v, o.t2, s, P, lane, cb, mid);
-        if constexpr (CYC) cyc_fix<S, L, 2>(v, o.t2.cyc, o.t2.clo, o.t2.chi, s, P, lane, cb);
+        tri<S, M, L, CYC>(v, o.t2, reinterpret_cast<const T *>(tabs + o.tab2), s, P, lane, cb, mid);
         w.store(v, OPD::OUT);
     } else if constexpr (OPD::KIND == OP_FILTER || OPD::KIND == OP_FILTERM) {
         V v[S + 8];
@@ -186,7 +186,7 @@ __device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o
         rhs_filter<S, CYC>(v, row0, n, o.asym, a.c, rd);
         if constexpr (OPD::KIND == OP_FILTER) pen_solve<S, L>(v, a.p, s, P, lane, cb, mid);
         else pen_solve_m<S / M, M, L>(v, a.p, s, P, lane, cb, mid);
-        if constexpr (CYC) cyc_fix<S, L, 4>(v, a.p.cyc, a.p.clo, a.p.chi, s, P, lane, cb);
+        if constexpr (CYC) cyc_fix<S, L, 4>(v, a.p.cyc + (size_t)s * S * 4, s >= a.p.clo && s < a.p.chi, s, P, lane, cb);
         w.store(v, OPD::OUT);
     } else {
         V v[S + 8];
@@ -227,12 +227,38 @@ struct RecipeInfo<Recipe<NIN, NT, OPS...>> {
 template <class R> struct RecipeRun;
 template <int NIN, int NT, class... OPS>
 struct RecipeRun<Recipe<NIN, NT, OPS...>> {
+    static constexpr bool uses1(int kind) { return kind == OP_D1 || kind == OP_D1ADD || kind == OP_LAP; }
+    static constexpr bool uses2(int kind) { return kind == OP_D2 || kind == OP_LAP; }
+    // host: places the operations' tridiagonal tables, returns their bytes
+    template <int S, int M, class T>
+    static unsigned place_tables(LineArgsT<T> &a) {
+        unsigned at = 0;
+        auto one = [&](int kind, OpArgT<T> &o) {
+            if (uses1(kind)) { o.tab = at; at += tri_bytes(o.t1, a.P * M, S / M, a.P, S); }
+            if (uses2(kind)) { o.tab2 = at; at += tri_bytes(o.t2, a.P * M, S / M, a.P, S); }
+        };
+        (one(OPS::KIND, a.op[OPS::ARG]), ...);
+        return at;
+    }
+    template <int S, int M, class T, class O>
+    __device__ __forceinline__ static void fill_one(const LineArgsT<T> &a, unsigned char *tabs) {
+        const OpArgT<T> &o = a.op[O::ARG];
+        if constexpr (O::KIND == OP_D1 || O::KIND == OP_D1ADD || O::KIND == OP_LAP)
+            tri_fill(reinterpret_cast<T *>(tabs + o.tab), o.t1, a.P * M, S / M, a.P, S);
+        if constexpr (O::KIND == OP_D2 || O::KIND == OP_LAP)
+            tri_fill(reinterpret_cast<T *>(tabs + o.tab2), o.t2, a.P * M, S / M, a.P, S);
+    }
+    template <int S, int M, class T>
+    __device__ __forceinline__ static void fill_tables(const LineArgsT<T> &a, unsigned char *tabs) {
+        (fill_one<S, M, T, OPS>(a, tabs), ...);
+    }
     // the operations in turn; hook(op) runs in thread 0 behind the first
     // barrier of each
     template <int S, int M, int L, bool YT, bool CYC, class T, class Hook, size_t... Q>
-    __device__ __forceinline__ static void run(const LineArgsT<T> &a, const View<S, L, YT, T> &w, int s, int lane,
+    __device__ __forceinline__ static void run(const LineArgsT<T> &a, const unsigned char *tabs, const View<S, L, YT, T> &w,
+                                               int s, int lane,
                                                const CarryT<typename Val<T>::V, L> &cb, Hook hook, std::index_sequence<Q...>) {
-        (run_op<S, M, L, YT, CYC, T, OPS>(a, a.op[OPS::ARG], w, s, lane, cb, [&] { hook(std::integral_constant<int, (int)Q>()); }), ...);
+        (run_op<S, M, L, YT, CYC, T, OPS>(a, a.op[OPS::ARG], tabs, w, s, lane, cb, [&] { hook(std::integral_constant<int, (int)Q>()); }), ...);
     }
 };
 
@@ -253,6 +279,7 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
                           reinterpret_cast<const V *>(tab)};
     const unsigned bars = smem_u32(tail + 2 * cbb + corner_bytes<V, L>());
     if constexpr (PEN) pen_fill(reinterpret_cast<double *>(tab), a.p, P * M, S / M, !PENM);
+    else RecipeRun<R>::template fill_tables<S, M, T>(a, tab);
 
     // thread 0: transfers of one tile of lines.  x lines: (y, z) at c0, c1
     // and rows along the third coordinate; z lines: (y, x) and rows along the
@@ -316,7 +343,7 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
         w.sm = smem + k * slot_b;
         const int next = tile + (K == 1 ? 1 : K - 1) * G;
         const bool more = next < a.ntile;
-        RecipeRun<R>::template run<S, M, L, YT, CYC, T>(a, w, s, lane, cb, [&](auto q) {
+        RecipeRun<R>::template run<S, M, L, YT, CYC, T>(a, tab, w, s, lane, cb, [&](auto q) {
             constexpr int OP = decltype(q)::value;
             // the result of the operation before leaves, and with one slot
             // the tiles that are free are filled for the next tile of lines
@@ -398,7 +425,7 @@ static int launch_lines(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *const
     // two slots do not fit.
     const unsigned slot = R::NT * a.tb, tail = carry_bytes<V, L>(a.P * M) +
                           (std::is_same<R, RecFilterM>::value ? 2u * carry_one<V, L>(a.P * M) : 0u) +
-                          (a.p.id ? pen_bytes(a.p, a.P * M, S / M) : 0u);
+                          (a.p.id ? pen_bytes(a.p, a.P * M, S / M) : 0u) + RecipeRun<R>::template place_tables<S, M, T>(a);
     const int threads = L * a.P;
     const int by_regs = 65536 / (80 * ((threads + 31) / 32 * 32));
     auto fit = [&](int ctas) { return ((long)(c->smem_sm / ctas) - 1024 - (long)tail) / (long)slot; };   // slots
@@ -428,7 +455,7 @@ template <class R, int S, int M, bool CYC, class T>
 static int launch_lines_L(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *const *out, const char *name) {
     a.P = a.n / S;
     if constexpr (R::NT == 4 && S == 16 && M == 1) {
-        if (4L * 128 * a.n + carry_bytes<typename Val<T>::V, 16>(a.P) > c->smem_cta) {
+        if (4L * 128 * a.n + carry_bytes<typename Val<T>::V, 16>(a.P) + RecipeRun<R>::template place_tables<S, M, T>(a) > c->smem_cta) {
             if (a.dir == 1) return launch_lines<R, S, M, 8, true, CYC, T>(c, a, in, out, name);
             return launch_lines<R, S, M, 8, false, CYC, T>(c, a, in, out, name);
         }
