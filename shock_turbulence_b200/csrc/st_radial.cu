@@ -5,19 +5,24 @@
 // Work decomposition: one CTA owns one problem at a time.  A problem's line
 // of n <= T*SMAX points is split into T contiguous segments of S = ceil(n/T)
 // rows, one per thread, held in registers.  Every line operator
-//   - stages its input line in shared memory (coalesced), so the explicit
-//     stencils read any neighbour directly and the boundary rows are plain
-//     index cases;
+//   - has its input line staged in shared memory row by row (coalesced, with a
+//     gap behind each thread's rows against bank conflicts) and leaves its
+//     result there; the boundary rows are plain index cases;
 //   - solves its constant-coefficient banded system by local recurrences per
-//     segment plus a block-wide scan of the segments' affine carry maps
-//     (scalar maps for the tridiagonal derivative systems, 2-vector maps with
-//     2x2 matrices for the pentadiagonal filter).  In exact arithmetic this is
-//     the forward elimination / back substitution of pentadiagonal_serial
-//     (src/pentadiagonal.f90:319-374); no per-length carry tables are needed.
+//     segment plus the carries between segments: a sum over the few segments
+//     that reach for the tridiagonal derivative systems, a block-wide scan of
+//     affine maps (2x2 matrices) for the pentadiagonal filter.  In exact
+//     arithmetic this is the forward elimination / back substitution of
+//     pentadiagonal_serial (src/pentadiagonal.f90:319-374); no per-length carry
+//     tables are needed.
 // LU factors: the rows of every system are the same for all problems except
-// the last few, so the factors of rows 0..n-5 are one universal table (the
-// elimination of row i only involves rows <= i) and only rows n-4..n-1 come
-// from a small per-length tail table.
+// the last few, so the factors of the first rows are one universal table, the
+// interior is at their fixed point (constants) and only rows n-4..n-1 come
+// from a small per-length tail table; a CTA keeps all of them in shared memory.
+// Measured, 512 problems of 128 to 4096 points, 4 steps: 18.5 ms; with scans of
+// maps for every system, factors from global memory and the lanes' segments
+// 64 bytes apart in shared memory 31.4 ms.  What is left is instructions (3000
+// per point and stage, a tenth of the FP64 rate) and the barriers of 16 warps.
 //
 // A persistent kernel pulls problems (longest first) from a queue and runs all
 // the requested LDDRK4 steps of a problem before taking the next; problems
@@ -48,12 +53,28 @@ struct K {
 
 __constant__ K c_k;        // scheme constants, identical for every batch
 
+// Away from the line's ends the eliminations reach a fixed point: rows i0 ..
+// n - kTail - 1 of every line have the factors below.  A thread whose rows all
+// lie there takes them (and the powers that its carry responses are) from the
+// constant bank instead of from the tables, whose rows a warp's lanes would
+// read one segment length apart.
+constexpr int kRowsMax = 16;        // rows per thread at most
+struct FlatTri { double l, id, u, g[kRowsMax + 1], h[kRowsMax + 1]; int i0; };   // g[q] = (-l)^q, h[q] = (-u id)^q
+struct FlatPen {
+    double p1, p2, q1, q2, id;
+    double f1[kRowsMax], f2[kRowsMax], b1[kRowsMax], b2[kRowsMax];   // response of row q to the carry's components
+    int i0;
+};
+struct Flat { FlatTri d1, d2; FlatPen f; };
+__constant__ Flat c_f;     // identical for every batch
+
 struct Tabs {
     const double *L1, *I1, *U1;       // first-derivative system: multiplier, 1/pivot, upper
     const double *L2, *I2, *U2;       // second-derivative system
     const double *P1, *P2, *Q1, *Q2, *IF;   // filter system
     const double *T1, *T2;            // tails [(nmax+1)][kTail][3]
     const double *TF;                 // tail  [(nmax+1)][kTail][5]
+    int rows;                         // rows of the prefix tables
 };
 
 struct Batch {
@@ -69,12 +90,17 @@ struct Batch {
 };
 
 // ---- factor access ------------------------------------------------------------
-__device__ __forceinline__ double tri_f(const double *pre, const double *tail, int n, int i, int k) {
-    return i >= n - kTail ? __ldg(tail + ((size_t)n * kTail + (i - (n - kTail))) * 3 + k) : __ldg(pre + i);
-}
-__device__ __forceinline__ double pen_f(const double *pre, const double *tail, int n, int i, int k) {
-    return i >= n - kTail ? __ldg(tail + ((size_t)n * kTail + (i - (n - kTail))) * 5 + k) : __ldg(pre + i);
-}
+// A CTA's copy of the factors in shared memory: of each quantity the first PR
+// rows (the same for every line), the interior value and the line's last kTail
+// rows.  The threads at the line's ends read them in every solve; from global
+// memory their loads held up the whole CTA.
+constexpr int kPrTri = 64, kPrPen = 128;
+template <int NQ, int PR> struct Factors {
+    double v[NQ][PR + 1 + kTail];
+    __device__ __forceinline__ static int row(int i, int n) { return i >= n - kTail ? PR + 1 + i - (n - kTail) : min(i, PR); }
+};
+using FacTri = Factors<3, kPrTri>;   // multiplier, 1/pivot, upper
+using FacPen = Factors<5, kPrPen>;   // p1, p2, q1, q2, id
 
 // ---- block scans of affine carry maps -----------------------------------------
 // scalar map c -> A + G c; "a then b" composes to (Ab + Gb Aa, Gb Ga)
@@ -164,128 +190,217 @@ __device__ __forceinline__ M block_scan_excl(M m, M *sh) {
 // ---- banded solves of one line (rows a..a+cnt-1 of this thread) ---------------
 // Tridiagonal system with factors (l, 1/pivot, upper): forward
 // r'_i = r_i - l_i r'_{i-1}, backward x_i = (r'_i - u_i x_{i+1}) / pivot_i.
-template <int SMAX, int T>
-__device__ __forceinline__ void tri_solve(double (&r)[SMAX], int a, int cnt, int n, const double *L,
-                                          const double *I, const double *U, const double *tail, Map1 *sh) {
-    double v = 0.0, g = 1.0;
+// Each thread runs its rows with zero carries and publishes its end value and
+// the factor it passes a carry on with; the carry is then summed over the
+// threads whose rows reach (56 rows: 0.38^56 < 1e-23), one barrier per
+// direction.
+constexpr int kReach = 56;
+template <int SMAX>
+__device__ __forceinline__ void tri_solve(double (&r)[SMAX], int a, int cnt, int n, const FlatTri &F, const FacTri &fac,
+                                          int Sr, Map1 *ef, Map1 *eb) {
+    const int t = threadIdx.x, reach = (kReach + Sr - 1) / Sr;
+    const bool flat = a >= F.i0 && a + cnt <= n - kTail;
+    double g = 1.0;
+    if (flat) {
+#pragma unroll
+        for (int q = 1; q < SMAX; q++)
+            if (q < cnt) r[q] = fma(-F.l, r[q - 1], r[q]);
+        g = F.g[cnt];
+    } else {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) {
+                const int i = a + q;
+                const double l = fac.v[0][fac.row(i, n)];
+                v = fma(-l, v, r[q]);
+                r[q] = v;
+                g = -l * g;
+            }
+    }
+    double end = 0.0;
 #pragma unroll
     for (int q = 0; q < SMAX; q++)
-        if (q < cnt) {
-            int i = a + q;
-            double l = i == 0 ? 0.0 : tri_f(L, tail, n, i, 0);
-            v = fma(-l, v, r[q]);
-            r[q] = v;
-            g = -l * g;
-        }
-    Map1 m = cnt > 0 ? Map1{v, g} : Map1{0.0, 1.0};
-    Map1 ex = block_scan_excl<Map1, true, T>(m, sh);
-    const double cin = ex.A;
-    g = 1.0;
+        if (q == cnt - 1) end = r[q];
+    ef[t] = Map1{end, g};
+    __syncthreads();
+    double cin = 0.0;
+    for (int k = min(t, reach); k > 0; k--) { const Map1 m = ef[t - k]; cin = fma(m.G, cin, m.A); }
+    double h = 1.0;
+    if (flat) {
 #pragma unroll
-    for (int q = 0; q < SMAX; q++)
-        if (q < cnt) {
-            int i = a + q;
-            double l = i == 0 ? 0.0 : tri_f(L, tail, n, i, 0);
-            g = -l * g;
-            r[q] = fma(g, cin, r[q]);
-        }
-    double x = 0.0, h = 1.0;
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) r[q] = fma(F.g[q + 1], cin, r[q]);
+        const double ui = -F.u * F.id;
+        double x = 0.0;
 #pragma unroll
-    for (int q = SMAX - 1; q >= 0; q--)
-        if (q < cnt) {
-            int i = a + q;
-            double u = i == n - 1 ? 0.0 : tri_f(U, tail, n, i, 2);
-            double id = tri_f(I, tail, n, i, 1);
-            x = fma(-u, x, r[q]) * id;
-            r[q] = x;
-            h = -u * id * h;
-        }
-    Map1 mb = cnt > 0 ? Map1{x, h} : Map1{0.0, 1.0};
-    Map1 eb = block_scan_excl<Map1, false, T>(mb, sh);
-    const double ein = eb.A;
-    h = 1.0;
+        for (int q = SMAX - 1; q >= 0; q--)
+            if (q < cnt) { x = fma(ui, x, r[q] * F.id); r[q] = x; }
+        h = F.h[cnt];
+    } else {
+        g = 1.0;
 #pragma unroll
-    for (int q = SMAX - 1; q >= 0; q--)
-        if (q < cnt) {
-            int i = a + q;
-            double u = i == n - 1 ? 0.0 : tri_f(U, tail, n, i, 2);
-            double id = tri_f(I, tail, n, i, 1);
-            h = -u * id * h;
-            r[q] = fma(h, ein, r[q]);
-        }
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) {
+                const int i = a + q;
+                const double l = fac.v[0][fac.row(i, n)];
+                g = -l * g;
+                r[q] = fma(g, cin, r[q]);
+            }
+        double x = 0.0;
+#pragma unroll
+        for (int q = SMAX - 1; q >= 0; q--)
+            if (q < cnt) {
+                const int i = a + q;
+                const double u = fac.v[2][fac.row(i, n)];
+                const double id = fac.v[1][fac.row(i, n)];
+                x = fma(-u, x, r[q]) * id;
+                r[q] = x;
+                h = -u * id * h;
+            }
+    }
+    eb[t] = Map1{cnt > 0 ? r[0] : 0.0, h};
+    __syncthreads();
+    double ein = 0.0;
+    for (int k = min((int)blockDim.x - 1 - t, reach); k > 0; k--) { const Map1 m = eb[t + k]; ein = fma(m.G, ein, m.A); }
+    if (flat) {
+#pragma unroll
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) r[q] = fma(F.h[cnt - q], ein, r[q]);
+    } else {
+        h = 1.0;
+#pragma unroll
+        for (int q = SMAX - 1; q >= 0; q--)
+            if (q < cnt) {
+                const int i = a + q;
+                const double u = fac.v[2][fac.row(i, n)];
+                const double id = fac.v[1][fac.row(i, n)];
+                h = -u * id * h;
+                r[q] = fma(h, ein, r[q]);
+            }
+    }
 }
 
 // Pentadiagonal system with the elimination order of pentadiagonal_serial:
 // r'_i = (r_i - p2_i r'_{i-2}) - p1_i r'_{i-1};
 // x_i = ((r'_i - q1_i x_{i+1}) - q2_i x_{i+2}) * id_i.
 template <int SMAX, int T>
-__device__ __forceinline__ void pen_solve(double (&r)[SMAX], int a, int cnt, int n, const Tabs *__restrict__ tb, Map2 *sh) {
+__device__ __forceinline__ void pen_solve(double (&r)[SMAX], int a, int cnt, int n, const FacPen &fac, Map2 *sh) {
+    const FlatPen &F = c_f.f;
+    const bool flat = a >= F.i0 && a + cnt <= n - kTail && cnt > 1;
     // forward: state (r'_{i-1}, r'_{i-2}); local run plus the responses to
     // the incoming state's two components
     double s1 = 0.0, s2 = 0.0, e11 = 1.0, e12 = 0.0, e21 = 0.0, e22 = 1.0;   // e_k: response to unit c_k
+    if (flat) {
 #pragma unroll
-    for (int q = 0; q < SMAX; q++)
-        if (q < cnt) {
-            int i = a + q;
-            double p1 = i == 0 ? 0.0 : pen_f(tb->P1, tb->TF, n, i, 0);
-            double p2 = i < 2 ? 0.0 : pen_f(tb->P2, tb->TF, n, i, 1);
-            double v = fma(-p1, s1, fma(-p2, s2, r[q]));
-            double w1 = fma(-p1, e11, -p2 * e21);   // response of row i to c1
-            double w2 = fma(-p1, e12, -p2 * e22);   // to c2
-            r[q] = v;
-            s2 = s1; s1 = v;
-            e21 = e11; e22 = e12; e11 = w1; e12 = w2;
-        }
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) {
+                const double v = fma(-F.p1, s1, fma(-F.p2, s2, r[q]));
+                r[q] = v;
+                s2 = s1; s1 = v;
+            }
+        e11 = F.f1[cnt - 1]; e12 = F.f2[cnt - 1]; e21 = F.f1[cnt - 2]; e22 = F.f2[cnt - 2];
+    } else {
+#pragma unroll
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) {
+                int i = a + q;
+                double p1 = fac.v[0][fac.row(i, n)];
+                double p2 = fac.v[1][fac.row(i, n)];
+                double v = fma(-p1, s1, fma(-p2, s2, r[q]));
+                double w1 = fma(-p1, e11, -p2 * e21);   // response of row i to c1
+                double w2 = fma(-p1, e12, -p2 * e22);   // to c2
+                r[q] = v;
+                s2 = s1; s1 = v;
+                e21 = e11; e22 = e12; e11 = w1; e12 = w2;
+            }
+    }
     // outgoing state (r'_{b-1}, r'_{b-2}) = A + M c
     Map2 m = cnt > 0 ? Map2{s1, s2, e11, e12, e21, e22} : Map2{0.0, 0.0, 1.0, 0.0, 0.0, 1.0};
     Map2 ex = block_scan_excl<Map2, true, T>(m, sh);
     const double c1 = ex.A0, c2 = ex.A1;
-    e11 = 1.0; e12 = 0.0; e21 = 0.0; e22 = 1.0;
+    if (flat) {
 #pragma unroll
-    for (int q = 0; q < SMAX; q++)
-        if (q < cnt) {
-            int i = a + q;
-            double p1 = i == 0 ? 0.0 : pen_f(tb->P1, tb->TF, n, i, 0);
-            double p2 = i < 2 ? 0.0 : pen_f(tb->P2, tb->TF, n, i, 1);
-            double w1 = fma(-p1, e11, -p2 * e21);
-            double w2 = fma(-p1, e12, -p2 * e22);
-            e21 = e11; e22 = e12; e11 = w1; e12 = w2;
-            r[q] = fma(w1, c1, fma(w2, c2, r[q]));
-        }
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) r[q] = fma(F.f1[q], c1, fma(F.f2[q], c2, r[q]));
+    } else {
+        e11 = 1.0; e12 = 0.0; e21 = 0.0; e22 = 1.0;
+#pragma unroll
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) {
+                int i = a + q;
+                double p1 = fac.v[0][fac.row(i, n)];
+                double p2 = fac.v[1][fac.row(i, n)];
+                double w1 = fma(-p1, e11, -p2 * e21);
+                double w2 = fma(-p1, e12, -p2 * e22);
+                e21 = e11; e22 = e12; e11 = w1; e12 = w2;
+                r[q] = fma(w1, c1, fma(w2, c2, r[q]));
+            }
+    }
     // backward: state (x_{i+1}, x_{i+2})
     double x1 = 0.0, x2 = 0.0;
     double f11 = 1.0, f12 = 0.0, f21 = 0.0, f22 = 1.0;
+    if (flat) {
 #pragma unroll
-    for (int q = SMAX - 1; q >= 0; q--)
-        if (q < cnt) {
-            int i = a + q;
-            double q1 = i >= n - 1 ? 0.0 : pen_f(tb->Q1, tb->TF, n, i, 2);
-            double q2 = i >= n - 2 ? 0.0 : pen_f(tb->Q2, tb->TF, n, i, 3);
-            double id = pen_f(tb->IF, tb->TF, n, i, 4);
-            double v = fma(-q2, x2, fma(-q1, x1, r[q])) * id;
-            double w1 = fma(-q2, f21, -q1 * f11) * id;
-            double w2 = fma(-q2, f22, -q1 * f12) * id;
-            r[q] = v;
-            x2 = x1; x1 = v;
-            f21 = f11; f22 = f12; f11 = w1; f12 = w2;
-        }
+        for (int q = SMAX - 1; q >= 0; q--)
+            if (q < cnt) {
+                const double v = fma(-F.q2, x2, fma(-F.q1, x1, r[q])) * F.id;
+                r[q] = v;
+                x2 = x1; x1 = v;
+            }
+        f11 = F.b1[cnt - 1]; f12 = F.b2[cnt - 1]; f21 = F.b1[cnt - 2]; f22 = F.b2[cnt - 2];
+    } else {
+#pragma unroll
+        for (int q = SMAX - 1; q >= 0; q--)
+            if (q < cnt) {
+                int i = a + q;
+                double q1 = fac.v[2][fac.row(i, n)];
+                double q2 = fac.v[3][fac.row(i, n)];
+                double id = fac.v[4][fac.row(i, n)];
+                double v = fma(-q2, x2, fma(-q1, x1, r[q])) * id;
+                double w1 = fma(-q2, f21, -q1 * f11) * id;
+                double w2 = fma(-q2, f22, -q1 * f12) * id;
+                r[q] = v;
+                x2 = x1; x1 = v;
+                f21 = f11; f22 = f12; f11 = w1; f12 = w2;
+            }
+    }
     Map2 mb = cnt > 0 ? Map2{x1, x2, f11, f12, f21, f22} : Map2{0.0, 0.0, 1.0, 0.0, 0.0, 1.0};
     Map2 eb = block_scan_excl<Map2, false, T>(mb, sh);
     const double d1 = eb.A0, d2 = eb.A1;
-    f11 = 1.0; f12 = 0.0; f21 = 0.0; f22 = 1.0;
+    if (flat) {
 #pragma unroll
-    for (int q = SMAX - 1; q >= 0; q--)
-        if (q < cnt) {
-            int i = a + q;
-            double q1 = i >= n - 1 ? 0.0 : pen_f(tb->Q1, tb->TF, n, i, 2);
-            double q2 = i >= n - 2 ? 0.0 : pen_f(tb->Q2, tb->TF, n, i, 3);
-            double id = pen_f(tb->IF, tb->TF, n, i, 4);
-            double w1 = fma(-q2, f21, -q1 * f11) * id;
-            double w2 = fma(-q2, f22, -q1 * f12) * id;
-            f21 = f11; f22 = f12; f11 = w1; f12 = w2;
-            r[q] = fma(w1, d1, fma(w2, d2, r[q]));
-        }
+        for (int q = 0; q < SMAX; q++)
+            if (q < cnt) r[q] = fma(F.b1[cnt - 1 - q], d1, fma(F.b2[cnt - 1 - q], d2, r[q]));
+    } else {
+        f11 = 1.0; f12 = 0.0; f21 = 0.0; f22 = 1.0;
+#pragma unroll
+        for (int q = SMAX - 1; q >= 0; q--)
+            if (q < cnt) {
+                int i = a + q;
+                double q1 = fac.v[2][fac.row(i, n)];
+                double q2 = fac.v[3][fac.row(i, n)];
+                double id = fac.v[4][fac.row(i, n)];
+                double w1 = fma(-q2, f21, -q1 * f11) * id;
+                double w2 = fma(-q2, f22, -q1 * f12) * id;
+                f21 = f11; f22 = f12; f11 = w1; f12 = w2;
+                r[q] = fma(w1, d1, fma(w2, d2, r[q]));
+            }
+    }
 }
+
+// ---- the staged line ----------------------------------------------------------
+// Row i of the line in work sits at X[i + i / Sr], one unused value behind each
+// thread's Sr rows: lanes then read and write their segments an odd number of
+// values apart (no bank conflicts; without the gaps segments of 8 rows hit two
+// banks), and consecutive rows are next to each other for the passes that go
+// through the line row by row.
+struct Line {
+    double *X;
+    unsigned inv;                    // ceil(2^16 / Sr): i / Sr = i inv >> 16 for i < 4096, Sr <= 16
+    __device__ __forceinline__ Line(double *x, int Sr) : X(x), inv((65536u + Sr - 1) / Sr) {}
+    __device__ __forceinline__ double &operator[](int i) const { return X[i + (int)(((unsigned)i * inv) >> 16)]; }
+};
 
 // ---- explicit right-hand sides from the staged line X -------------------------
 enum Op { OP_D1 = 0, OP_D2, OP_FILT, OP_GAUSS, OP_RHS, OP_HYPER };
@@ -294,7 +409,7 @@ enum Op { OP_D1 = 0, OP_D2, OP_FILT, OP_GAUSS, OP_RHS, OP_HYPER };
 // DFDX src/derivCDopt6_radial.f:703-760, D2FDX2 :862-918,
 // Compact_Filter_X src/filters_nonperiodic.f:479-589 and
 // Gaussian_Filter_X :1108-1221 (symmetric reflection at both ends)
-__device__ __noinline__ double boundary_row(int op, int i, const double *X, int n, double fac) {
+__device__ __noinline__ double boundary_row(int op, int i, const Line X, int n, double fac) {
     if (op == OP_D1) {
         if (i >= 3 && i <= n - 4) return fac * (c_k.b1 * (X[i + 2] - X[i - 2]) + c_k.a1 * (X[i + 1] - X[i - 1]));
         if (i == 2) return fac * (c_k.cl3 * (X[4] - X[0]) + c_k.cl4 * (X[3] - X[1]));
@@ -352,29 +467,32 @@ __device__ __noinline__ double boundary_row(int op, int i, const double *X, int 
            g[1] * (f(i + 1) + f(i - 1)) + g[0] * X[i];
 }
 
-// explicit right-hand side of rows a..a+cnt-1 (interior rows inline)
+// explicit right-hand side of rows a..a+cnt-1 (interior rows from a window of
+// the thread's rows and four on either side)
 template <int SMAX>
-__device__ __forceinline__ void rhs_rows(double (&r)[SMAX], int op, const double *X, int a, int cnt, int n,
-                                         double fac) {
+__device__ __forceinline__ void rhs_rows(double (&r)[SMAX], int op, const Line &X, int a, int cnt, int n, double fac) {
+    double w[SMAX + 8];
+    const int lo = op <= OP_D2 ? 2 : 4;
+#pragma unroll
+    for (int q = 0; q < SMAX + 8; q++)
+        if (q >= 4 - lo && q < cnt + 4 + lo) w[q] = X[max(0, min(n - 1, a + q - 4))];
 #pragma unroll
     for (int q = 0; q < SMAX; q++)
         if (q < cnt) {
             const int i = a + q;
-            double w;
+            auto x = [&](int k) { return w[q + 4 + k]; };
             if (i >= 4 && i <= n - 5) {
-                if (op == OP_D1) w = fac * (c_k.b1 * (X[i + 2] - X[i - 2]) + c_k.a1 * (X[i + 1] - X[i - 1]));
-                else if (op == OP_D2)
-                    w = fac * (c_k.b2 * (X[i + 2] + X[i - 2]) + c_k.a2 * (X[i + 1] + X[i - 1]) - c_k.d2 * X[i]);
+                if (op == OP_D1) r[q] = fac * (c_k.b1 * (x(2) - x(-2)) + c_k.a1 * (x(1) - x(-1)));
+                else if (op == OP_D2) r[q] = fac * (c_k.b2 * (x(2) + x(-2)) + c_k.a2 * (x(1) + x(-1)) - c_k.d2 * x(0));
                 else if (op == OP_FILT)
-                    w = c_k.fa4 * (X[i + 4] + X[i - 4]) + c_k.fa3 * (X[i + 3] + X[i - 3]) + c_k.fa2 * (X[i + 2] + X[i - 2]) +
-                        c_k.fa1 * (X[i + 1] + X[i - 1]) + c_k.fa0 * X[i];
+                    r[q] = c_k.fa4 * (x(4) + x(-4)) + c_k.fa3 * (x(3) + x(-3)) + c_k.fa2 * (x(2) + x(-2)) +
+                           c_k.fa1 * (x(1) + x(-1)) + c_k.fa0 * x(0);
                 else
-                    w = c_k.g[4] * (X[i + 4] + X[i - 4]) + c_k.g[3] * (X[i + 3] + X[i - 3]) +
-                        c_k.g[2] * (X[i + 2] + X[i - 2]) + c_k.g[1] * (X[i + 1] + X[i - 1]) + c_k.g[0] * X[i];
+                    r[q] = c_k.g[4] * (x(4) + x(-4)) + c_k.g[3] * (x(3) + x(-3)) + c_k.g[2] * (x(2) + x(-2)) +
+                           c_k.g[1] * (x(1) + x(-1)) + c_k.g[0] * x(0);
             } else {
-                w = boundary_row(op, i, X, n, fac);
+                r[q] = boundary_row(op, i, X, n, fac);
             }
-            r[q] = w;
         }
 }
 
@@ -402,137 +520,176 @@ __device__ __forceinline__ double radius(int i, const Geo &g) {
 template <int T, int SMAX>
 struct Smem {
     static constexpr int N = T * SMAX;
-    double X[N];          // staged input line
-    double Y[N];          // line-operator result
+    double X[N + T];      // the line in work (see Line); a line operator leaves its result there
     double Ru[N], Rr[N], Rs[N];   // dQ of the stage (u, rho, s)
     double Du[N];         // -du/dr (DFDX(u, -1)), reused by Hyper_RHS
-    Map2 sc[2 * (T / 32)];   // scan scratch (also holds Map1 values)
+    Map1 ef[T], eb[T];       // tridiagonal carries
+    Map2 sc[2 * (T / 32)];   // filter scan scratch
+    FacTri t1, t2;           // first and second derivative
+    FacPen tf;
     double red[T / 32][4];
     int prob;
 };
 
-// One line operator on the staged line S.X; this thread's rows of the result
-// go to S.Y (rows a..a+cnt-1, read back by the same thread).  DFDX flips the
+// the factors of a line of n rows (their first rows and interior values once
+// per CTA); the caller synchronises
+template <int T, int SMAX>
+__device__ __forceinline__ void fill_tails(Smem<T, SMAX> &S, int n, const Tabs *__restrict__ tb) {
+    const int t = threadIdx.x;
+    if (t < 3 * kTail) {
+        const int k = t / kTail, q = t % kTail;
+        const bool end = k == 2 && q == kTail - 1;                 // the last row has no upper entry
+        S.t1.v[k][kPrTri + 1 + q] = end ? 0.0 : tb->T1[((size_t)n * kTail + q) * 3 + k];
+        S.t2.v[k][kPrTri + 1 + q] = end ? 0.0 : tb->T2[((size_t)n * kTail + q) * 3 + k];
+    }
+    if (t >= 32 && t < 32 + 5 * kTail) {
+        const int k = (t - 32) / kTail, q = (t - 32) % kTail;
+        const bool end = (k == 2 && q == kTail - 1) || (k == 3 && q >= kTail - 2);
+        S.tf.v[k][kPrPen + 1 + q] = end ? 0.0 : tb->TF[((size_t)n * kTail + q) * 5 + k];
+    }
+}
+template <int T, int SMAX>
+__device__ __forceinline__ void fill_heads(Smem<T, SMAX> &S, const Tabs *__restrict__ tb) {
+    const double *p1[3] = {tb->L1, tb->I1, tb->U1}, *p2[3] = {tb->L2, tb->I2, tb->U2};
+    const double *pf[5] = {tb->P1, tb->P2, tb->Q1, tb->Q2, tb->IF};
+    const double c1[3] = {c_f.d1.l, c_f.d1.id, c_f.d1.u}, c2[3] = {c_f.d2.l, c_f.d2.id, c_f.d2.u};
+    const double cf[5] = {c_f.f.p1, c_f.f.p2, c_f.f.q1, c_f.f.q2, c_f.f.id};
+    for (int i = threadIdx.x; i <= kPrTri; i += T)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            S.t1.v[k][i] = i >= c_f.d1.i0 ? c1[k] : (k == 0 && i == 0) ? 0.0 : i < tb->rows ? p1[k][i] : 0.0;
+            S.t2.v[k][i] = i >= c_f.d2.i0 ? c2[k] : (k == 0 && i == 0) ? 0.0 : i < tb->rows ? p2[k][i] : 0.0;
+        }
+    for (int i = threadIdx.x; i <= kPrPen; i += T)
+#pragma unroll
+        for (int k = 0; k < 5; k++)
+            S.tf.v[k][i] = i >= c_f.f.i0 ? cf[k] : (k < 2 && i <= k) ? 0.0 : i < tb->rows ? pf[k][i] : 0.0;
+}
+
+// One line operator on the staged line, in place; the caller synchronises
+// before it reads other threads' rows.  DFDX flips the
 // sign on the left half (dF/dr = -dF/dx for II <= Nx/2,
 // src/derivCDopt6_radial.f:772-784).  fac: cadd*sx*(n-1) (DFDX) or
-// (n-1)^2*sx^2 (D2FDX2).
+// (n-1)^2*sx^2 (D2FDX2).  mag: the magnitude of the result.
 template <int T, int SMAX>
-__device__ __noinline__ void line_op(Smem<T, SMAX> &S, int op, int n, double fac, const Tabs *__restrict__ tb) {
+__device__ __noinline__ void line_op(Smem<T, SMAX> &S, int op, int n, double fac, bool mag = false) {
     const int t = threadIdx.x, Sr = (n + T - 1) / T, a = t * Sr, cnt = max(0, min(Sr, n - a));
+    const Line X(S.X, Sr);
     double r[SMAX];
-    rhs_rows<SMAX>(r, op, S.X, a, cnt, n, fac);
-    if (op == OP_D1 || op == OP_D2) {
-        const bool d1 = op == OP_D1;
-        tri_solve<SMAX, T>(r, a, cnt, n, d1 ? tb->L1 : tb->L2, d1 ? tb->I1 : tb->I2, d1 ? tb->U1 : tb->U2,
-                           d1 ? tb->T1 : tb->T2, reinterpret_cast<Map1 *>(S.sc));
-    } else if (op == OP_FILT) {
-        pen_solve<SMAX, T>(r, a, cnt, n, tb, S.sc);
-    }
+    rhs_rows<SMAX>(r, op, X, a, cnt, n, fac);
+    if (op == OP_D1) tri_solve<SMAX>(r, a, cnt, n, c_f.d1, S.t1, Sr, S.ef, S.eb);
+    else if (op == OP_D2) tri_solve<SMAX>(r, a, cnt, n, c_f.d2, S.t2, Sr, S.ef, S.eb);
+    else if (op == OP_FILT) pen_solve<SMAX, T>(r, a, cnt, n, S.tf, S.sc);
+    else __syncthreads();            // (the solves have barriers) every thread has read its rows
+    double *out = S.X + t * (Sr + 1);
 #pragma unroll
     for (int q = 0; q < SMAX; q++)
-        if (q < cnt) S.Y[a + q] = (op == OP_D1 && a + q + 1 <= n / 2) ? -r[q] : r[q];
+        if (q < cnt) {
+            const double v = (op == OP_D1 && a + q + 1 <= n / 2) ? -r[q] : r[q];
+            out[q] = mag ? fabs(v) : v;
+        }
 }
 
-// stage a line into S.X: X[i] = f(i) for i < n, then synchronise.  The
-// caller guarantees every earlier reader of X has passed a barrier.
-template <int T, int SMAX, class F>
-__device__ __forceinline__ void stage(Smem<T, SMAX> &S, int n, F f) {
-    for (int i = threadIdx.x; i < n; i += T) S.X[i] = f(i);
-    __syncthreads();
-}
-
-// this thread's rows a..a+cnt-1
-#define RAD_ROWS(T_, n_)                                                                       \
-    const int Sr_ = ((n_) + (T_) - 1) / (T_), a = (int)threadIdx.x * Sr_, cnt = max(0, min(Sr_, (n_) - a))
+// Row-by-row passes over a line: thread t takes rows t, t + T, ... (neighbouring
+// threads on neighbouring rows, in shared and in global memory), the same in
+// every pass, so that a pass may read the result of an operator and stage the
+// next operand without a barrier in between.  Unrolled, with the fields
+// declared not to overlap, for four rows' loads in flight.
+#define RAD_PASS(S_, n_, ...)                                                                   \
+    {                                                                                           \
+        const Line X((S_).X, ((n_) + T - 1) / T);                                               \
+        _Pragma("unroll 4")                                                                     \
+        for (int i = threadIdx.x; i < (n_); i += T) __VA_ARGS__                                 \
+        __syncthreads();                                                                        \
+    }
 
 // Compute_hyper src/hyper_radial.f:9-62: d4 = D2(D2(u)), hyp = (1, 2e-3) *
 // Gauss(|d4|) * DX^5
 template <int T, int SMAX>
-__device__ __noinline__ void problem_hyper_core(Smem<T, SMAX> &S, const Geo &G, const double *u, double *hyp,
-                                                const Tabs *__restrict__ tb) {
+__device__ __noinline__ void problem_hyper_core(Smem<T, SMAX> &S, const Geo &G, const double *__restrict__ u,
+                                                double *__restrict__ hyp) {
     const int n = G.n;
-    RAD_ROWS(T, n);
-    stage(S, n, [&](int i) { return u[i]; });
-    line_op<T, SMAX>(S, OP_D2, n, G.fac2, tb);
-    __syncthreads();                                        // every read of X is done
-    for (int q = 0; q < cnt; q++) S.X[a + q] = S.Y[a + q];
+    RAD_PASS(S, n, { X[i] = u[i]; })
+    line_op<T, SMAX>(S, OP_D2, n, G.fac2);
     __syncthreads();
-    line_op<T, SMAX>(S, OP_D2, n, G.fac2, tb);
+    line_op<T, SMAX>(S, OP_D2, n, G.fac2, true);
     __syncthreads();
-    for (int q = 0; q < cnt; q++) S.X[a + q] = fabs(S.Y[a + q]);
+    line_op<T, SMAX>(S, OP_GAUSS, n, 0.0);
     __syncthreads();
-    line_op<T, SMAX>(S, OP_GAUSS, n, 0.0, tb);
     const double DX5 = pow(G.DX, 5.0);
-    for (int q = 0; q < cnt; q++) {
-        hyp[a + q] = 1.0 * S.Y[a + q] * DX5;
-        hyp[n + a + q] = 2.0e-3 * S.Y[a + q] * DX5;
-    }
-    __syncthreads();
+    RAD_PASS(S, n, {
+        hyp[i] = 1.0 * X[i] * DX5;
+        hyp[n + i] = 2.0e-3 * X[i] * DX5;
+    })
 }
 
 // RHS_r (src/rhsv_radial.f:30-157) and, when hyper, Hyper_RHS
 // (src/hyper_radial.f:75-187) of one problem: leaves dQ in S.Ru/Rr/Rs and
 // refreshes /HYPER/ (hyp).
 template <int T, int SMAX>
-__device__ __noinline__ void problem_rhs(Smem<T, SMAX> &S, const Geo &G, const double *u, const double *rho,
-                                         const double *s, double *hyp, double gam, int hyper,
-                                         const Tabs *__restrict__ tb) {
+__device__ __noinline__ void problem_rhs(Smem<T, SMAX> &S, const Geo &G, const double *__restrict__ u,
+                                         const double *__restrict__ rho, const double *__restrict__ s, double *hyp, double gam,
+                                         int hyper) {
     const int n = G.n;
-    RAD_ROWS(T, n);
     // d rho/dt = -u d rho/dr  (DFDX(rho, Qrhs4, 1, -1): 0 + W)
-    stage(S, n, [&](int i) { return rho[i]; });
-    line_op<T, SMAX>(S, OP_D1, n, -G.fac1, tb);
-    for (int q = 0; q < cnt; q++) S.Rr[a + q] = S.Y[a + q] * u[a + q];
+    RAD_PASS(S, n, { X[i] = rho[i]; })
+    line_op<T, SMAX>(S, OP_D1, n, -G.fac1);
     __syncthreads();
     // - rho/r^2 d(u r^2)/dr
-    stage(S, n, [&](int i) { double rd = radius(i, G); return u[i] * rd * rd; });
-    line_op<T, SMAX>(S, OP_D1, n, G.fac1, tb);
-    for (int q = 0; q < cnt; q++) {
-        const int i = a + q;
-        double rd = radius(i, G);
-        S.Rr[i] = S.Rr[i] - S.Y[i] * (rho[i] / (rd * rd));
-    }
+    RAD_PASS(S, n, {
+        const double rd = radius(i, G);
+        const double ui = u[i];
+        S.Rr[i] = X[i] * ui;
+        X[i] = ui * rd * rd;
+    })
+    line_op<T, SMAX>(S, OP_D1, n, G.fac1);
     __syncthreads();
     // d u/dt = -u du/dr
-    stage(S, n, [&](int i) { return u[i]; });
-    line_op<T, SMAX>(S, OP_D1, n, -G.fac1, tb);
-    for (int q = 0; q < cnt; q++) { S.Du[a + q] = S.Y[a + q]; S.Ru[a + q] = u[a + q] * S.Y[a + q]; }
+    RAD_PASS(S, n, {
+        const double rd = radius(i, G);
+        S.Rr[i] = S.Rr[i] - X[i] * (rho[i] / (rd * rd));
+        X[i] = u[i];
+    })
+    line_op<T, SMAX>(S, OP_D1, n, -G.fac1);
     __syncthreads();
     // - (dP/dr)/rho,  P = s rho^gamma
-    stage(S, n, [&](int i) { return s[i] * pow(rho[i], gam); });
-    line_op<T, SMAX>(S, OP_D1, n, G.fac1, tb);
-    for (int q = 0; q < cnt; q++) S.Ru[a + q] = S.Ru[a + q] - (S.Y[a + q] / rho[a + q]);
+    RAD_PASS(S, n, {
+        S.Du[i] = X[i];
+        S.Ru[i] = u[i] * X[i];
+        X[i] = s[i] * pow(rho[i], gam);
+    })
+    line_op<T, SMAX>(S, OP_D1, n, G.fac1);
     __syncthreads();
     // d s/dt = -u ds/dr
-    stage(S, n, [&](int i) { return s[i]; });
-    line_op<T, SMAX>(S, OP_D1, n, -G.fac1, tb);
-    for (int q = 0; q < cnt; q++) S.Rs[a + q] = S.Y[a + q] * u[a + q];
+    RAD_PASS(S, n, {
+        S.Ru[i] = S.Ru[i] - (X[i] / rho[i]);
+        X[i] = s[i];
+    })
+    line_op<T, SMAX>(S, OP_D1, n, -G.fac1);
     __syncthreads();
+    RAD_PASS(S, n, { S.Rs[i] = X[i] * u[i]; })
     if (!hyper) return;
-    problem_hyper_core<T, SMAX>(S, G, u, hyp, tb);
-    const double *bh = hyp, *vh = hyp + n;
+    problem_hyper_core<T, SMAX>(S, G, u, hyp);
+    const double *__restrict__ bh = hyp, *__restrict__ vh = hyp + n;
     // 1/r^2 d/dr(r^2 2 nu du/dr)   (du/dr = -Du exactly: DFDX is odd in cadd)
-    stage(S, n, [&](int i) { double rd = radius(i, G); return rd * rd * 2.0 * vh[i] * (-S.Du[i]); });
-    line_op<T, SMAX>(S, OP_D1, n, G.fac1, tb);
-    double qh[SMAX];                          // first Hyper_RHS term of this thread's rows
-#pragma unroll
-    for (int q = 0; q < SMAX; q++)
-        if (q < cnt) { double rd = radius(a + q, G); qh[q] = (1.0 / (rd * rd)) * S.Y[a + q]; }
+    RAD_PASS(S, n, { const double rd = radius(i, G); X[i] = rd * rd * 2.0 * vh[i] * (-S.Du[i]); })
+    line_op<T, SMAX>(S, OP_D1, n, G.fac1);
     __syncthreads();
-    // 1/r^2 d/dr(r^2 (beta - 2/3 nu)(du/dr + 2u/r))
-    stage(S, n, [&](int i) {
-        double rd = radius(i, G);
-        return rd * rd * (bh[i] - (2.0 / 3.0) * vh[i]) * (-S.Du[i] + 2.0 * u[i] / rd);
-    });
-    line_op<T, SMAX>(S, OP_D1, n, G.fac1, tb);
-#pragma unroll
-    for (int q = 0; q < SMAX; q++)
-        if (q < cnt) {
-            double rd = radius(a + q, G);
-            double h = qh[q] + (1.0 / (rd * rd)) * S.Y[a + q];
-            S.Ru[a + q] = S.Ru[a + q] + h;
-        }
+    // 1/r^2 d/dr(r^2 (beta - 2/3 nu)(du/dr + 2u/r)); the first term waits in
+    // Du, whose value the second operand has taken
+    RAD_PASS(S, n, {
+        const double rd = radius(i, G);
+        const double q = (1.0 / (rd * rd)) * X[i];
+        X[i] = rd * rd * (bh[i] - (2.0 / 3.0) * vh[i]) * (-S.Du[i] + 2.0 * u[i] / rd);
+        S.Du[i] = q;
+    })
+    line_op<T, SMAX>(S, OP_D1, n, G.fac1);
     __syncthreads();
+    RAD_PASS(S, n, {
+        const double rd = radius(i, G);
+        const double h = S.Du[i] + (1.0 / (rd * rd)) * X[i];
+        S.Ru[i] = S.Ru[i] + h;
+    })
 }
 
 // block reductions (T/32 partials in S.red)
@@ -570,7 +727,7 @@ __constant__ double c_beta2[6] = {1.1584888181285561688e-1, 3.728769905165286491
 // Compute_CFL + Compute_Tstep (src/lddrk4_nonperiodic_sf.f:7-146, x term),
 // then LDDRK4 (:376-468; no Fix_Pressure: its radial source is not shipped).
 template <int T, int SMAX>
-__device__ __noinline__ void problem_step(Smem<T, SMAX> &S, const Batch &B, int p, const Tabs *__restrict__ tb) {
+__device__ __noinline__ void problem_step(Smem<T, SMAX> &S, const Batch &B, int p) {
     const int n = B.n[p];
     const Geo G = geo(n, B.xl[p]);
     const size_t o = (size_t)B.off[p];
@@ -579,7 +736,6 @@ __device__ __noinline__ void problem_step(Smem<T, SMAX> &S, const Batch &B, int 
     double *hyp = B.hyp + 2 * o;
     const double gam = B.gamma, fac = gam * (gam - 1.0);
     const int t = threadIdx.x;
-    RAD_ROWS(T, n);
     // CFL and hyperviscous limits
     double m2 = 0.0, m3 = INFINITY, m4 = INFINITY;
     const double khug = 2.199, del = G.DX;
@@ -610,25 +766,26 @@ __device__ __noinline__ void problem_step(Smem<T, SMAX> &S, const Batch &B, int 
             else if (B.rk_mode == 1) { al = c_alpha2[K]; be = c_beta2[K]; }
             else { al = 0.0; be = 0.0; }
             const bool first = K == 0;          // QW = 0 at the loop start and alpha(1) = 0
-            problem_rhs<T, SMAX>(S, G, u, rho, s, hyp, gam, B.hyper, tb);
+            problem_rhs<T, SMAX>(S, G, u, rho, s, hyp, gam, B.hyper);
             // update, then filter u, rho, s in place (Compact_Filter x pass)
-            for (int i = t; i < n; i += T) {
-                const double d0 = S.Ru[i], d1 = S.Rr[i], d2 = S.Rs[i];
-                double q0 = first ? dt * d0 : al * wu[i] + dt * d0;
-                double q1 = first ? dt * d1 : al * wr[i] + dt * d1;
-                double q2 = first ? dt * d2 : al * ws[i] + dt * d2;
+            RAD_PASS(S, n, {
+                const double d0 = S.Ru[i];
+                const double d1 = S.Rr[i];
+                const double d2 = S.Rs[i];
+                const double q0 = first ? dt * d0 : al * wu[i] + dt * d0;
+                const double q1 = first ? dt * d1 : al * wr[i] + dt * d1;
+                const double q2 = first ? dt * d2 : al * ws[i] + dt * d2;
                 wu[i] = q0; wr[i] = q1; ws[i] = q2;
-                u[i] = u[i] + be * q0;
+                X[i] = u[i] + be * q0;
                 rho[i] = rho[i] + be * q1;
                 s[i] = s[i] + be * q2;
-            }
-            __syncthreads();
+            })
             for (int f = 0; f < 3; f++) {
-                double *F = f == 0 ? u : (f == 1 ? rho : s);
-                stage(S, n, [&](int i) { return F[i]; });
-                line_op<T, SMAX>(S, OP_FILT, n, 0.0, tb);
-                for (int q = 0; q < cnt; q++) F[a + q] = S.Y[a + q];
+                line_op<T, SMAX>(S, OP_FILT, n, 0.0);
                 __syncthreads();
+                double *F = f == 0 ? u : (f == 1 ? rho : s);
+                const double *next = f == 0 ? rho : s;
+                RAD_PASS(S, n, { F[i] = X[i]; if (f < 2) X[i] = next[i]; })
             }
         }
         tm = tm + dt;
@@ -645,6 +802,7 @@ __global__ void __launch_bounds__(T) k_rad_steps(Batch B, const Tabs *__restrict
                                                    int *queue) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem<T, SMAX> &S = *reinterpret_cast<Smem<T, SMAX> *>(smem_raw);
+    fill_heads(S, tb);
     for (;;) {
         if (threadIdx.x == 0) S.prob = first + atomicAdd(queue, 1);
         __syncthreads();
@@ -652,11 +810,13 @@ __global__ void __launch_bounds__(T) k_rad_steps(Batch B, const Tabs *__restrict
         __syncthreads();
         if (idx >= last) return;
         const int p = B.order[idx];
+        fill_tails(S, B.n[p], tb);
+        __syncthreads();
         if (B.step[p] == 0) {
             const size_t o = (size_t)B.off[p];
-            problem_hyper_core<T, SMAX>(S, geo(B.n[p], B.xl[p]), B.Q + 3 * o, B.hyp + 2 * o, tb);
+            problem_hyper_core<T, SMAX>(S, geo(B.n[p], B.xl[p]), B.Q + 3 * o, B.hyp + 2 * o);
         }
-        for (int it = 0; it < nsteps; it++) problem_step<T, SMAX>(S, B, p, tb);
+        for (int it = 0; it < nsteps; it++) problem_step<T, SMAX>(S, B, p);
     }
 }
 
@@ -670,24 +830,32 @@ __global__ void __launch_bounds__(T) k_rad_op(Batch B, const Tabs *__restrict__ 
     const int n = B.n[p];
     const Geo G = geo(n, B.xl[p]);
     const size_t o = (size_t)B.off[p];
-    RAD_ROWS(T, n);
+    fill_heads(S, tb);
+    fill_tails(S, n, tb);
+    __syncthreads();
     if (op == OP_RHS || op == OP_HYPER) {
         const double *u = F + 3 * o, *rho = u + n, *s = rho + n;
-        problem_rhs<T, SMAX>(S, G, u, rho, s, B.hyp + 2 * o, B.gamma, op == OP_HYPER ? B.hyper : 0, tb);
+        problem_rhs<T, SMAX>(S, G, u, rho, s, B.hyp + 2 * o, B.gamma, op == OP_HYPER ? B.hyper : 0);
         double *R = O1 + 3 * o;
         for (int i = threadIdx.x; i < n; i += T) { R[i] = S.Ru[i]; R[n + i] = S.Rr[i]; R[2 * n + i] = S.Rs[i]; }
         return;
     }
     const double *f = F + o;
-    stage(S, n, [&](int i) { return f[i]; });
+    RAD_PASS(S, n, { X[i] = f[i]; })
     const double fac = op == OP_D1 ? cadd * (1.0 / B.xl[p]) * (double)(n - 1) : G.fac2;
-    line_op<T, SMAX>(S, op, n, fac, tb);
+    line_op<T, SMAX>(S, op, n, fac);
+    __syncthreads();
     double *out = (op == OP_D2 ? O2 : O1) + o;
-    for (int q = 0; q < cnt; q++) out[a + q] = (op == OP_D1 && iadd == 1) ? out[a + q] + S.Y[a + q] : S.Y[a + q];
-    if (op == OP_D2 && iadd == 1) {
+    const bool both = op == OP_D2 && iadd == 1;
+    RAD_PASS(S, n, {
+        const double v = X[i];
+        if (both) X[i] = f[i];
+        out[i] = (op == OP_D1 && iadd == 1) ? out[i] + v : v;
+    })
+    if (both) {
+        line_op<T, SMAX>(S, OP_D1, n, 1.0 * (1.0 / B.xl[p]) * (double)(n - 1));
         __syncthreads();
-        line_op<T, SMAX>(S, OP_D1, n, 1.0 * (1.0 / B.xl[p]) * (double)(n - 1), tb);
-        for (int q = 0; q < cnt; q++) O1[o + a + q] = S.Y[a + q];
+        RAD_PASS(S, n, { O1[o + i] = X[i]; })
     }
 }
 
@@ -751,6 +919,60 @@ static void filt_factor(int n, std::vector<double> f[5]) {
     for (int i = 0; i <= n - 2; i++) f[2][i] = D[i];
     for (int i = 0; i <= n - 3; i++) f[3][i] = E[i];
     for (int i = 0; i < n; i++) f[4][i] = 1.0 / (C[i] + kTiny);
+}
+
+// The interior fixed point of the three systems, from an elimination in long
+// double that starts as every line's does; i0 is the first row whose factors,
+// rounded to double, have reached it.
+static void fill_flat(Flat &f) {
+    typedef long double R;
+    const int NF = 512;
+    std::vector<double> B, C, D;
+    for (int order = 1; order <= 2; order++) {
+        FlatTri &t = order == 1 ? f.d1 : f.d2;
+        deriv_rows(NF, order, B, C, D);
+        std::vector<R> l(NF, 0.0L), c(C.begin(), C.end());
+        for (int i = 1; i < NF; i++) { l[i] = B[i] / c[i - 1]; c[i] = C[i] - D[i - 1] * l[i]; }
+        const int m = NF / 2;
+        t.l = (double)l[m]; t.id = (double)(1.0L / c[m]); t.u = D[m];
+        t.i0 = m;
+        while (t.i0 > 0 && (double)l[t.i0 - 1] == t.l && (double)(1.0L / c[t.i0 - 1]) == t.id && D[t.i0 - 1] == t.u) t.i0--;
+        t.g[0] = t.h[0] = 1.0;
+        for (int q = 1; q <= kRowsMax; q++) { t.g[q] = -t.l * t.g[q - 1]; t.h[q] = -t.u * t.id * t.h[q - 1]; }
+    }
+    const double af = 6.6624e-01, bf = 1.6688e-01, ab = 0.45;
+    std::vector<R> a(NF, bf), b(NF, af), c(NF, 1.0L), d(NF, af), e(NF, bf), k1(NF, 0.0L), k2(NF, 0.0L);
+    auto row = [&](int r, double A, double Bv, double Cv, double Dv, double E) { a[r] = A; b[r] = Bv; c[r] = Cv; d[r] = Dv; e[r] = E; };
+    row(0, 0, 0, 1, 0, 0);
+    row(1, 0, ab, 1, ab, 0);
+    row(2, 0, ab, 1, ab, 0);
+    for (int i = 0; i <= NF - 3; i++) {
+        k1[i] = b[i + 1] / c[i];
+        c[i + 1] -= d[i] * k1[i];
+        d[i + 1] -= e[i] * k1[i];
+        k2[i] = a[i + 2] / c[i];
+        b[i + 2] -= d[i] * k2[i];
+        c[i + 2] -= e[i] * k2[i];
+    }
+    FlatPen &p = f.f;
+    auto is = [&](int i, int m) {
+        return (double)k1[i - 1] == (double)k1[m - 1] && (double)k2[i - 2] == (double)k2[m - 2] && (double)d[i] == (double)d[m] &&
+               (double)e[i] == (double)e[m] && (double)(1.0L / c[i]) == (double)(1.0L / c[m]);
+    };
+    const int m = NF / 2;
+    p.p1 = (double)k1[m - 1]; p.p2 = (double)k2[m - 2]; p.q1 = (double)d[m]; p.q2 = (double)e[m]; p.id = (double)(1.0L / c[m]);
+    p.i0 = m;
+    while (p.i0 > 2 && is(p.i0 - 1, m)) p.i0--;
+    for (int w = 0; w < 2; w++) {
+        double h1 = w == 0 ? 1.0 : 0.0, h2 = 1.0 - h1, x1 = h1, x2 = h2;
+        for (int q = 0; q < kRowsMax; q++) {
+            const double v = std::fma(-p.p1, h1, -p.p2 * h2), x = std::fma(-p.q2, x2, -p.q1 * x1) * p.id;
+            (w == 0 ? p.f1 : p.f2)[q] = v;
+            (w == 0 ? p.b1 : p.b2)[q] = x;
+            h2 = h1; h1 = v;
+            x2 = x1; x1 = x;
+        }
+    }
 }
 
 static void fill_k(K &k) {
@@ -929,6 +1151,8 @@ int st_radial_create(const st_radial_params *p, int nprob, const int *n, const d
         return bail(ST_E_CUDA, "stream/event creation");
     h->stream = h->own;
     fill_k(h->k);
+    Flat flat;
+    fill_flat(flat);
     // factor tables: universal prefixes from the longest length, tails per length
     const int NM = std::max(h->nmax, kMinN);
     std::vector<double> B, C, D, l1, i1, u1, l2, i2, u2, F[5];
@@ -995,10 +1219,12 @@ int st_radial_create(const st_radial_params *p, int nprob, const int *n, const d
     h->tb.L1 = T0 + o_l1; h->tb.I1 = T0 + o_i1; h->tb.U1 = T0 + o_u1;
     h->tb.L2 = T0 + o_l2; h->tb.I2 = T0 + o_i2; h->tb.U2 = T0 + o_u2;
     h->tb.P1 = T0 + o_f[0]; h->tb.P2 = T0 + o_f[1]; h->tb.Q1 = T0 + o_f[2]; h->tb.Q2 = T0 + o_f[3]; h->tb.IF = T0 + o_f[4];
+    h->tb.rows = NM;
     h->tb.T1 = T0 + o_t1; h->tb.T2 = T0 + o_t2; h->tb.TF = T0 + o_tf;
     if (cudaMalloc((void **)&h->dtb, sizeof(Tabs)) != cudaSuccess ||
         cudaMemcpy(h->dtb, &h->tb, sizeof(Tabs), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpyToSymbol(c_k, &h->k, sizeof(K)) != cudaSuccess) {
+        cudaMemcpyToSymbol(c_k, &h->k, sizeof(K)) != cudaSuccess ||
+        cudaMemcpyToSymbol(c_f, &flat, sizeof(Flat)) != cudaSuccess) {
         cudaGetLastError();
         return bail(ST_E_CUDA, "uploading the radial constants");
     }
