@@ -119,29 +119,59 @@ __device__ __forceinline__ int find_bin(const double *r, int na, double rad) {
     return lo;
 }
 
-// Ur of every cell (pproc/pproc_mf.f:98-121) and the shell sums of Ur and Y
-// over the bins of Compute_Shell_Avg (table rs): per-block shared histograms
+// velocity and Ur of a cell (pproc/pproc_mf.f:98-121); both passes form them
+// from Q, which is as many fields as the stored ones would be
+struct CellU { double u1, u2, u3, rad, ur; };
+__device__ __forceinline__ CellU cell_velocity(const double *Q, const Grid &g, size_t n3, size_t p, int i, int j, int k) {
+    CellU c;
+    const double tmp = 1.0 / Q[3 * n3 + p];
+    c.u1 = Q[p] * tmp; c.u2 = Q[n3 + p] * tmp; c.u3 = Q[2 * n3 + p] * tmp;
+    c.rad = g.rad(i, j, k);
+    c.ur = (i == 0 && j == 0 && k == 0)
+               ? 0.0
+               : (g.cor(0, i) / c.rad) * c.u1 + (g.cor(1, j) / c.rad) * c.u2 + (g.cor(2, k) / c.rad) * c.u3;
+    return c;
+}
+
+// The shell sums of Ur and Y over the bins of Compute_Shell_Avg (table rs):
+// per-block shared histograms.  Neighbouring cells of a row fall into the same
+// few bins, so a warp first sums each run of lanes with one bin (a segmented
+// scan) and the last lane of the run adds it: a few shared-memory additions per
+// warp instead of 96 that collide (192^3: 199 us with one per cell and four
+// fields stored).
 __global__ void k_shell_sums(const double *Q, const double *Y, Grid g, int My, int Mz, size_t n3,
-                             const double *rs, int na, double *U, double *Ur, double *bsum, unsigned long long *bcnt) {
+                             const double *rs, int na, double *bsum, unsigned long long *bcnt) {
     extern __shared__ double hs[];   // [2][na] sums, then [na] counts (as doubles)
     for (int q = threadIdx.x; q < 3 * na; q += blockDim.x) hs[q] = 0.0;
     __syncthreads();
-    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n3; p += (size_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        cell_ijk(p, My, Mz, i, j, k);
-        double tmp = 1.0 / Q[3 * n3 + p];
-        double u1 = Q[p] * tmp, u2 = Q[n3 + p] * tmp, u3 = Q[2 * n3 + p] * tmp;
-        U[p] = u1; U[n3 + p] = u2; U[2 * n3 + p] = u3;
-        double rad = g.rad(i, j, k);
-        double ur = (i == 0 && j == 0 && k == 0)
-                        ? 0.0
-                        : (g.cor(0, i) / rad) * u1 + (g.cor(1, j) / rad) * u2 + (g.cor(2, k) / rad) * u3;
-        Ur[p] = ur;
-        int M = find_bin(rs, na, rad);
-        if (M >= 0) {
+    const int lane = threadIdx.x & 31;
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    const size_t p0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x - lane;      // the warp's first cell
+    for (size_t w = p0; w < n3; w += step) {
+        const size_t p = w + lane;
+        int M = -1;
+        double ur = 0.0, y = 0.0;
+        if (p < n3) {
+            int i, j, k;
+            cell_ijk(p, My, Mz, i, j, k);
+            const CellU c = cell_velocity(Q, g, n3, p, i, j, k);
+            M = find_bin(rs, na, c.rad);
+            ur = c.ur;
+            y = Y[p];
+        }
+        const int prev = __shfl_up_sync(0xffffffffu, M, 1);
+        const bool head = lane == 0 || prev != M;
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));      // first lane of the run
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const double a = __shfl_up_sync(0xffffffffu, ur, d), b = __shfl_up_sync(0xffffffffu, y, d);
+            if (lane - d >= first) { ur += a; y += b; }
+        }
+        if (M >= 0 && (lane == 31 || (heads >> (lane + 1) & 1u))) {
             atomicAdd(&hs[M], ur);
-            atomicAdd(&hs[na + M], Y[p]);
-            atomicAdd(&hs[2 * na + M], 1.0);
+            atomicAdd(&hs[na + M], y);
+            atomicAdd(&hs[2 * na + M], (double)(lane - first + 1));
         }
     }
     __syncthreads();
@@ -154,23 +184,25 @@ __global__ void k_shell_sums(const double *Q, const double *Y, Grid g, int My, i
     }
 }
 
-// tke over the uniform bins ru of Compute_SRM_Stats (pproc/pproc_mf.f:131-164)
-__global__ void k_tke(const double *U, const double *Ur, const double *ura, Grid g, int My, int Mz, size_t n3,
+// tke over the uniform bins ru of Compute_SRM_Stats (pproc/pproc_mf.f:131-164);
+// the bins' mean Ur from the sums and counts of the pass before
+__global__ void k_tke(const double *Q, const double *bsum, const unsigned long long *bcnt, Grid g, int My, int Mz, size_t n3,
                       const double *ru, int na, double *part) {
     double acc[1] = {0.0};
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n3; p += (size_t)gridDim.x * blockDim.x) {
         int i, j, k;
         cell_ijk(p, My, Mz, i, j, k);
-        double rad = g.rad(i, j, k);
+        const CellU c = cell_velocity(Q, g, n3, p, i, j, k);
+        const double rad = c.rad, ur = c.ur;
         int M = find_bin(ru, na, rad);
         if (M < 0) continue;   // unassigned in the reference: contributes 0
-        double d = Ur[p] - ura[M];
+        double d = ur - bsum[M] / (double)bcnt[M];
         double urp2 = d * d, t1 = 0.0, t2 = 0.0, t3 = 0.0;
         if (i > 0 && j > 0 && k > 0) {
             double ix = (double)(i + 1) - 1.0, iy = (double)(j + 1) - 1.0, iz = (double)(k + 1) - 1.0;
-            t1 = U[p] - Ur[p] * (ix * g.D[0] / rad);
-            t2 = U[n3 + p] - Ur[p] * (iy * g.D[1] / rad);
-            t3 = U[2 * n3 + p] - Ur[p] * (iz * g.D[2] / rad);
+            t1 = c.u1 - ur * (ix * g.D[0] / rad);
+            t2 = c.u2 - ur * (iy * g.D[1] / rad);
+            t3 = c.u3 - ur * (iz * g.D[2] / rad);
         }
         acc[0] += (t1 * t1 + t2 * t2 + t3 * t3) + urp2;
     }
@@ -180,6 +212,7 @@ __global__ void k_tke(const double *U, const double *Ur, const double *ura, Grid
 // ---- Generate_Shock_Surface -------------------------------------------------------
 __global__ void k_max(const double *b, size_t n3, double *part) {
     double m = -INFINITY;
+#pragma unroll 8
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n3; p += (size_t)gridDim.x * blockDim.x)
         m = fmax(m, b[p]);
     __shared__ double sh[kRB];
@@ -201,20 +234,31 @@ __global__ void k_shock(const double *b, double thr, Grid g, int My, int Mz, siz
     constexpr int NV = PASS == 0 ? 4 : 1;
     double acc[NV];
     for (int v = 0; v < NV; v++) acc[v] = 0.0;
-    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n3; p += (size_t)gridDim.x * blockDim.x) {
-        if (!(b[p] > thr)) continue;
-        int i, j, k;
-        cell_ijk(p, My, Mz, i, j, k);
-        if constexpr (PASS == 0) {
-            acc[0] += g.cor(0, i);
-            acc[NV > 1 ? 1 : 0] += g.cor(1, j);
-            acc[NV > 2 ? 2 : 0] += g.cor(2, k);
-            acc[NV > 3 ? 3 : 0] += 1.0;
-        } else {
-            double dx = g.cor(0, i) - cx, dy = g.cor(1, j) - cy, dz = g.cor(2, k) - cz;
-            double r = sqrt(dx * dx + dy * dy + dz * dz);
-            if constexpr (PASS == 1) acc[0] += r;
-            else { double d = r - ra; acc[0] += d * d; }
+    // few cells are shock cells: eight values are looked at per turn, so that
+    // their loads are in flight together
+    constexpr int U = 8;
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    for (size_t p0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p0 < n3; p0 += U * step) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = p0 + u * step < n3 ? b[p0 + u * step] : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!(v[u] > thr)) continue;
+            const size_t p = p0 + u * step;
+            int i, j, k;
+            cell_ijk(p, My, Mz, i, j, k);
+            if constexpr (PASS == 0) {
+                acc[0] += g.cor(0, i);
+                acc[NV > 1 ? 1 : 0] += g.cor(1, j);
+                acc[NV > 2 ? 2 : 0] += g.cor(2, k);
+                acc[NV > 3 ? 3 : 0] += 1.0;
+            } else {
+                double dx = g.cor(0, i) - cx, dy = g.cor(1, j) - cy, dz = g.cor(2, k) - cz;
+                double r = sqrt(dx * dx + dy * dy + dz * dz);
+                if constexpr (PASS == 1) acc[0] += r;
+                else { double d = r - ra; acc[0] += d * d; }
+            }
         }
     }
     block_sums<NV>(acc, part);
@@ -283,11 +327,13 @@ int dev_compute_grad(st_ctx *c, double *Grad, double *maxdil, double *enstrophy)
     c->launches++;
     k_vort<<<kRG, kRB, 0, c->stream>>>(g9, Grad, n3, part);
     ST_CUDA(c, cudaGetLastError());
-    double s[2];
-    ST_TRY(fetch_max(c, part, &s[0]));
-    ST_TRY(fetch_sums(c, part + kRG, 1, &s[1]));
-    *maxdil = s[0];
-    *enstrophy = 0.5 * s[1] / (double)(c->dm.n[0] * c->dm.n[1] * c->dm.n[2]);
+    std::vector<double> h(2 * kRG);             // maxima, then sums, of the blocks
+    ST_CUDA(c, cudaMemcpyAsync(h.data(), part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    ST_TRY(sync_stream(c));
+    double mx = -INFINITY, sum = 0.0;
+    for (int q = 0; q < kRG; q++) { mx = std::fmax(mx, h[q]); sum += h[kRG + q]; }
+    *maxdil = mx;
+    *enstrophy = 0.5 * sum / (double)(c->dm.n[0] * c->dm.n[1] * c->dm.n[2]);
     return ST_OK;
 }
 
@@ -298,43 +344,40 @@ int dev_compute_srm_stats(st_ctx *c, double *hmix, double *tke_total, double *ur
     const size_t n3 = c->dm.n3;
     const int na = shell_count(c);
     const int My = c->dm.n[1], Mz = c->dm.n[2];
-    Scratch Us(c, 3), Urs(c, 1), parts(c, 1);
-    double *U = Us, *Ur = Urs, *part = parts;
+    Scratch parts(c, 1);
+    double *part = parts;
     // bin tables, sums and counts in the parts buffer: rs[na+1], ru[na+1],
-    // bsum[2na], bcnt[na], ura[na] after the kRG partials
+    // bsum[2na], bcnt[na] after the kRG partials
     std::vector<double> rs(na + 1), ru(na + 1);
     rs[0] = 0.0; ru[0] = 0.0;
     for (int M = 2; M <= na + 1; M++) {
         rs[M - 1] = rs[M - 2] + (M <= 4 ? c->DX * 2.0 * std::sqrt(3.0) : c->DX * std::sqrt(3.0));
         ru[M - 1] = ru[M - 2] + c->DX * std::sqrt(3.0);
     }
-    double *d_rs = part + kRG, *d_ru = d_rs + na + 1, *d_sum = d_ru + na + 1, *d_ura = d_sum + 2 * na;
-    unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(d_ura + na);
+    double *d_rs = part + kRG, *d_ru = d_rs + na + 1, *d_sum = d_ru + na + 1;
+    unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(d_sum + 2 * na);
     ST_CUDA(c, cudaMemcpyAsync(d_rs, rs.data(), (na + 1) * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     ST_CUDA(c, cudaMemcpyAsync(d_ru, ru.data(), (na + 1) * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     ST_CUDA(c, cudaMemsetAsync(d_sum, 0, 2 * na * sizeof(double), c->stream));
     ST_CUDA(c, cudaMemsetAsync(d_cnt, 0, na * sizeof(unsigned long long), c->stream));
     const Grid g = grid_of(c);
     c->launches++;
-    k_shell_sums<<<kRG, kRB, 3 * na * sizeof(double), c->stream>>>(c->Q, c->Y, g, My, Mz, n3, d_rs, na, U, Ur, d_sum,
-                                                                   d_cnt);
+    k_shell_sums<<<kRG, kRB, 3 * na * sizeof(double), c->stream>>>(c->Q, c->Y, g, My, Mz, n3, d_rs, na, d_sum, d_cnt);
+    ST_CUDA(c, cudaGetLastError());
+    c->launches++;
+    k_tke<<<kRG, kRB, 0, c->stream>>>(c->Q, d_sum, d_cnt, g, My, Mz, n3, d_ru, na, part);
     ST_CUDA(c, cudaGetLastError());
     std::vector<double> hsum(2 * na);
     std::vector<unsigned long long> hcnt(na);
     ST_CUDA(c, cudaMemcpyAsync(hsum.data(), d_sum, 2 * na * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     ST_CUDA(c, cudaMemcpyAsync(hcnt.data(), d_cnt, na * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    ST_TRY(sync_stream(c));
+    double tke;
+    ST_TRY(fetch_sums(c, part, 1, &tke));       // waits for both
     std::vector<double> ura(na), ya(na);
     for (int M = 0; M < na; M++) {
         ura[M] = hsum[M] / (double)hcnt[M];
         ya[M] = hsum[na + M] / (double)hcnt[M];
     }
-    ST_CUDA(c, cudaMemcpyAsync(d_ura, ura.data(), na * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    c->launches++;
-    k_tke<<<kRG, kRB, 0, c->stream>>>(U, Ur, d_ura, g, My, Mz, n3, d_ru, na, part);
-    ST_CUDA(c, cudaGetLastError());
-    double tke;
-    ST_TRY(fetch_sums(c, part, 1, &tke));
     *tke_total = tke / (double)(c->dm.n[0] * c->dm.n[1] * c->dm.n[2]);
     double h = 0.0;
     for (int M = 0; M < na; M++)

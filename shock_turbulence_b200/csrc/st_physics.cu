@@ -4,6 +4,7 @@
 // Each routine keeps the operand order of the reference expression it
 // implements (the library is compiled with --fmad=false, so products and sums
 // round exactly as written); explicit fma() appears only in the line solvers.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include "st_internal.h"
@@ -1383,8 +1384,10 @@ __global__ void k_monitor_partial(const double *Q, const double *g, size_t n3c, 
 }
 
 int dev_monitors(st_ctx *c) {
-    const int nb = 256;
-    Scratch parts(c);   // >= 8*nb doubles for every supported grid (n3 >= 32^3)
+    // four blocks per SM (a power and a logarithm per cell: 192^3 202 us in 256
+    // blocks); never more partials than the scratch field holds
+    const int nb = (int)std::min<size_t>(592, c->dm.n3 / 8);
+    Scratch parts(c);   // 8*nb doubles
     double *part = parts;
     c->launches++;
     k_monitor_partial<<<nb, 256, 0, c->stream>>>(c->Q, c->gamma_eff, c->dm.n3, c->fs, part,
