@@ -222,8 +222,12 @@ int dev_compute_gamma(st_ctx *c, const double *Y) {
 // the FP32 mode.  Qr is the state in that type (Q itself in FP64); the
 // derivative operands come from Qr, the pointwise thermodynamics from Q.
 // gamma_from_Y: also Compute_gamma (gamma_eff of Y) in the first pass.
+// keep: T, u, v and w go to these fields, which outlive the call, for the
+// routines of the same stage that would form them again.
+template <class R> struct KeepT { R *T, *u, *v, *w; };
 template <class R>
-static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bool gamma_from_Y = false) {
+static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bool gamma_from_Y = false,
+                 const KeepT<R> *keep = nullptr) {
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
     const Phys f = phys(c);
     // src/rhsv_periodic_sf.f:1381 adds Qvisc unconditionally
@@ -237,8 +241,9 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bo
     R *GTx = G[G_DTDX], *GTy = G[G_DTDY], *GTz = G[G_DTDZ];
     ScratchT<R> sQcx(c, 5), sQcy(c, 5), sQcz(c, 5);
     R *Qcx = sQcx, *Qcy = sQcy, *Qcz = sQcz;
-    ScratchNT<R> s(c, 8);
-    R *P = s[0], *T = s[1], *u = s[2], *v = s[3], *w = s[4], *mu = s[5], *dmu = s[6], *FF = s[7];
+    ScratchNT<R> s(c, 4), own(c, keep ? 0 : 4);
+    R *P = s[0], *mu = s[1], *dmu = s[2], *FF = s[3];
+    R *T = keep ? keep->T : own[0], *u = keep ? keep->u : own[1], *v = keep ? keep->v : own[2], *w = keep ? keep->w : own[3];
     // second derivatives and derivatives of /GRAD/ (one field each: all of
     // them are formed before the one pointwise pass that uses them)
     ScratchNT<R> dd(c, 18);
@@ -630,59 +635,70 @@ static int compute_hyper_t(st_ctx *c, const double *Q, const double *Y, const R 
 // is accumulated by the derivative kernels themselves in the reference's
 // x, y, z order (iadd), so dF*/dE* are never stored; fluxes that are products
 // of stored fields are formed by the derivative kernels while loading.
+// FP64: the sums go straight to Qrhs (four fields less to store, reload and
+// add), and keep gives the velocities; the FP32 mode forms its sum apart, as
+// its rounding depends on it, and its velocities by division as the reference
+// does.
 template <class R>
-static int hyper_rhs_t(st_ctx *c, const double *Q, R *Qrhs, const double *Y, const R *Yr) {
+static int hyper_rhs_t(st_ctx *c, const double *Q, R *Qrhs, const double *Y, const R *Yr, const KeepT<R> *keep = nullptr) {
     if (c->p.hyper_param == 0) return ST_OK;
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
     ST_TRY(compute_hyper_t<R>(c, Q, Y, Yr));
     const double *Q1 = Q, *Q2 = Q + n3, *Q3 = Q + 2 * n3, *Q4 = Q + 3 * n3;
-    ScratchNT<R> s(c, 9);
-    R *U1 = s[0], *U2 = s[1], *U3 = s[2], *dila = s[3], *S1 = s[4], *S2 = s[5], *S3 = s[6];
-    R *Flux = s[7], *Flux2 = s[8];
-    ScratchT<R> Qhs(c, 5);
-    R *Qh = Qhs;   // Qh(:,:,:,4) stays zero and is never added
-    R *h1 = Qh, *h2 = Qh + n3, *h3 = Qh + 2 * n3, *h5 = Qh + 4 * n3;
+    const bool direct = is_fp64<R>(), have_u = direct && keep;
+    ScratchNT<R> s(c, 6), us(c, have_u ? 0 : 3);
+    R *U1 = have_u ? keep->u : us[0], *U2 = have_u ? keep->v : us[1], *U3 = have_u ? keep->w : us[2];
+    R *S1 = s[0], *S2 = s[1], *S3 = s[2], *Flux = s[3], *Flux2 = s[4], *Flux3 = s[5];
+    ScratchNT<R> Qhs(c, direct ? 0 : 4);
+    R *h1 = direct ? Qrhs : Qhs[0], *h2 = direct ? Qrhs + n3 : Qhs[1], *h3 = direct ? Qrhs + 2 * n3 : Qhs[2];
+    R *h5 = direct ? Qrhs + 4 * n3 : Qhs[3];
+    const int first = direct ? 1 : 0;   // the first term of a sum adds to Qrhs, or starts the sum
     R *const *Gr = Store<R>::grad(c);
     const R *G0 = Gr[0], *G1 = Gr[1], *G2 = Gr[2], *G3 = Gr[3], *G4 = Gr[4], *G5 = Gr[5], *G6 = Gr[6],
             *G7 = Gr[7], *G8 = Gr[8];
     const R *GTx = Gr[G_DTDX], *GTy = Gr[G_DTDY], *GTz = Gr[G_DTDZ];
     R *const *H = Store<R>::hyp(c);
     const R *vh = H[H_VISC], *bh = H[H_BETA], *kh = H[H_K];
-    PFOR(c, nc, io(Q1, Q2, Q3, Q4, G0, G1, G2, G3, G4, G5, G6, G7, G8, vh, bh, U1, U2, U3, dila, S1, S2, S3, Flux, Flux2), {
-        U1[p] = Q1[p] / Q4[p];
-        U2[p] = Q2[p] / Q4[p];
-        U3[p] = Q3[p] / Q4[p];
-        dila[p] = G0[p] + G4[p] + G8[p];
+    PFOR(c, nc, io(G0, G1, G2, G3, G4, G5, G6, G7, G8, vh, bh, S1, S2, S3, Flux, Flux2, Flux3) + (have_u ? 0.0 : io(Q1, Q2, Q3, Q4, U1, U2, U3)), {
+        if (!have_u) {
+            U1[p] = Q1[p] / Q4[p];
+            U2[p] = Q2[p] / Q4[p];
+            U3[p] = Q3[p] / Q4[p];
+        }
+        const R dila = G0[p] + G4[p] + G8[p];
         S1[p] = G3[p] + G1[p];
         S2[p] = G6[p] + G2[p];
         S3[p] = G7[p] + G5[p];
-        Flux[p] = 2.0 * vh[p] * G0[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila[p];
-        Flux2[p] = 2.0 * vh[p] * G4[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila[p];
+        Flux[p] = 2.0 * vh[p] * G0[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila;
+        Flux2[p] = 2.0 * vh[p] * G4[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila;
+        Flux3[p] = 2.0 * vh[p] * G8[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila;
     });
     // x momentum: Qh1 = dFx + dFy + dFz, Qh5 = dEx + dEy + dEz
     // (each line pair: a flux and its product with a velocity component, the
     // second reading what the first reads; one launch per pair)
-    const R *cF = Flux, *cF2 = Flux2;
-    ST_TRY(dfd_pair<R>(c, 0, pr_one(cF), h1, 0, 0, pr_mul(U1, cF), h5, 1, 0));
+    const R *cF = Flux, *cF2 = Flux2, *cF3 = Flux3;
+    ST_TRY(dfd_pair<R>(c, 0, pr_one(cF), h1, 0, first, pr_mul(U1, cF), h5, 1, first));
     ST_TRY(dfd_pair<R>(c, 1, pr_mul(vh, S1), h1, 1, 1, pr_mulmul(vh, S1, U1), h5, 1, 1));
     ST_TRY(dfd_pair<R>(c, 2, pr_mul(vh, S2), h1, 1, 1, pr_mulmul(vh, S2, U1), h5, 1, 1));
     // y momentum (x, y, z accumulation order)
-    ST_TRY(dfd_pair<R>(c, 0, pr_mul(vh, S1), h2, 1, 0, pr_mulmul(vh, S1, U2), h5, 1, 1));
+    ST_TRY(dfd_pair<R>(c, 0, pr_mul(vh, S1), h2, 1, first, pr_mulmul(vh, S1, U2), h5, 1, 1));
     ST_TRY(dfd_pair<R>(c, 1, pr_one(cF2), h2, 0, 1, pr_mul(U2, cF2), h5, 1, 1));
     ST_TRY(dfd_pair<R>(c, 2, pr_mul(vh, S3), h2, 1, 1, pr_mulmul(vh, S3, U2), h5, 1, 1));
     // z momentum
-    PFOR(c, nc, io(vh, G8, bh, dila, Flux), { Flux[p] = 2.0 * vh[p] * G8[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila[p]; });
-    ST_TRY(dfd_pair<R>(c, 0, pr_mul(vh, S2), h3, 1, 0, pr_mulmul(vh, S2, U3), h5, 1, 1));
+    ST_TRY(dfd_pair<R>(c, 0, pr_mul(vh, S2), h3, 1, first, pr_mulmul(vh, S2, U3), h5, 1, 1));
     ST_TRY(dfd_pair<R>(c, 1, pr_mul(vh, S3), h3, 1, 1, pr_mulmul(vh, S3, U3), h5, 1, 1));
-    ST_TRY(dfd_pair<R>(c, 2, pr_one(cF), h3, 0, 1, pr_mul(U3, cF), h5, 1, 1));
+    ST_TRY(dfd_pair<R>(c, 2, pr_one(cF3), h3, 0, 1, pr_mul(U3, cF3), h5, 1, 1));
     // artificial heat flux
     ST_TRY(dfd(c, 0, 0, pr_mul(kh, GTx), h5, 1, 1.0));
     ST_TRY(dfd(c, 1, 0, pr_mul(kh, GTy), h5, 1, 1.0));
     ST_TRY(dfd(c, 2, 0, pr_mul(kh, GTz), h5, 1, 1.0));
-    PFOR(c, nc, 4 * io(Qrhs, Qrhs, Qh), {
-        for (int l = 0; l < 5; l++)
-            if (l != 3) Qrhs[l * n3 + p] = Qrhs[l * n3 + p] + Qh[l * n3 + p];
-    });
+    if (!direct)
+        PFOR(c, nc, io(h1, h2, h3, h5) + 8 * io(Qrhs), {
+            Qrhs[p] = Qrhs[p] + h1[p];
+            Qrhs[n3 + p] = Qrhs[n3 + p] + h2[p];
+            Qrhs[2 * n3 + p] = Qrhs[2 * n3 + p] + h3[p];
+            Qrhs[4 * n3 + p] = Qrhs[4 * n3 + p] + h5[p];
+        });
     return ST_OK;
 }
 
@@ -691,22 +707,30 @@ static int hyper_rhs_t(st_ctx *c, const double *Q, R *Qrhs, const double *Y, con
 // Yrhs = Yconvx + Yconvy + Yconvz + Ydiff does.
 template <class R>
 static int species_rhs_t(st_ctx *c, const double *Q, const R *Qr, R *Qrhs, const double *Y, const R *Yr,
-                         R *Yrhs) {
+                         R *Yrhs, const R *Tkept = nullptr) {
     if (c->p.hyper_param == 0) return ST_OK;
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
     Phys f = phys(c);
     const double *Q1 = Q, *Q2 = Q + n3, *Q3 = Q + 2 * n3, *Q4 = Q + 3 * n3, *Q5 = Q + 4 * n3;
     const R *q1r = Qr, *q2r = Qr + n3, *q3r = Qr + 2 * n3, *q4r = Qr + 3 * n3;
-    ScratchNT<R> s(c, 2);
-    R *Yd = s[0], *T = s[1];
+    // FP64: Ydiff's terms go straight to Yrhs.  Tkept: RHS's T of this stage
+    // (the momentum round trip between the two changes it in the last bit in
+    // FP64, and is not made in the FP32 mode).
+    const bool direct = is_fp64<R>();
+    ScratchNT<R> Yds(c, direct ? 0 : 1), Ts(c, Tkept ? 0 : 1);
+    R *Yd = direct ? Yrhs : Yds[0];
+    const R *T = Tkept ? Tkept : Ts[0];
     R *const *dYd = Store<R>::dYd(c);
     const R *Dh = Store<R>::hyp(c)[H_D];
     const double *g = c->gamma_eff;
-    PFOR(c, nc, io(g, Y, Q1, Q2, Q3, Q4, Q5, T), {
-        double Vs, P, Tt;
-        thermo(f, g[p], Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], Vs, P, Tt);
-        T[p] = Tt;
-    });
+    if (!Tkept) {
+        R *Tw = Ts[0];
+        PFOR(c, nc, io(g, Y, Q1, Q2, Q3, Q4, Q5, Tw), {
+            double Vs, P, Tt;
+            thermo(f, g[p], Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], Vs, P, Tt);
+            Tw[p] = Tt;
+        });
+    }
     // dY/dx_i and d(rho u_i Y)/dx_i per direction, one launch each (the
     // gradient and the flux are independent; the flux keeps its x, y, z order)
     const R *qr[3] = {q1r, q2r, q3r};
@@ -722,13 +746,101 @@ static int species_rhs_t(st_ctx *c, const double *Q, const R *Qr, R *Qrhs, const
         fl.op = PR_SPEC; fl.a = q4r; fl.b = Dh; fl.c = dYd[d]; fl.k0 = f.Re1_inv; fl.k1 = f.Sc_inv;
         ProdT<R> ft = fl;
         ft.op = PR_SPECT; ft.d = T; ft.k2 = cst;
-        ST_TRY(dfd_pair<R>(c, d, fl, Yd, 1, d == 0 ? 0 : 1, ft, Qrhs + 4 * n3, 1, 1));
+        ST_TRY(dfd_pair<R>(c, d, fl, Yd, 1, direct || d > 0 ? 1 : 0, ft, Qrhs + 4 * n3, 1, 1));
     }
-    PFOR(c, nc, io(Yrhs, Yrhs, Yd), { Yrhs[p] = Yrhs[p] + Yd[p]; });
+    if (!direct) PFOR(c, nc, io(Yrhs, Yrhs, Yd), { Yrhs[p] = Yrhs[p] + Yd[p]; });
     return ST_OK;
 }
 
-// bc_RHS src/bc_mf.f:11-463 (active face blocks)
+// ---- bc_RHS src/bc_mf.f:11-463 (active face blocks) ----------------------------
+// The characteristic conditions at one cell of an outflow face (normal
+// direction `face`): overwrites its right-hand sides.
+struct BcArgs {
+    const double *Q, *g;
+    size_t n3;
+};
+template <class R>
+__device__ __forceinline__ void bc_cell(const BcArgs &b, int face, size_t q, double Pq, double dPn, double dun, R *Qrhs, R *Yrhs) {
+    const size_t n3 = b.n3;
+    const double q1 = b.Q[q], q2 = b.Q[n3 + q], q3 = b.Q[2 * n3 + q], q4 = b.Q[3 * n3 + q], g = b.g[q];
+    double Vs = 1.0 / q4;
+    double U[3] = {q1 * Vs, q2 * Vs, q3 * Vs};
+    double Ur = sqrt(U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
+    double tmp2 = sqrt(g * Vs * Pq);
+    double un = U[face];
+    double L1 = 0.0, L2 = 0.0, L3 = 0.0, L4 = 0.0, L6 = 0.0;
+    double L5 = (un + tmp2) * (dPn + tmp2 * q4 * dun);
+    double d1 = (1.0 / (tmp2 * tmp2)) * (L2 + 5.0e-1 * (L1 + L5));
+    double d2 = 5.0e-1 * (L5 + L1);
+    double d3 = (5.0e-1 / (q4 * tmp2)) * (L5 - L1);
+    double d4 = L3, d5 = L4, d6 = L6;
+    double Qm[3] = {q1, q2, q3};
+    // normal momentum component gets d3; the two tangential get d4, d5
+    int t1 = face == 0 ? 1 : 0, t2 = face == 2 ? 1 : 2;
+    Qrhs[3 * n3 + q] = -d1;
+    Qrhs[4 * n3 + q] = -5.0e-1 * Ur * Ur * d1 - d2 / (g - 1.0) - Qm[face] * d3 - Qm[t1] * d4 - Qm[t2] * d5;
+    Qrhs[face * n3 + q] = -U[face] * d1 - q4 * d3;
+    Qrhs[t1 * n3 + q] = -U[t1] * d1 - q4 * d4;
+    Qrhs[t2 * n3 + q] = -U[t2] * d1 - q4 * d5;
+    Yrhs[q] = -q4 * d6;
+}
+
+// One outflow face in FP64.  Of the pressure's normal derivative only the last
+// row of each line is wanted, which the elimination gives without the back
+// substitution, and which the rows more than 48 before it do not reach (0.38
+// per row: 2e-20).  A block takes 32 lines: its threads form the pressure of
+// their last rows, one warp runs the elimination and the conditions.  Against
+// the pressure as a field and three whole derivatives (120 bytes per cell): see
+// bc_rhs_t.
+constexpr int kFaceRows = 48;
+struct FaceArgs {
+    BcArgs b;
+    const double *Gn, *l, *id;
+    double *Qrhs, *Yrhs;
+    double fac, a1, b1, closure1, closure2;
+    int n, nf, My, Mz, Mx;
+    size_t n3c;
+};
+template <int FACE>
+__global__ void __launch_bounds__(256) k_bc_face(FaceArgs a) {
+    __shared__ double P[kFaceRows + 2][33];
+    pdl_wait();
+    const size_t n3 = a.b.n3, c0 = (size_t)blockIdx.y * a.n3c;
+    const int n = a.n, i0 = max(0, n - kFaceRows), r0 = max(0, i0 - 2), rows = n - r0, pl0 = blockIdx.x * 32;
+    auto cell = [&](int pl, int r) -> size_t {
+        if (FACE == 0) return c0 + pl + (size_t)a.My * a.Mz * r;                                     // pl = j + My*k
+        if (FACE == 1) return c0 + r + (size_t)a.My * pl;                                            // pl = k + Mz*i
+        return c0 + (pl % a.My) + (size_t)a.My * r + (size_t)a.My * a.Mz * (pl / a.My);              // pl = j + My*i
+    };
+    for (int q = threadIdx.x; q < rows * 32; q += 256) {
+        const int line = FACE == 1 ? q / rows : q % 32, r = FACE == 1 ? q % rows : q / 32;
+        if (pl0 + line >= a.nf) continue;
+        const size_t p = cell(pl0 + line, r0 + r);
+        const double q1 = a.b.Q[p], q2 = a.b.Q[n3 + p], q3 = a.b.Q[2 * n3 + p], q4 = a.b.Q[3 * n3 + p], q5 = a.b.Q[4 * n3 + p];
+        const double Vs = 1.0 / q4;
+        P[r][line] = (a.b.g[p] - 1.0) * (q5 - 5.0e-1 * Vs * (q1 * q1 + q2 * q2 + q3 * q3));
+    }
+    __syncthreads();
+    const int line = threadIdx.x, pl = pl0 + line;
+    if (line < 32 && pl < a.nf) {
+        auto f = [&](int i) { return P[i - r0][line]; };
+        double r = 0.0;
+#pragma unroll 4
+        for (int i = i0; i < n; i++) {
+            double w;
+            if (i == n - 1) w = a.fac * (2.5 * f(i) - 2.0 * f(i - 1) - 5.0e-1 * f(i - 2));
+            else if (i == n - 2) w = a.fac * (a.closure1 * f(i + 1) + 5.0e-1 * f(i) - f(i - 1) - a.closure2 * f(i - 2));
+            else if (i == 0) w = 0.0;
+            else if (i == 1) w = a.fac * (a.b1 * (f(3) - f(1)) + a.a1 * (f(2) - f(0)));
+            else w = a.fac * (a.b1 * (f(i + 2) - f(i - 2)) + a.a1 * (f(i + 1) - f(i - 1)));
+            r = fma(-__ldg(a.l + i), r, w);
+        }
+        const size_t q = cell(pl, n - 1);
+        bc_cell<double>(a.b, FACE, q, f(n - 1), r * __ldg(a.id + n - 1), a.Gn[q], a.Qrhs, a.Yrhs);
+    }
+    pdl_next();
+}
+
 template <class R>
 static int bc_rhs_t(st_ctx *c, double *Q, R *Qrhs, const double *Y, R *Yrhs) {
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
@@ -755,106 +867,121 @@ static int bc_rhs_t(st_ctx *c, double *Q, R *Qrhs, const double *Y, R *Yrhs) {
             Q2[k * n3c + (size_t)My * (p - k * MzMx)] = 0.0;
         });
     }
-    ScratchNT<R> s(c, 4);
-    R *P = s[0], *dPx = s[1], *dPy = s[2], *dPz = s[3];
-    PFOR(c, nc, io(g, Y, Q1, Q2, Q3, Q4, Q5, P), {
-        double Vs, Pp, T;
-        thermo(f, g[p], Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], Vs, Pp, T);
-        P[p] = Pp;
-    });
-    ST_TRY(dfd(c, 0, 0, P, dPx, 0, 1.0));
-    ST_TRY(dfd(c, 1, 0, P, dPy, 0, 1.0));
-    ST_TRY(dfd(c, 2, 0, P, dPz, 0, 1.0));
-    R *const *Gr = Store<R>::grad(c);
-    const R *Gxx = Gr[G_DUX_DX], *Gyy = Gr[G_DUY_DY], *Gzz = Gr[G_DUZ_DZ];
+    R *const *Gn = Store<R>::grad(c);
     // faces in the reference order x, y, z (later faces overwrite edges)
-    for (int face = 0; face < 3; face++) {
-        size_t nf = face == 0 ? (size_t)My * Mz : face == 1 ? (size_t)Mx * Mz : (size_t)Mx * My;
-        PFOR(c, na * nf, io(Q1, Q2, Q3, Q4, P, g, dPx, Gxx, Yrhs) + 5 * io(Qrhs), {
-            const size_t k = p / nf, pl = p - k * nf;
-            size_t q;
-            if (face == 0) q = pl + (size_t)My * Mz * (Mx - 1);                    // pl = j + My*k
-            else if (face == 1) q = (My - 1) + (size_t)My * pl;                    // pl = k + Mz*i
-            else q = (pl % My) + (size_t)My * (Mz - 1) + (size_t)My * Mz * (pl / My);  // pl = j + My*i
-            q += k * n3c;
-            double Vs = 1.0 / Q4[q];
-            double Pq = P[q];
-            double U[3] = {Q1[q] * Vs, Q2[q] * Vs, Q3[q] * Vs};
-            double Ur = sqrt(U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
-            double tmp2 = sqrt(g[q] * Vs * Pq);
-            double dPn = face == 0 ? dPx[q] : face == 1 ? dPy[q] : dPz[q];
-            double dun = face == 0 ? Gxx[q] : face == 1 ? Gyy[q] : Gzz[q];
-            double un = U[face];
-            double L1 = 0.0, L2 = 0.0, L3 = 0.0, L4 = 0.0, L6 = 0.0;
-            double L5 = (un + tmp2) * (dPn + tmp2 * Q4[q] * dun);
-            double d1 = (1.0 / (tmp2 * tmp2)) * (L2 + 5.0e-1 * (L1 + L5));
-            double d2 = 5.0e-1 * (L5 + L1);
-            double d3 = (5.0e-1 / (Q4[q] * tmp2)) * (L5 - L1);
-            double d4 = L3, d5 = L4, d6 = L6;
-            double Qm[3] = {Q1[q], Q2[q], Q3[q]};
-            // normal momentum component gets d3; the two tangential get d4, d5
-            int t1 = face == 0 ? 1 : 0, t2 = face == 2 ? 1 : 2;
-            Qrhs[3 * n3 + q] = -d1;
-            Qrhs[4 * n3 + q] = -5.0e-1 * Ur * Ur * d1 - d2 / (g[q] - 1.0) - Qm[face] * d3 - Qm[t1] * d4 -
-                               Qm[t2] * d5;
-            Qrhs[face * n3 + q] = -U[face] * d1 - Q4[q] * d3;
-            Qrhs[t1 * n3 + q] = -U[t1] * d1 - Q4[q] * d4;
-            Qrhs[t2 * n3 + q] = -U[t2] * d1 - Q4[q] * d5;
-            Yrhs[q] = -Q4[q] * d6;
+    if constexpr (is_fp64<R>()) {
+        for (int face = 0; face < 3; face++) {
+            FaceArgs a{};
+            a.b = BcArgs{Q, g, n3};
+            a.Gn = Gn[face == 0 ? G_DUX_DX : face == 1 ? G_DUY_DY : G_DUZ_DZ];
+            a.l = c->tri[face][K_D1S].l; a.id = c->tri[face][K_D1S].id;
+            a.Qrhs = Qrhs; a.Yrhs = Yrhs;
+            a.n = c->dm.n[face];
+            a.fac = 1.0 * c->s1[face] * (double)(a.n - 1);
+            a.a1 = c->k.a1; a.b1 = c->k.b1; a.closure1 = c->k.closure1; a.closure2 = c->k.closure2;
+            a.nf = face == 0 ? My * Mz : face == 1 ? Mx * Mz : Mx * My;
+            a.My = My; a.Mz = Mz; a.Mx = Mx;
+            a.n3c = n3c;
+            const int rows = std::min(a.n, kFaceRows + 2);
+            const int pi = prof_start(c, "k_bc_face", (double)na * a.nf * (rows * 6 + 12) * 8.0);
+            const dim3 grid((a.nf + 31) / 32, (unsigned)na);
+            const cudaError_t e = face == 0   ? launch_pdl(k_bc_face<0>, grid, dim3(256), 0, c->stream, a)
+                                  : face == 1 ? launch_pdl(k_bc_face<1>, grid, dim3(256), 0, c->stream, a)
+                                              : launch_pdl(k_bc_face<2>, grid, dim3(256), 0, c->stream, a);
+            prof_stop(c, pi);
+            ST_CUDA(c, e);
+        }
+    } else {
+        ScratchNT<R> s(c, 4);
+        R *P = s[0], *dPx = s[1], *dPy = s[2], *dPz = s[3];
+        PFOR(c, nc, io(g, Y, Q1, Q2, Q3, Q4, Q5, P), {
+            double Vs, Pp, T;
+            thermo(f, g[p], Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], Vs, Pp, T);
+            P[p] = Pp;
         });
+        ST_TRY(dfd(c, 0, 0, P, dPx, 0, 1.0));
+        ST_TRY(dfd(c, 1, 0, P, dPy, 0, 1.0));
+        ST_TRY(dfd(c, 2, 0, P, dPz, 0, 1.0));
+        const R *Gxx = Gn[G_DUX_DX], *Gyy = Gn[G_DUY_DY], *Gzz = Gn[G_DUZ_DZ];
+        const BcArgs ba{Q, g, n3};
+        for (int face = 0; face < 3; face++) {
+            size_t nf = face == 0 ? (size_t)My * Mz : face == 1 ? (size_t)Mx * Mz : (size_t)Mx * My;
+            PFOR(c, na * nf, io(Q1, Q2, Q3, Q4, P, g, dPx, Gxx, Yrhs) + 5 * io(Qrhs), {
+                const size_t k = p / nf, pl = p - k * nf;
+                size_t q;
+                if (face == 0) q = pl + (size_t)My * Mz * (Mx - 1);                    // pl = j + My*k
+                else if (face == 1) q = (My - 1) + (size_t)My * pl;                    // pl = k + Mz*i
+                else q = (pl % My) + (size_t)My * (Mz - 1) + (size_t)My * Mz * (pl / My);  // pl = j + My*i
+                q += k * n3c;
+                const double dPn = face == 0 ? dPx[q] : face == 1 ? dPy[q] : dPz[q];
+                const double dun = face == 0 ? Gxx[q] : face == 1 ? Gyy[q] : Gzz[q];
+                bc_cell<R>(ba, face, q, P[q], dPn, dun, Qrhs, Yrhs);
+            });
+        }
     }
     return ST_OK;
 }
 
-// Sponge_Forcing src/sponge_mf.f:7-127
+// Sponge_Forcing src/sponge_mf.f:7-127: the forcing's strength at a cell and
+// its reference state
+struct Sponge {
+    double ref[5], Y_ref;
+    int st[3], len[3], My, Mz;
+    size_t n3c;
+    bool one, idx32;
+    double shell;      // fraction of the cells in the sponge shell (the only ones touched)
+    __device__ __forceinline__ static double sig(int gI, int st, int ln) {
+        if (gI >= st) {
+            const double r = (float)(gI - st) / (float)ln;   // REAL/REAL, src/sponge_mf.f:87-89
+            return 4.0 * (r * r * r);                        // r r is exact: r is a float
+        }
+        return 0.0;
+    }
+    __device__ __forceinline__ double at(size_t p) const {
+        int j, k, i;
+        if (idx32) {                                        // 32-bit index arithmetic when it suffices
+            unsigned q = (unsigned)p;
+            if (!one) q -= (q / (unsigned)n3c) * (unsigned)n3c;   // position within the case
+            const unsigned r = q / (unsigned)My;
+            j = (int)(q - r * (unsigned)My); k = (int)(r % (unsigned)Mz); i = (int)(r / (unsigned)Mz);
+        } else {
+            const size_t q = one ? p : p - (p / n3c) * n3c;
+            const size_t r = q / My;
+            j = (int)(q - r * My); k = (int)(r % Mz); i = (int)(r / Mz);
+        }
+        return sig(i + 1, st[0], len[0]) + sig(j + 1, st[1], len[1]) + sig(k + 1, st[2], len[2]);
+    }
+};
+static Sponge sponge_of(const st_ctx *c) {
+    Sponge s{};
+    const double g1 = c->p.gamma1, base_pressure = 0.71429, Ms = 1.8;
+    const double P_ref = ((2.0 * g1 / (g1 + 1.0)) * (Ms * Ms - 1.0) + 1.0) * base_pressure;
+    s.ref[3] = (g1 + 1.0) * Ms * Ms / ((g1 - 1.0) * Ms * Ms + 2.0);
+    s.ref[4] = P_ref / (g1 - 1.0);
+    s.Y_ref = 1.0;
+    for (int d = 0; d < 3; d++) {
+        s.st[d] = c->dm.n[d] - (int)ceil(0.1 * c->dm.n[d]);
+        s.len[d] = c->dm.n[d] - s.st[d];
+    }
+    s.My = c->dm.n[1]; s.Mz = c->dm.n[2];
+    s.n3c = c->dm.n3;
+    s.one = c->na == 1;
+    s.idx32 = c->ncell() <= 0xffffffffull;
+    s.shell = (double)(s.n3c - (size_t)s.st[0] * s.st[1] * s.st[2]) / (double)s.n3c;
+    return s;
+}
 template <class R>
 static int sponge_t(st_ctx *c, const double *Q, R *Qrhs, const double *Y, R *Yrhs) {
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
-    const int Mx = c->dm.n[0], My = c->dm.n[1], Mz = c->dm.n[2];
-    const double g1 = c->p.gamma1;
-    const double base_pressure = 0.71429, Ms = 1.8;
-    const double rho_ref = (g1 + 1.0) * Ms * Ms / ((g1 - 1.0) * Ms * Ms + 2.0);
-    const double P_ref = ((2.0 * g1 / (g1 + 1.0)) * (Ms * Ms - 1.0) + 1.0) * base_pressure;
-    const double E_ref = P_ref / (g1 - 1.0), Y_ref = 1.0;
-    int start[3], len[3];
-    const int Ns[3] = {Mx, My, Mz};
-    for (int d = 0; d < 3; d++) {
-        start[d] = Ns[d] - (int)ceil(0.1 * Ns[d]);
-        len[d] = Ns[d] - start[d];
-    }
-    const int sx = start[0], sy = start[1], sz = start[2], lx = len[0], ly = len[1], lz = len[2];
-    const size_t n3c = c->dm.n3;
-    const bool idx32 = nc <= 0xffffffffull;   // 32-bit index arithmetic when it suffices
-    const bool one = c->na == 1;
-    // fraction of the cells in the sponge shell (the only ones touched)
-    const double shell = (double)(n3c - (size_t)sx * sy * sz) / (double)n3c;
-    PFOR(c, nc, shell * (10 * io(Qrhs) + 5 * io(Q) + io(Y) + 2 * io(Yrhs)), {
-        int j, k, i;
-        if (idx32) {
-            unsigned q = (unsigned)p;
-            if (!one) q -= (q / (unsigned)n3c) * (unsigned)n3c;   // position within the case
-            unsigned r = q / (unsigned)My;
-            j = (int)(q - r * (unsigned)My); k = (int)(r % (unsigned)Mz); i = (int)(r / (unsigned)Mz);
-        } else {
-            size_t q = one ? p : p - (p / n3c) * n3c;
-            size_t r = q / My;
-            j = (int)(q - r * My); k = (int)(r % Mz); i = (int)(r / Mz);
-        }
-        auto sig = [](int gI, int st, int ln) -> double {
-            if (gI >= st) {
-                float r = (float)(gI - st) / (float)ln;   // REAL/REAL, src/sponge_mf.f:87-89
-                return 4.0 * pow((double)r, 3.0);
-            }
-            return 0.0;
-        };
-        double s = sig(i + 1, sx, lx) + sig(j + 1, sy, ly) + sig(k + 1, sz, lz);
+    const Sponge sp = sponge_of(c);
+    PFOR(c, nc, sp.shell * (10 * io(Qrhs) + 5 * io(Q) + io(Y) + 2 * io(Yrhs)), {
+        const double s = sp.at(p);
         // outside the sponge shell the forcing is 0*(...): the right-hand
         // sides keep their values (up to the sign of a zero), so those cells
         // are not touched
         if (s == 0.0) return;
-        double Qref[5] = {0.0, 0.0, 0.0, rho_ref, E_ref};
-        for (int l = 0; l < 5; l++) Qrhs[l * n3 + p] = Qrhs[l * n3 + p] - s * (Q[l * n3 + p] - Qref[l]);
-        Yrhs[p] = Yrhs[p] - s * (Q[3 * n3 + p] * Y[p] - Q[3 * n3 + p] * Y_ref);
+        for (int l = 0; l < 5; l++) Qrhs[l * n3 + p] = Qrhs[l * n3 + p] - s * (Q[l * n3 + p] - sp.ref[l]);
+        Yrhs[p] = Yrhs[p] - s * (Q[3 * n3 + p] * Y[p] - Q[3 * n3 + p] * sp.Y_ref);
     });
     return ST_OK;
 }
@@ -1221,6 +1348,8 @@ static int lddrk4_sf(st_ctx *c) {
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
     Scratch Qfs(c, 5);
     double *Qf = Qfs;
+    ScratchNT<R> kept(c, 4);
+    const KeepT<R> keep{kept[0], kept[1], kept[2], kept[3]};
     StateCopy<R> sc(c);
     bool fresh = false;   // the float state copy holds the current state
     const double *dtp = c->dscal + SC_DT;     // time step and time of case k at k*kScal
@@ -1238,8 +1367,8 @@ static int lddrk4_sf(st_ctx *c) {
             double *Q = c->Q, *QW = c->QW;
             R *dQ = Store<R>::dQ(c);
             if (!fresh) ST_TRY(refresh<R>(c, sc, Q, c->Y, false));
-            ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, c->Y));
-            ST_TRY(hyper_rhs_t<R>(c, Q, dQ, c->Y, sc.y(c->Y)));
+            ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, c->Y, false, &keep));
+            ST_TRY(hyper_rhs_t<R>(c, Q, dQ, c->Y, sc.y(c->Y), &keep));
             PFOR(c, nc, 5 * io(dQ, Q, Q, QW) + (first ? 0.0 : 5 * io(QW)), {
                 double dt = dtp[(one ? 0 : p / n3c) * kScal];
                 for (int l = 0; l < 5; l++) {
@@ -1275,6 +1404,8 @@ static int lddrk4_mf(st_ctx *c) {
     const size_t n3 = c->fs, nc = c->ncell();   // field stride; cells processed
     Scratch rYs(c), Qfs(c, 5);
     double *rY = rYs, *Qf = Qfs;
+    ScratchNT<R> kept(c, 4);
+    const KeepT<R> keep{kept[0], kept[1], kept[2], kept[3]};
     StateCopy<R> sc(c);
     bool fresh = false;   // the float state copy holds the current state
     const double *dtp = c->dscal + SC_DT;     // time step and time of case k at k*kScal
@@ -1289,21 +1420,40 @@ static int lddrk4_mf(st_ctx *c) {
             double *Q = c->Q, *QW = c->QW, *Y = c->Y, *rYW = c->rYW;
             R *dQ = Store<R>::dQ(c), *drYi = Store<R>::drYi(c);
             if (!fresh) ST_TRY(refresh<R>(c, sc, Q, Y, true));
-            ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, Y, true));   // Compute_gamma and RHS
-            ST_TRY(hyper_rhs_t<R>(c, Q, dQ, Y, sc.y(Y)));
-            ST_TRY(species_rhs_t<R>(c, Q, sc.q(Q), dQ, Y, sc.y(Y), drYi));
+            ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, Y, true, &keep));   // Compute_gamma and RHS
+            ST_TRY(hyper_rhs_t<R>(c, Q, dQ, Y, sc.y(Y), &keep));
+            ST_TRY(species_rhs_t<R>(c, Q, sc.q(Q), dQ, Y, sc.y(Y), drYi, keep.T));
             ST_TRY(bc_rhs_t<R>(c, Q, dQ, Y, drYi));
-            ST_TRY(sponge_t<R>(c, Q, dQ, Y, drYi));
-            PFOR(c, nc, 5 * io(dQ, Q, Q, QW) + (first ? 0.0 : 5 * io(QW)) + io(Y, drYi, rYW, rY) + (first ? 0.0 : io(rYW)), {
-                double dt = dtp[(one ? 0 : p / n3c) * kScal];
-                double ry = Q[3 * n3 + p] * Y[p];
+            // Sponge_Forcing and the update in one pass; the forced right-hand
+            // sides of the shell's cells are stored as the routine leaves them
+            const Sponge sp = sponge_of(c);
+            PFOR(c, nc, 5 * io(dQ, Q, Q, QW) + (first ? 0.0 : 5 * io(QW)) + io(Y, drYi, rYW, rY) + (first ? 0.0 : io(rYW)) + sp.shell * (5 * io(dQ) + io(drYi)), {
+                // every load before the first store (which might alias them)
+                double qo[5], w[5], d[5];
                 for (int l = 0; l < 5; l++) {
-                    size_t q = l * n3 + p;
-                    double qw = first ? dt * dQ[q] : al * QW[q] + dt * dQ[q];
-                    QW[q] = qw;
-                    Q[q] = Q[q] + be * qw;
+                    qo[l] = Q[l * n3 + p];
+                    d[l] = dQ[l * n3 + p];
+                    w[l] = first ? 0.0 : QW[l * n3 + p];
                 }
-                double rw = first ? dt * drYi[p] : al * rYW[p] + dt * drYi[p];
+                const double y = Y[p], yw = first ? 0.0 : rYW[p];
+                double dy = drYi[p];
+                const double dt = dtp[(one ? 0 : p / n3c) * kScal];
+                const double ry = qo[3] * y;
+                const double s = sp.at(p);
+                if (s != 0.0) {
+                    dy = (R)(dy - s * (qo[3] * y - qo[3] * sp.Y_ref));
+                    drYi[p] = dy;
+                    for (int l = 0; l < 5; l++) {
+                        d[l] = (R)(d[l] - s * (qo[l] - sp.ref[l]));
+                        dQ[l * n3 + p] = d[l];
+                    }
+                }
+                for (int l = 0; l < 5; l++) {
+                    const double qw = first ? dt * d[l] : al * w[l] + dt * d[l];
+                    QW[l * n3 + p] = qw;
+                    Q[l * n3 + p] = qo[l] + be * qw;
+                }
+                const double rw = first ? dt * dy : al * yw + dt * dy;
                 rYW[p] = rw;
                 rY[p] = ry + be * rw;
             });
