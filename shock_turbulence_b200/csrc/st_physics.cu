@@ -253,16 +253,23 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bo
     // P, T, u, and (the same expressions the reference evaluates later from
     // the same inputs) v, w, mu, dmu/dT
     PFOR(c, nc, io(g, Y, Q1, Q2, Q3, Q4, Q5, P, T, u, v, w, mu, dmu), {
+        // (as in every pass: all loads before the first store, which the
+        // compiler could not move them across)
+        const double y = Y[p];
+        const double q1 = Q1[p];
+        const double q2 = Q2[p];
+        const double q3 = Q3[p];
+        const double q4 = Q4[p];
+        const double q5 = Q5[p];
+        const double ge = gamma_from_Y ? gamma_of(f, y) : g[p];
         double vs, pp, tt, m, dm;
-        double ge;
-        if (gamma_from_Y) { ge = gamma_of(f, Y[p]); g[p] = ge; }
-        else ge = g[p];
-        thermo(f, ge, Y[p], Q1[p], Q2[p], Q3[p], Q4[p], Q5[p], vs, pp, tt);
+        thermo(f, ge, y, q1, q2, q3, q4, q5, vs, pp, tt);
+        viscosity(f, (R)tt, y, m, dm);
+        if (gamma_from_Y) g[p] = ge;
         P[p] = pp; T[p] = tt;
-        u[p] = Q1[p] * vs;
-        v[p] = Q2[p] * vs;
-        w[p] = Q3[p] * vs;
-        viscosity(f, (R)tt, Y[p], m, dm);
+        u[p] = q1 * vs;
+        v[p] = q2 * vs;
+        w[p] = q3 * vs;
         mu[p] = m;
         dmu[p] = dm;
     });
@@ -573,28 +580,30 @@ static int compute_hyper_t(st_ctx *c, const double *Q, const double *Y, const R 
     {
         PFOR(c, nc, io(G0, G1, G2, G3, G4, G5, G6, G7, G8, g, Y, Q1, Q2, Q3, Q4, Q5, Cbeta, Vs, P, T, e, S), {
             // G0..G8 = dux_dx, duy_dx, duz_dx, dux_dy, duy_dy, duz_dy, dux_dz, duy_dz, duz_dz
-            double w1 = G5[p] - G7[p];
-            double w2 = G6[p] - G2[p];
-            double w3 = G1[p] - G3[p];
-            double dil = G0[p] + G4[p] + G8[p];
+            const R a0 = G0[p], a1 = G1[p], a2 = G2[p], a3 = G3[p], a4 = G4[p], a5 = G5[p], a6 = G6[p], a7 = G7[p], a8 = G8[p];
+            const double ge = g[p], y = Y[p], q1 = Q1[p], q2 = Q2[p], q3 = Q3[p], q4 = Q4[p], q5 = Q5[p];
+            double w1 = a5 - a7;
+            double w2 = a6 - a2;
+            double w3 = a1 - a3;
+            double dil = a0 + a4 + a8;
             double eps = 1.0e-7, fac2 = 0.2;
             double fac = 5.0e-1 * (1.0 - tanh(2.5 + fac2 * dil));
             double om2 = w1 * w1 + w2 * w2 + w3 * w3;
-            Cbeta[p] = (fac * dil * dil / (dil * dil + om2 + eps)) * scale;
-            double s1 = G0[p], s5 = G4[p], s9 = G8[p];
-            double s2 = 5.0e-1 * (G3[p] + G1[p]);
-            double s3 = 5.0e-1 * (G6[p] + G2[p]);
-            double s6 = 5.0e-1 * (G7[p] + G5[p]);
+            double s1 = a0, s5 = a4, s9 = a8;
+            double s2 = 5.0e-1 * (a3 + a1);
+            double s3 = 5.0e-1 * (a6 + a2);
+            double s6 = 5.0e-1 * (a7 + a5);
             double s4 = s2, s7 = s3, s8 = s6;
-            double fac1 = g[p] - 1.0;
+            double fac1 = ge - 1.0;
             double fac3 = f.g1 / (f.g1 - 1.0);
-            fac3 = fac3 * 1.0 / (Y[p] + f.eps * (1.0 - Y[p]));
-            double vs = 1.0 / Q4[p];
-            double pp = fac1 * (Q5[p] - 5.0e-1 * vs * (Q1[p] * Q1[p] + Q2[p] * Q2[p] + Q3[p] * Q3[p]));
+            fac3 = fac3 * 1.0 / (y + f.eps * (1.0 - y));
+            double vs = 1.0 / q4;
+            double pp = fac1 * (q5 - 5.0e-1 * vs * (q1 * q1 + q2 * q2 + q3 * q3));
+            Cbeta[p] = (fac * dil * dil / (dil * dil + om2 + eps)) * scale;
             Vs[p] = vs;
             P[p] = pp;
             T[p] = fac3 * vs * pp;
-            e[p] = vs * (Q5[p] - 5.0e-1 * vs * (Q1[p] * Q1[p] + Q2[p] * Q2[p] + Q3[p] * Q3[p]));
+            e[p] = vs * (q5 - 5.0e-1 * vs * (q1 * q1 + q2 * q2 + q3 * q3));
             S[p] = sqrt(5.0e-1 * (s1 * s1 + s5 * s5 + s9 * s9 + 2.0 * (s2 * s4 + s3 * s7 + s6 * s8)));
         });
         ST_TRY(laplacian(c, S, d2));
@@ -606,15 +615,17 @@ static int compute_hyper_t(st_ctx *c, const double *Q, const double *Y, const R 
         const double C_mu = 2.0e-3, C_k = 1.0e-2;
         PFOR(c, nc, io(d4S, d4e, d4Y, g, P, Vs, Q4, T, Cbeta, Y) + 5 * io(eta), {
             double a4S = fabs(d4S[p]), a4e = fabs(d4e[p]), a4Y = fabs(d4Y[p]);
-            double cs = sqrt(g[p] * P[p] * Vs[p]);
-            double fac3 = (Q4[p] / T[p]) * sqrt(g[p] * P[p] * Vs[p]);
-            eta[p] = C_mu * Q4[p] * a4S;
-            eta[2 * n3 + p] = Cbeta[p] * Q4[p] * a4S;
+            const R pr = P[p], vs = Vs[p], cb = Cbeta[p], tt = T[p];
+            const double ge = g[p], q4 = Q4[p], y = Y[p];
+            double cs = sqrt(ge * pr * vs);
+            double fac3 = (q4 / tt) * sqrt(ge * pr * vs);
+            double tmp1 = (y < 1.0) ? 0.0 : 1.0;
+            double tmp2 = (y < 0.0) ? 0.0 : 1.0;
+            eta[p] = C_mu * q4 * a4S;
+            eta[2 * n3 + p] = cb * q4 * a4S;
             eta[n3 + p] = C_k * fac3 * a4e;
             eta[4 * n3 + p] = cs * a4Y;
-            double tmp1 = (Y[p] < 1.0) ? 0.0 : 1.0;
-            double tmp2 = (Y[p] < 0.0) ? 0.0 : 1.0;
-            eta[3 * n3 + p] = cs * ((Y[p] - 1.0) * tmp1 - Y[p] * (1.0 - tmp2));
+            eta[3 * n3 + p] = cs * ((y - 1.0) * tmp1 - y * (1.0 - tmp2));
         });
         ST_TRY(gaussian_filter_t<R>(c, eta, etag, 5));
         const double DX6 = pow(c->DX, 6.0), DX5 = pow(c->DX, 5.0), DX = c->DX;
@@ -622,10 +633,11 @@ static int compute_hyper_t(st_ctx *c, const double *Q, const double *Y, const R 
         R **H = Store<R>::hyp(c);
         R *hb = H[H_BETA], *hv = H[H_VISC], *hk = H[H_K], *hd = H[H_D];
         PFOR(c, nc, 5 * io(etag) + io(hb, hv, hk, hd), {
-            hb[p] = etag[2 * n3 + p] * DX6;
-            hv[p] = etag[p] * DX6;
-            hk[p] = etag[n3 + p] * DX5;
-            hd[p] = C_D * etag[4 * n3 + p] * DX5 + C_Y * etag[3 * n3 + p] * DX;
+            const R e0 = etag[p], e1 = etag[n3 + p], e2 = etag[2 * n3 + p], e3 = etag[3 * n3 + p], e4 = etag[4 * n3 + p];
+            hb[p] = e2 * DX6;
+            hv[p] = e0 * DX6;
+            hk[p] = e1 * DX5;
+            hd[p] = C_D * e4 * DX5 + C_Y * e3 * DX;
         });
     }
     return ST_OK;
@@ -660,18 +672,22 @@ static int hyper_rhs_t(st_ctx *c, const double *Q, R *Qrhs, const double *Y, con
     R *const *H = Store<R>::hyp(c);
     const R *vh = H[H_VISC], *bh = H[H_BETA], *kh = H[H_K];
     PFOR(c, nc, io(G0, G1, G2, G3, G4, G5, G6, G7, G8, vh, bh, S1, S2, S3, Flux, Flux2, Flux3) + (have_u ? 0.0 : io(Q1, Q2, Q3, Q4, U1, U2, U3)), {
+        const R a0 = G0[p], a1 = G1[p], a2 = G2[p], a3 = G3[p], a4 = G4[p], a5 = G5[p], a6 = G6[p], a7 = G7[p], a8 = G8[p];
+        const R nu = vh[p], be = bh[p];
+        double q1 = 0.0, q2 = 0.0, q3 = 0.0, q4 = 1.0;
+        if (!have_u) { q1 = Q1[p]; q2 = Q2[p]; q3 = Q3[p]; q4 = Q4[p]; }
+        const R dila = a0 + a4 + a8;
         if (!have_u) {
-            U1[p] = Q1[p] / Q4[p];
-            U2[p] = Q2[p] / Q4[p];
-            U3[p] = Q3[p] / Q4[p];
+            U1[p] = q1 / q4;
+            U2[p] = q2 / q4;
+            U3[p] = q3 / q4;
         }
-        const R dila = G0[p] + G4[p] + G8[p];
-        S1[p] = G3[p] + G1[p];
-        S2[p] = G6[p] + G2[p];
-        S3[p] = G7[p] + G5[p];
-        Flux[p] = 2.0 * vh[p] * G0[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila;
-        Flux2[p] = 2.0 * vh[p] * G4[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila;
-        Flux3[p] = 2.0 * vh[p] * G8[p] + (bh[p] - (2.0 / 3.0) * vh[p]) * dila;
+        S1[p] = a3 + a1;
+        S2[p] = a6 + a2;
+        S3[p] = a7 + a5;
+        Flux[p] = 2.0 * nu * a0 + (be - (2.0 / 3.0) * nu) * dila;
+        Flux2[p] = 2.0 * nu * a4 + (be - (2.0 / 3.0) * nu) * dila;
+        Flux3[p] = 2.0 * nu * a8 + (be - (2.0 / 3.0) * nu) * dila;
     });
     // x momentum: Qh1 = dFx + dFy + dFz, Qh5 = dEx + dEy + dEz
     // (each line pair: a flux and its product with a velocity component, the
@@ -694,10 +710,12 @@ static int hyper_rhs_t(st_ctx *c, const double *Q, R *Qrhs, const double *Y, con
     ST_TRY(dfd(c, 2, 0, pr_mul(kh, GTz), h5, 1, 1.0));
     if (!direct)
         PFOR(c, nc, io(h1, h2, h3, h5) + 8 * io(Qrhs), {
-            Qrhs[p] = Qrhs[p] + h1[p];
-            Qrhs[n3 + p] = Qrhs[n3 + p] + h2[p];
-            Qrhs[2 * n3 + p] = Qrhs[2 * n3 + p] + h3[p];
-            Qrhs[4 * n3 + p] = Qrhs[4 * n3 + p] + h5[p];
+            const R a1 = h1[p], a2 = h2[p], a3 = h3[p], a5 = h5[p];
+            const R r1 = Qrhs[p], r2 = Qrhs[n3 + p], r3 = Qrhs[2 * n3 + p], r5 = Qrhs[4 * n3 + p];
+            Qrhs[p] = r1 + a1;
+            Qrhs[n3 + p] = r2 + a2;
+            Qrhs[2 * n3 + p] = r3 + a3;
+            Qrhs[4 * n3 + p] = r5 + a5;
         });
     return ST_OK;
 }
@@ -789,9 +807,10 @@ __device__ __forceinline__ void bc_cell(const BcArgs &b, int face, size_t q, dou
 // row of each line is wanted, which the elimination gives without the back
 // substitution, and which the rows more than 48 before it do not reach (0.38
 // per row: 2e-20).  A block takes 32 lines: its threads form the pressure of
-// their last rows, one warp runs the elimination and the conditions.  Against
-// the pressure as a field and three whole derivatives (120 bytes per cell): see
-// bc_rhs_t.
+// their last rows, one warp runs the elimination and the conditions.  Latency
+// of that serial elimination bounds it: 384^3, three faces at 0.10 ms a stage,
+// where the pressure as a field and its three whole derivatives (120 bytes per
+// cell) took 0.45 + 3 * 0.2 ms.
 constexpr int kFaceRows = 48;
 struct FaceArgs {
     BcArgs b;
@@ -1370,12 +1389,17 @@ static int lddrk4_sf(st_ctx *c) {
             ST_TRY(rhs_t<R>(c, Q, sc.q(Q), dQ, c->Y, false, &keep));
             ST_TRY(hyper_rhs_t<R>(c, Q, dQ, c->Y, sc.y(c->Y), &keep));
             PFOR(c, nc, 5 * io(dQ, Q, Q, QW) + (first ? 0.0 : 5 * io(QW)), {
-                double dt = dtp[(one ? 0 : p / n3c) * kScal];
+                const double dt = dtp[(one ? 0 : p / n3c) * kScal];
+                double qo[5], w[5], d[5];
                 for (int l = 0; l < 5; l++) {
-                    size_t q = l * n3 + p;
-                    double qw = first ? dt * dQ[q] : al * QW[q] + dt * dQ[q];
-                    QW[q] = qw;
-                    Q[q] = Q[q] + be * qw;
+                    qo[l] = Q[l * n3 + p];
+                    d[l] = dQ[l * n3 + p];
+                    w[l] = first ? 0.0 : QW[l * n3 + p];
+                }
+                for (int l = 0; l < 5; l++) {
+                    const double qw = first ? dt * d[l] : al * w[l] + dt * d[l];
+                    QW[l * n3 + p] = qw;
+                    Q[l * n3 + p] = qo[l] + be * qw;
                 }
             });
             for (int l = 0; l < 5; l++) {
@@ -1428,7 +1452,10 @@ static int lddrk4_mf(st_ctx *c) {
             // sides of the shell's cells are stored as the routine leaves them
             const Sponge sp = sponge_of(c);
             PFOR(c, nc, 5 * io(dQ, Q, Q, QW) + (first ? 0.0 : 5 * io(QW)) + io(Y, drYi, rYW, rY) + (first ? 0.0 : io(rYW)) + sp.shell * (5 * io(dQ) + io(drYi)), {
-                // every load before the first store (which might alias them)
+                // every load before the first store (which might alias them):
+                // 384^3 FP64 2.05 ms at 6.7 TB/s, memory-bound (3.1 ms with loads
+                // between the stores, 2.23 + 0.75 ms as update and sponge apart);
+                // 256^3 FP32 0.54 ms (0.66 + 0.23)
                 double qo[5], w[5], d[5];
                 for (int l = 0; l < 5; l++) {
                     qo[l] = Q[l * n3 + p];
@@ -1472,12 +1499,12 @@ static int lddrk4_mf(st_ctx *c) {
             float *qs = nullptr, *ys = nullptr;
             if constexpr (!is_fp64<R>()) { qs = sc.qs; ys = sc.ys; fresh = true; }
             PFOR(c, nc, 5 * io(Q) + io(rY, g, Y, Q) + (qs ? 5 * io(qs) + io(ys) : 0.0), {
-                double q1 = Q[p], q2 = Q[n3 + p], q3 = Q[2 * n3 + p], q4 = Q[3 * n3 + p];
-                double y = rY[p] / q4;
+                const double q1 = Q[p], q2 = Q[n3 + p], q3 = Q[2 * n3 + p], q4 = Q[3 * n3 + p], qe = Q[4 * n3 + p], ge = g[p];
+                const double y = rY[p] / q4;
                 Y[p] = y;
-                double fac1 = g[p] - 1.0;
+                double fac1 = ge - 1.0;
                 double Vs = 1.0 / q4;
-                double P = fac1 * (Q[4 * n3 + p] - 5.0e-1 * Vs * (q1 * q1 + q2 * q2 + q3 * q3));
+                double P = fac1 * (qe - 5.0e-1 * Vs * (q1 * q1 + q2 * q2 + q3 * q3));
                 if (P < 0.0) P = 0.71429;
                 double q5 = (1.0 / fac1) * P + 5.0e-1 * Vs * (q1 * q1 + q2 * q2 + q3 * q3);
                 Q[4 * n3 + p] = q5;
