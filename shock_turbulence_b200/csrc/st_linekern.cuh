@@ -31,6 +31,7 @@
 #include <type_traits>
 #include <utility>
 #include "st_line.cuh"
+#include "st_once.h"
 
 namespace st {
 
@@ -387,13 +388,17 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
 // with the 128-byte swizzle for y lines
 int line_map(st_ctx *c, CUtensorMap *m, const void *p, bool f32, int dir, int nl, int box);
 
+// The dynamic shared memory a kernel may ask for is an attribute of the kernel
+// on one device.  It is raised to the device's maximum before the kernel's
+// first launch there: a limit that follows the launches' sizes would have to be
+// raised again for each, and two threads with contexts of different sizes could
+// lower it under each other's launch.
 template <auto Kern>
-static void set_smem(size_t bytes) {
-    static size_t done = 0;   // one counter per kernel instantiation
-    if (bytes > done) {
-        cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        done = bytes;
-    }
+static cudaError_t allow_smem(const st_ctx *c) {
+    static OncePerDevice once;   // one mark per kernel instantiation
+    return (cudaError_t)once(c->dev, [&] {
+        return (int)cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_cta);
+    });
 }
 
 // One launch: fields in[0..NIN-1], outputs out[0..NOUT-1] (a.red set), the
@@ -440,8 +445,8 @@ static int launch_lines(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *const
     const size_t smem = (size_t)K * slot + tail;
     long grid = (long)c->sms * ctas;
     if (grid > a.ntile) grid = a.ntile;
+    ST_CUDA(c, (allow_smem<k_lines<R, S, M, L, YT, CYC, T>>(c)));
     int pi = prof_start(c, name, fields * sizeof(T) * (double)c->ncell());
-    set_smem<k_lines<R, S, M, L, YT, CYC, T>>(smem);
     void (*kern)(const LineArgsT<T>) = k_lines<R, S, M, L, YT, CYC, T>;
     const cudaError_t e = launch_pdl(kern, dim3((unsigned)grid), dim3(threads), smem, c->stream, a);
     prof_stop(c, pi);
