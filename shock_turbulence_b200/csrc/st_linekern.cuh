@@ -109,17 +109,27 @@ __device__ __forceinline__ void bar_init(unsigned bar) { asm volatile("mbarrier.
 __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase to complete, at most ~2e6 polls (a poll suspends the
-// thread for a while, so this is seconds); past that the flag is set and the
-// results are garbage, which the host reports at the next synchronising call.
-__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, int *flag) {
-    for (int i = 0; i < 2000000; i++) {
-        unsigned ok;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return;
+__device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits for the phase to complete; false if it does not within a second.  (By
+// the clock, because how long a poll suspends the thread is the hardware's
+// choice, and by polls, so that a kernel which was itself not running for a
+// second looks again.)
+constexpr unsigned long long kWaitNs = 1000000000ull;
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+    unsigned long long t0 = 0;
+    for (;;) {
+        for (int i = 0; i < 64; i++)
+            if (bar_try(bar, parity)) return true;
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > kWaitNs) return false;
     }
-    *reinterpret_cast<volatile int *>(flag) = 1;
 }
 __device__ __forceinline__ void tma_load(unsigned dst, const CUtensorMap *m, int c0, int c1, int c2, int c3, unsigned bar) {
     asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
@@ -138,16 +148,17 @@ __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.
 
 // ---- the kernel ------------------------------------------------------------
 // shared memory: K slots of NT tiles, the carry buffers, the slots' barriers
-constexpr int kSlotsMax = 4;
+constexpr int kSlotsMax = 3;
+constexpr unsigned kRingBytes = 8u * kSlotsMax + 8u;      // barriers, and the mark of a wait that ran out
 template <class V, int L> __host__ __device__ constexpr unsigned corner_bytes() { return 4 * L * sizeof(V); }
 // bytes behind the tiles: the carry buffers (two of one value per segment and
 // column, or one of two values for the filter), the corner values, the
-// barriers, the filter's outer factors
+// barriers and the mark, the filter's outer factors
 // (a scan of float carries needs one column more)
 template <class V, int L>
 __host__ __device__ inline unsigned carry_one(int P) { return (unsigned)(P + (std::is_same<V, F2>::value ? 1 : 0)) * L * (unsigned)sizeof(V); }
 template <class V, int L>
-__host__ __device__ inline unsigned carry_bytes(int P) { return 2u * carry_one<V, L>(P) + corner_bytes<V, L>() + 8u * kSlotsMax; }
+__host__ __device__ inline unsigned carry_bytes(int P) { return 2u * carry_one<V, L>(P) + corner_bytes<V, L>() + kRingBytes; }
 
 template <int S, int M, int L, bool YT, bool CYC, class T, class OPD, class Mid>
 __device__ __forceinline__ void run_op(const LineArgsT<T> &a, const OpArgT<T> &o, const unsigned char *tabs,
@@ -275,10 +286,11 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
     const int tid = threadIdx.x, lane = tid % L, s = tid / L;
     unsigned char *tail = smem + K * slot_b;
     const unsigned cbb = (PENM ? 2u : 1u) * carry_one<V, L>(P * M);
-    unsigned char *tab = tail + 2 * cbb + corner_bytes<V, L>() + 8 * kSlotsMax;
+    unsigned char *tab = tail + 2 * cbb + corner_bytes<V, L>() + kRingBytes;
     const CarryT<V, L> cb{reinterpret_cast<V *>(tail), reinterpret_cast<V *>(tail + cbb), reinterpret_cast<V *>(tail + 2 * cbb),
                           reinterpret_cast<const V *>(tab)};
     const unsigned bars = smem_u32(tail + 2 * cbb + corner_bytes<V, L>());
+    volatile int *const late = reinterpret_cast<int *>(tail + 2 * cbb + corner_bytes<V, L>() + 8 * kSlotsMax);
     if constexpr (PEN) pen_fill(reinterpret_cast<double *>(tab), a.p, P * M, S / M, !PENM);
     else RecipeRun<R>::template fill_tables<S, M, T>(a, tab);
 
@@ -325,6 +337,7 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
 #pragma unroll
         for (int f = 0; f < I::stores(); f++) asm volatile("prefetch.tensormap [%0];" ::"l"(&a.out[f]) : "memory");
         for (int k = 0; k < K; k++) bar_init(bars + 8 * k);
+        *late = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         proxy_fence();
     }
@@ -337,27 +350,46 @@ __global__ void __maxnreg__(80) k_lines(const __grid_constant__ LineArgsT<T> a) 
     View<S, L, YT, T> w;
     w.tb = tb; w.lane = lane; w.n = n; w.a = s * S; w.mid = TileAcc<L, YT, T>::start(lane, s * S);
     w.k0 = (typename Val<T>::A)a.k0; w.k1 = (typename Val<T>::A)a.k1; w.k2 = (typename Val<T>::A)a.k2;
+    // A wait that runs out ends the CTA: nothing of its tile is stored or
+    // loaded, the host reports the flag at the next synchronising call.  Threads
+    // may differ about it, so the mark decides: it is written before the first
+    // barrier of a tile and read between that and the barrier at its end.  (The
+    // end on the mark costs 7 % of the second derivative with the first along y
+    // and 1 % elsewhere at most; a barrier that reduces the threads' results
+    // instead, or loops that run on without it, cost more.)
     int k = 0, kp = K - 1;          // slot of this tile and of the one before
     unsigned par = 0;
     for (int tile = blockIdx.x; tile < a.ntile; tile += G) {
-        bar_wait(bars + 8 * k, par, a.wait_flag);
+        if (!bar_wait(bars + 8 * k, par)) {
+            *late = 1;
+            *reinterpret_cast<volatile int *>(a.wait_flag) = 1;
+        }
         w.sm = smem + k * slot_b;
         const int next = tile + (K == 1 ? 1 : K - 1) * G;
         const bool more = next < a.ntile;
         RecipeRun<R>::template run<S, M, L, YT, CYC, T>(a, tab, w, s, lane, cb, [&](auto q) {
             constexpr int OP = decltype(q)::value;
+            constexpr bool STORES = OP > 0 && I::io(OP > 0 ? OP - 1 : 0) >= 0;
+            if ((STORES || K == 1) && *late) return;
             // the result of the operation before leaves, and with one slot
             // the tiles that are free are filled for the next tile of lines
-            if constexpr (OP > 0) {
-                if constexpr (I::io(OP > 0 ? OP - 1 : 0) >= 0) store_out(tile, k, OP - 1);
-            }
+            if constexpr (STORES) store_out(tile, k, OP - 1);
             if (K == 1 && more) {
                 if constexpr (OP == 0) expect(0);
                 constexpr unsigned FREED = I::freed(OP);
                 if constexpr (FREED != 0) load_tiles(next, 0, FREED);
             }
         }, std::make_index_sequence<I::N>());
+        const int dead = *late;
         __syncthreads();
+        if (dead) {
+            // the slots that loads are in flight to, the tile's own first: the
+            // CTA's shared memory has to stay until they have landed
+            if (tid == 0)
+                for (int j = 0, m = K > 1 && tile >= G ? K - 1 : K; j < m && tile + j * G < a.ntile; j++)
+                    bar_wait(bars + 8 * (k + j < K ? k + j : k + j - K), k + j < K ? par : par ^ 1);
+            break;
+        }
         if (tid == 0) {
             store_out(tile, k, I::N - 1);
             if (K == 1) {
