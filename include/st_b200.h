@@ -148,8 +148,8 @@ int  st_pentadiagonal(st_ctx *c, const double *A, const double *B, const double 
 /* No counterpart in the reference.  st_tridiagonal for callers that must not
  * allocate device memory (a host program that owns the device's memory through
  * its own pool, or a time-critical loop where a cudaMalloc may block on the
- * driver): the working copies of A and B live in a fixed static device array
- * instead of cudaMalloc'd buffers.
+ * driver): the workspace is a fixed static device array instead of a
+ * cudaMalloc'd buffer.  As in st_tridiagonal, R may overlap A, B or C.
  * n*lot <= 262144 (ST_E_ARG beyond); A, B, C, R must be device arrays of the
  * context's device (ST_E_ARG for host arrays).  The first call on a device
  * looks the array up (cudaGetSymbolAddress) and should come before any stream

@@ -12,10 +12,12 @@
 // from a fixed array in the library's static device memory instead.
 //
 // Limits and rules:
-//  - n * lot must not exceed kNoAllocMaxElems (262144, i.e. 2 x 2 MiB of
+//  - n * lot must not exceed kNoAllocMaxElems (262144, i.e. 3 x 2 MiB of
 //    scratch per device); larger systems are rejected with ST_E_ARG.
 //  - A, B, C and R must be device memory of the context's device; host arrays
 //    are rejected (staging them would allocate).
+//  - R may overlap A, B or C (at any offset): the solve reads them ahead of the
+//    rows it writes, so such an R is solved in the scratch and copied back.
 //  - The first call on each device looks up the scratch array's address with
 //    cudaGetSymbolAddress; the driver may load the library's device code at
 //    that moment.  Make that first call before any stream capture begins.
@@ -37,8 +39,8 @@ constexpr size_t kNoAllocMaxElems = size_t(1) << 18;
 constexpr int kMaxDevices = 64;
 
 // a call with N = n*lot elements uses the first N entries, or 2N for periodic
-// lines
-__device__ __align__(256) double g_tri_scratch[2 * kNoAllocMaxElems];
+// lines, and N more for an R that overlaps a coefficient
+__device__ __align__(256) double g_tri_scratch[3 * kNoAllocMaxElems];
 
 std::mutex g_setup_mu;
 double *g_scratch_ptr[kMaxDevices] = {};
@@ -94,7 +96,12 @@ static int tridiagonal_noalloc(st_ctx *c, const double *A, const double *B, cons
     double *a = nullptr;
     int rc = scratch_on(c, c->dev, &a);
     if (rc != ST_OK) return rc;
-    ST_TRY(dev_tridiagonal(c, A, B, C, R, a, n, lot, nper));
+    double *x = R;
+    for (const double *co : {A, B, C})
+        if (co < R + N && R < co + N) x = a + (size_t)solver_fields(false, nper) * N;
+    if (x != R) ST_CUDA(c, cudaMemcpyAsync(x, R, N * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    ST_TRY(dev_tridiagonal(c, A, B, C, x, a, n, lot, nper));
+    if (x != R) ST_CUDA(c, cudaMemcpyAsync(R, x, N * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     ST_CUDA(c, cudaStreamSynchronize(c->stream));
     return ST_OK;
 }

@@ -94,3 +94,28 @@ def test_rejects_host_arrays(solver):
     assert st == ST_E_ARG
     assert b"device arrays" in solver.lib.st_last_error(solver._h)
     assert np.all(R == 1.0)
+
+
+@pytest.mark.parametrize("nper", [0, 1])
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("rows", [0, 24, -24, 40])
+def test_right_hand_side_overlaps_a_coefficient(solver, nper, which, rows):
+    """R starts some rows behind (before) A, B or C in one array; 24 rows are
+    more than the solve reads ahead, 40 lie within its 64 rows.  Bits as with
+    an array of its own."""
+    import torch
+    n, lot = 64, 96
+    N = n * lot
+    rng = np.random.default_rng(5)
+    A, B, C, _ = (torch.from_numpy(x.ravel()).cuda() for x in _system(rng, n, lot))
+    buf = torch.from_numpy(rng.uniform((0.1, 0.9, 0.1)[which], (0.4, 1.1, 0.4)[which], 3 * N)).cuda()
+    co = [A, B, C]
+    co[which] = buf[N:2 * N]
+    R = buf[N + rows * lot:2 * N + rows * lot]
+    own = [x.clone() for x in (*co, R)]
+    torch.cuda.synchronize()
+    st = _noalloc(solver, *own, n, lot, nper)
+    assert st == 0, solver.lib.st_last_error(solver._h)
+    st = _noalloc(solver, *co, R, n, lot, nper)
+    assert st == 0, solver.lib.st_last_error(solver._h)
+    assert torch.equal(R, own[3])
