@@ -272,7 +272,9 @@ int  st_get_time(st_ctx *c, double *time);
 int  st_set_time(st_ctx *c, double time);
 int  st_query(st_ctx *c);
 /* No reference counterpart: device bytes the context holds (COMMON mirrors,
- * scratch pool, tables); the pool grows during the first steps. */
+ * scratch pool, tables, workspace of the line solvers); the pool grows during
+ * the first steps, the workspace with the largest solve (what is above 1 GiB is
+ * given back when the call ends). */
 int  st_memory(st_ctx *c, long long *bytes);
 
 /* ---- Output-side diagnostics (_mf family) ----------------------------------

@@ -1109,9 +1109,10 @@ int st_memory(st_ctx *c, long long *bytes) {
     if (!c || !bytes) return ST_E_ARG;
     const size_t fb = c->fs * sizeof(double);
     // COMMON mirrors (13 double state fields; 25 intermediate fields, float in
-    // the FP32 mode), tables, scalars and the scratch pool
+    // the FP32 mode), tables, scalars, the line solvers' workspace and the
+    // scratch pool
     const size_t ib = fp32_mode(c) ? fb / 2 : fb;
-    size_t b = 13 * fb + 25 * ib + c->table_bytes + (size_t)c->nb * kScal * sizeof(double);
+    size_t b = 13 * fb + 25 * ib + c->table_bytes + (size_t)c->nb * kScal * sizeof(double) + c->solver_ws_bytes;
     for (auto &e : c->pool) b += e.bytes;
     *bytes = (long long)b;
     return ST_OK;

@@ -82,3 +82,29 @@ def test_overlapping_right_hand_side(solver, nper):
     torch.cuda.synchronize()
     solver.tridiagonal(A, B, y, y, n, lot, nper)
     assert torch.equal(x, y)
+
+
+def test_memory_counts_the_workspace():
+    """st_memory follows the solvers' workspace: room for one field of a
+    tridiagonal solve of device arrays, for its four arrays too from the host."""
+    import ctypes
+    import torch
+    from shock_turbulence_b200 import Solver
+
+    def held(s):
+        b = ctypes.c_longlong()
+        assert s.lib.st_memory(s._h, ctypes.byref(b)) == 0
+        return b.value
+
+    s = Solver(default_params(16))
+    n, lot = 100, 200
+    rng = np.random.default_rng(4)
+    host = rows(rng, n, lot, 0.3, 1.0, 0.3, 0.0)
+    dev = [torch.from_numpy(x).cuda() for x in host]
+    torch.cuda.synchronize()
+    start = held(s)
+    s.tridiagonal(*dev, n, lot, 0)
+    assert held(s) - start == 8 * n * lot
+    s.tridiagonal(*host, n, lot, 0)
+    assert held(s) - start == 5 * 8 * n * lot
+    s.close()
