@@ -35,7 +35,14 @@ void *scratch_bytes(st_ctx *c, size_t bytes) {
     for (auto &e : c->pool)
         if (!e.used && e.bytes == bytes) { e.used = true; return e.p; }
     void *p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && c->solver_ws) {
+        // the line solvers' workspace is kept only while there is room (no
+        // call that uses it takes scratch fields)
+        solver_workspace_free(c);
+        e = cudaMalloc(&p, bytes);
+    }
+    if (e != cudaSuccess) {
         cudaGetLastError();
         c->pool_oom = true;
         throw OomError();
@@ -402,7 +409,7 @@ int st_destroy(st_ctx *c) {
     for (float *a : c->hypf) if (a) cudaFree(a);
     for (float *a : c->dYdf) if (a) cudaFree(a);
     for (auto &e : c->pool) cudaFree(e.p);
-    if (c->solver_ws) cudaFree(c->solver_ws);
+    solver_workspace_free(c);
     if (c->hpinned) cudaFreeHost(c->hpinned);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;

@@ -324,6 +324,7 @@ int dev_to_double(st_ctx *c, const float *x, double *y, size_t n);
 int solver_fields(bool pen, int nper);
 double *solver_workspace(st_ctx *c, size_t bytes);
 void solver_workspace_trim(st_ctx *c);
+void solver_workspace_free(st_ctx *c);
 int dev_tridiagonal(st_ctx *c, const double *A, const double *B, const double *C, double *R, double *ws, int n, int lot,
                     int nper);
 int dev_pentadiagonal(st_ctx *c, const double *A, const double *B, const double *C, const double *D, const double *E, double *R,

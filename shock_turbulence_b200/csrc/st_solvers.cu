@@ -280,24 +280,25 @@ __global__ void __launch_bounds__(32) k_pen_per(const double *__restrict__ A, co
 
 }  // namespace
 
-// The solvers' workspace: grows to the largest call's need; what is left of a
-// call above kKeep is given back when it ends.
+// The solvers' workspace: grows to the largest call's need; one above kKeep is
+// given back when its call ends, any when a scratch field finds no room.
 constexpr size_t kKeep = (size_t)1 << 30;
+void solver_workspace_free(st_ctx *c) {
+    if (c->solver_ws) { cudaStreamSynchronize(c->stream); cudaFree(c->solver_ws); }
+    cudaGetLastError();
+    c->solver_ws = nullptr;
+    c->solver_ws_bytes = 0;
+}
 double *solver_workspace(st_ctx *c, size_t bytes) {
     if (bytes > c->solver_ws_bytes) {
-        if (c->solver_ws) { cudaStreamSynchronize(c->stream); cudaFree(c->solver_ws); }
-        c->solver_ws = nullptr;
-        c->solver_ws_bytes = 0;
+        solver_workspace_free(c);
         if (cudaMalloc(&c->solver_ws, bytes) != cudaSuccess) { cudaGetLastError(); c->solver_ws = nullptr; return nullptr; }
         c->solver_ws_bytes = bytes;
     }
     return (double *)c->solver_ws;
 }
 void solver_workspace_trim(st_ctx *c) {
-    if (c->solver_ws_bytes <= kKeep) return;
-    cudaFree(c->solver_ws);
-    c->solver_ws = nullptr;
-    c->solver_ws_bytes = 0;
+    if (c->solver_ws_bytes > kKeep) solver_workspace_free(c);
 }
 
 // fields of workspace the solvers need beside their arguments

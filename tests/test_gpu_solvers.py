@@ -108,3 +108,42 @@ def test_memory_counts_the_workspace():
     s.tridiagonal(*host, n, lot, 0)
     assert held(s) - start == 5 * 8 * n * lot
     s.close()
+
+
+def test_workspace_makes_room_for_scratch():
+    """On a device that is full but for 32 MiB, a routine whose scratch fields
+    need more gets the room that a large solve has left in its context."""
+    import torch
+    from shock_turbulence_b200 import Solver
+    p = default_params(64, 64, 64, re=100.0)
+    s, other = Solver(p), Solver(p)
+    rng = np.random.default_rng(8)
+    Q = np.empty((5,) + s.shape)
+    Q[:3], Q[3], Q[4] = 0.1 * rng.standard_normal((3,) + s.shape), 1.0, 2.0
+    Y = np.full(s.shape, 0.5)
+    ref = other.field(5)
+    other.Compute_gamma(Y)
+    other.RHS(Q.copy(), ref, Y)
+    other.close()
+    n, lot = 512, 120000                       # half a gigabyte of workspace
+    co = [torch.full((n * lot,), v, dtype=torch.float64, device="cuda") for v in (0.3, 1.0, 0.3, 0.0)]
+    torch.cuda.synchronize()
+    s.tridiagonal(*co, n, lot, 0)
+    del co
+    torch.cuda.empty_cache()
+    full = []
+    for size in (1 << 30, 1 << 25, 1 << 21):
+        while torch.cuda.mem_get_info()[0] > size + (1 << 25):
+            try:
+                full.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                break
+    out = s.field(5)
+    try:
+        s.Compute_gamma(Y)
+        s.RHS(Q.copy(), out, Y)
+    finally:
+        del full
+        torch.cuda.empty_cache()
+        s.close()
+    assert np.array_equal(out, ref)
