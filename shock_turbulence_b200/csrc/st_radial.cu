@@ -1153,6 +1153,10 @@ int st_radial_create(const st_radial_params *p, int nprob, const int *n, const d
     fill_k(h->k);
     Flat flat;
     fill_flat(flat);
+    // the blocks keep the first kPrTri and kPrPen rows; those behind them take
+    // the constant factors
+    if (flat.d1.i0 > kPrTri || flat.d2.i0 > kPrTri || flat.f.i0 > kPrPen)
+        return bail(ST_E_UNSUPPORTED, "the factors are not constant behind the rows that are kept");
     // factor tables: universal prefixes from the longest length, tails per length
     const int NM = std::max(h->nmax, kMinN);
     std::vector<double> B, C, D, l1, i1, u1, l2, i2, u2, F[5];
