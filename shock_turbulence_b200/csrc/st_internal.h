@@ -17,7 +17,6 @@ namespace st {
 
 constexpr int kMaxSeg = 32;       // max segments per line
 constexpr int kLanes = 16;        // columns of a line-kernel CTA (half a warp; a warp holds two segments)
-constexpr int kLineThreads = kLanes * kMaxSeg;     // threads of a line-kernel CTA at most
 constexpr int kMaxRows = 16;      // max rows per segment
 
 // A line of n rows is split into P = n/S <= kMaxSeg segments of S rows (8 or

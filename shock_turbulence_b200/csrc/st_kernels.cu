@@ -90,8 +90,15 @@ static void set_d1(st_ctx *c, LineArgsT<T> &a, int k, int asym, int iadd, double
 
 template <class T>
 static int dfd_t(st_ctx *c, int dir, int asym, const ProdT<T> &F, T *dF, int iadd, double cadd) {
-    static const RecId rec[] = {R_D1, R_MUL, R_ADDMUL, R_MULMUL, R_SPEC, R_SPECT, R_HMULADD};
-    static const int nin[] = {1, 2, 3, 3, 3, 4, 3};
+    RecId id;
+    int nin;
+    switch (F.op) {
+        case PR_A: id = R_D1; nin = 1; break;
+        case PR_MUL: id = R_MUL; nin = 2; break;
+        case PR_ADDMUL: id = R_ADDMUL; nin = 3; break;
+        case PR_HMULADD: id = R_HMULADD; nin = 3; break;
+        default: return fail(c, ST_E_UNSUPPORTED, "this operand has a derivative in a pair only");
+    }
     LineArgsT<T> a = make_args<T>(c, dir);
     set_d1(c, a, 0, asym, iadd, cadd);
     a.k0 = F.k0; a.k1 = F.k1; a.k2 = F.k2;
@@ -99,9 +106,9 @@ static int dfd_t(st_ctx *c, int dir, int asym, const ProdT<T> &F, T *dF, int iad
     // plus that of c
     if (F.op == PR_HMULADD && sizeof(T) == 4) { a.op[1] = a.op[0]; a.op[1].fac1 = 0.5 * a.op[0].fac1; }
     const T *in[4] = {F.a, F.b, F.c, F.d};
-    for (int k = 0; k < nin[F.op]; k++) ST_TRY(aligned(c, in[k]));
+    for (int k = 0; k < nin; k++) ST_TRY(aligned(c, in[k]));
     ST_TRY(aligned(c, dF));
-    return launch(c, rec[F.op], a, in, &dF);
+    return launch(c, id, a, in, &dF);
 }
 
 // D2F*2: d2F, and dF where given (iadd)
@@ -180,8 +187,8 @@ int dev_gauss_f(st_ctx *c, int dir, const float *F, float *Fg) { return gauss_t<
 //   A  F, U F            B  a b, c (a b)            C  the species flux, its energy counterpart
 //   D  a u, (b + c) u    E  a u, b u
 // Each operation is the single one's arithmetic, so the results are those of
-// two launches.  Any other pair, and one whose operations add to the same
-// field, runs as two launches.
+// two launches.  A pair of other operands that have one of their own runs as
+// two launches.
 template <class T>
 static int dfd_pair_t(st_ctx *c, int dir, const D1SpecT<T> *ops) {
     const ProdT<T> &p = ops[0].F, &q = ops[1].F;

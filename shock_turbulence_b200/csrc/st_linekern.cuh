@@ -56,13 +56,10 @@ struct Recipe {
 using RecD1 = Recipe<1, 1, Op<OP_D1, Src<PR_A, 0>, 0, 0>>;
 using RecMul = Recipe<2, 2, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, 0>>;
 using RecAddMul = Recipe<3, 3, Op<OP_D1, Src<PR_ADDMUL, 0, 1, 2>, 0, 0>>;
-using RecMulMul = Recipe<3, 3, Op<OP_D1, Src<PR_MULMUL, 0, 1, 2>, 0, 0>>;
 using RecHMulAdd = Recipe<3, 3, Op<OP_D1, Src<PR_HMULADD, 0, 1, 2>, 0, 0>>;
 // a b, plus c's derivative: the FP32 mode's form of RecHMulAdd, which would
 // round the sum to the pressure's magnitude before it is differenced
 using RecMulPlus = Recipe<3, 3, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, -1, 1>, Op<OP_D1ADD, Src<PR_A, 2>, 0, 0>>;
-using RecSpec = Recipe<3, 3, Op<OP_D1, Src<PR_SPEC, 0, 1, 2>, 0, 0>>;
-using RecSpecT = Recipe<4, 4, Op<OP_D1, Src<PR_SPECT, 0, 1, 2, 3>, 0, 0>>;
 using RecD2 = Recipe<1, 1, Op<OP_D2, Src<PR_A, 0>, 0, 0>>;
 using RecD2D1 = Recipe<1, 2, Op<OP_D2, Src<PR_A, 0>, 1, 0>, Op<OP_D1, Src<PR_A, 0>, 0, 1>>;
 using RecFilter = Recipe<1, 1, Op<OP_FILTER, Src<PR_A, 0>, 0, 0>>;
@@ -502,15 +499,14 @@ static int launch_lines_L(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *con
 }
 
 // recipe by number
-enum RecId { R_D1, R_MUL, R_ADDMUL, R_MULMUL, R_HMULADD, R_SPEC, R_SPECT, R_D2, R_D2D1, R_FILTER, R_GAUSS, R_LAP,
-             R_PAIRA, R_PAIRB, R_PAIRC, R_PAIRD, R_PAIRE };
+enum RecId { R_D1, R_MUL, R_ADDMUL, R_HMULADD, R_D2, R_D2D1, R_FILTER, R_GAUSS, R_LAP, R_PAIRA, R_PAIRB, R_PAIRC, R_PAIRD,
+             R_PAIRE };
 
 template <int S, int M, bool CYC, class T>
 static int launch_rec_S(st_ctx *c, RecId id, LineArgsT<T> &a, const T *const *in, T *const *out) {
     switch (id) {
 #define REC(id_, rec_, name_) case id_: return launch_lines_L<rec_, S, M, CYC, T>(c, a, in, out, name_);
         REC(R_D1, RecD1, "k_dfd") REC(R_MUL, RecMul, "k_dfd") REC(R_ADDMUL, RecAddMul, "k_dfd")
-        REC(R_MULMUL, RecMulMul, "k_dfd")
         case R_HMULADD:
             return launch_lines_L<std::conditional_t<sizeof(T) == 8, RecHMulAdd, RecMulPlus>, S, M, CYC, T>(c, a, in, out, "k_dfd");
         REC(R_D2, RecD2, "k_d2fd2") REC(R_D2D1, RecD2D1, "k_d2fd2") REC(R_GAUSS, RecGauss, "k_gauss")
@@ -520,8 +516,6 @@ static int launch_rec_S(st_ctx *c, RecId id, LineArgsT<T> &a, const T *const *in
             if constexpr (sizeof(T) == 8) return launch_lines_L<RecFilter, S, M, CYC, T>(c, a, in, out, "k_filter");
             break;                    // the compact filter acts on the FP64 state only
         // the species terms and the first-derivative Laplacian exist in the _mf family only
-        case R_SPEC: if constexpr (!CYC) return launch_lines_L<RecSpec, S, M, CYC, T>(c, a, in, out, "k_dfd"); break;
-        case R_SPECT: if constexpr (!CYC) return launch_lines_L<RecSpecT, S, M, CYC, T>(c, a, in, out, "k_dfd"); break;
         case R_PAIRC: if constexpr (!CYC) return launch_lines_L<RecPairC, S, M, CYC, T>(c, a, in, out, "k_dfd_pair"); break;
         case R_LAP: if constexpr (!CYC) return launch_lines_L<RecLap, S, M, CYC, T>(c, a, in, out, "k_lap"); break;
 #undef REC

@@ -731,10 +731,11 @@ static int species_rhs_t(st_ctx *c, const double *Q, const R *Qr, R *Qrhs, const
     Phys f = phys(c);
     const double *Q1 = Q, *Q2 = Q + n3, *Q3 = Q + 2 * n3, *Q4 = Q + 3 * n3, *Q5 = Q + 4 * n3;
     const R *q1r = Qr, *q2r = Qr + n3, *q3r = Qr + 2 * n3, *q4r = Qr + 3 * n3;
-    // FP64: Ydiff's terms go straight to Yrhs.  Tkept: RHS's T of this stage
+    // FP64: Ydiff's terms go straight to Yrhs (where it is a field of its own:
+    // the pairs below do not add to one field twice).  Tkept: RHS's T of this stage
     // (the momentum round trip between the two changes it in the last bit in
     // FP64, and is not made in the FP32 mode).
-    const bool direct = is_fp64<R>();
+    const bool direct = is_fp64<R>() && Yrhs != Qrhs + 4 * n3;
     ScratchNT<R> Yds(c, direct ? 0 : 1), Ts(c, Tkept ? 0 : 1);
     R *Yd = direct ? Yrhs : Yds[0];
     const R *T = Tkept ? Tkept : Ts[0];
