@@ -101,7 +101,7 @@ enum ProdOp {
     PR_MULMUL,       // c*(a*b)
     PR_SPEC,         // a*b*c + a*c*k0*k1             (Species_RHS flux)
     PR_SPECT,        // (k0*d)*(a*b*c + a*c*k0b*k1)    (its energy counterpart)
-    PR_HMULADD,      // a*b/2 + c        (half a momentum flux plus the pressure: one derivative for both)
+    PR_MULPLUS,      // a*b, and c       (half the derivative of a momentum flux plus that of the pressure)
 };
 template <class T>
 struct ProdT {

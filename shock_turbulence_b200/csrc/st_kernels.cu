@@ -96,15 +96,14 @@ static int dfd_t(st_ctx *c, int dir, int asym, const ProdT<T> &F, T *dF, int iad
         case PR_A: id = R_D1; nin = 1; break;
         case PR_MUL: id = R_MUL; nin = 2; break;
         case PR_ADDMUL: id = R_ADDMUL; nin = 3; break;
-        case PR_HMULADD: id = R_HMULADD; nin = 3; break;
+        case PR_MULPLUS: id = R_MULPLUS; nin = 3; break;
         default: return fail(c, ST_E_UNSUPPORTED, "this operand has a derivative in a pair only");
     }
     LineArgsT<T> a = make_args<T>(c, dir);
     set_d1(c, a, 0, asym, iadd, cadd);
     a.k0 = F.k0; a.k1 = F.k1; a.k2 = F.k2;
-    // a*b/2 + c in the FP32 mode: the derivative of a*b with half the factor,
-    // plus that of c
-    if (F.op == PR_HMULADD && sizeof(T) == 4) { a.op[1] = a.op[0]; a.op[1].fac1 = 0.5 * a.op[0].fac1; }
+    // the derivative of a*b with half the factor, plus that of c
+    if (F.op == PR_MULPLUS) { a.op[1] = a.op[0]; a.op[1].fac1 = 0.5 * a.op[0].fac1; }
     const T *in[4] = {F.a, F.b, F.c, F.d};
     for (int k = 0; k < nin; k++) ST_TRY(aligned(c, in[k]));
     ST_TRY(aligned(c, dF));

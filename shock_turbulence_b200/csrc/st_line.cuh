@@ -112,7 +112,6 @@ __device__ __forceinline__ V prod_val(V a, V b, V c, V d, A k0, A k1, A k2) {
     if constexpr (OP == PR_MUL) return a * b;
     else if constexpr (OP == PR_ADDMUL) return (a + b) * c;
     else if constexpr (OP == PR_MULMUL) return c * (a * b);
-    else if constexpr (OP == PR_HMULADD) return (a * b) * (A)0.5 + c;
     else if constexpr (OP == PR_SPEC) return a * b * c + a * c * k0 * k1;
     else if constexpr (OP == PR_SPECT) { V fl = a * b * c + a * c * k0 * k1; return k2 * d * fl; }
     else return a;

@@ -56,9 +56,10 @@ struct Recipe {
 using RecD1 = Recipe<1, 1, Op<OP_D1, Src<PR_A, 0>, 0, 0>>;
 using RecMul = Recipe<2, 2, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, 0>>;
 using RecAddMul = Recipe<3, 3, Op<OP_D1, Src<PR_ADDMUL, 0, 1, 2>, 0, 0>>;
-using RecHMulAdd = Recipe<3, 3, Op<OP_D1, Src<PR_HMULADD, 0, 1, 2>, 0, 0>>;
-// a b, plus c's derivative: the FP32 mode's form of RecHMulAdd, which would
-// round the sum to the pressure's magnitude before it is differenced
+// a b with half the factor, plus c's derivative.  (One derivative of a b / 2 + c
+// rounds the sum to the magnitude of c, the pressure, before it is differenced:
+// the rms error of the y and z momentum right-hand sides against an extended
+// precision grew by 2 to 7 %.)
 using RecMulPlus = Recipe<3, 3, Op<OP_D1, Src<PR_MUL, 0, 1>, 0, -1, 1>, Op<OP_D1ADD, Src<PR_A, 2>, 0, 0>>;
 using RecD2 = Recipe<1, 1, Op<OP_D2, Src<PR_A, 0>, 0, 0>>;
 using RecD2D1 = Recipe<1, 2, Op<OP_D2, Src<PR_A, 0>, 1, 0>, Op<OP_D1, Src<PR_A, 0>, 0, 1>>;
@@ -499,7 +500,7 @@ static int launch_lines_L(st_ctx *c, LineArgsT<T> &a, const T *const *in, T *con
 }
 
 // recipe by number
-enum RecId { R_D1, R_MUL, R_ADDMUL, R_HMULADD, R_D2, R_D2D1, R_FILTER, R_GAUSS, R_LAP, R_PAIRA, R_PAIRB, R_PAIRC, R_PAIRD,
+enum RecId { R_D1, R_MUL, R_ADDMUL, R_MULPLUS, R_D2, R_D2D1, R_FILTER, R_GAUSS, R_LAP, R_PAIRA, R_PAIRB, R_PAIRC, R_PAIRD,
              R_PAIRE };
 
 template <int S, int M, bool CYC, class T>
@@ -507,8 +508,7 @@ static int launch_rec_S(st_ctx *c, RecId id, LineArgsT<T> &a, const T *const *in
     switch (id) {
 #define REC(id_, rec_, name_) case id_: return launch_lines_L<rec_, S, M, CYC, T>(c, a, in, out, name_);
         REC(R_D1, RecD1, "k_dfd") REC(R_MUL, RecMul, "k_dfd") REC(R_ADDMUL, RecAddMul, "k_dfd")
-        case R_HMULADD:
-            return launch_lines_L<std::conditional_t<sizeof(T) == 8, RecHMulAdd, RecMulPlus>, S, M, CYC, T>(c, a, in, out, "k_dfd");
+        REC(R_MULPLUS, RecMulPlus, "k_dfd")
         REC(R_D2, RecD2, "k_d2fd2") REC(R_D2D1, RecD2D1, "k_d2fd2") REC(R_GAUSS, RecGauss, "k_gauss")
         REC(R_PAIRA, RecPairA, "k_dfd_pair") REC(R_PAIRB, RecPairB, "k_dfd_pair")
         REC(R_PAIRD, RecPairD, "k_dfd_pair") REC(R_PAIRE, RecPairE, "k_dfd_pair")

@@ -61,11 +61,11 @@ template <class R>
 static ProdT<R> pr_mulmul(const R *a, const R *b, const R *c) {
     ProdT<R> p{}; p.op = PR_MULMUL; p.a = a; p.b = b; p.c = c; return p;
 }
-// a*b/2 + c: a momentum flux taken with the factor -1/2 and the pressure taken
-// with -1 along the same direction are one derivative (with -1) of this sum
+// a momentum flux a*b taken with the factor -1/2 and the pressure c taken with
+// -1 along the same direction: one launch (with -1) that adds their derivatives
 template <class R>
-static ProdT<R> pr_hmuladd(const R *a, const R *b, const R *c) {
-    ProdT<R> p{}; p.op = PR_HMULADD; p.a = a; p.b = b; p.c = c; return p;
+static ProdT<R> pr_mulplus(const R *a, const R *b, const R *c) {
+    ProdT<R> p{}; p.op = PR_MULPLUS; p.a = a; p.b = b; p.c = c; return p;
 }
 
 // Line operators by field type: double arrays, or float arrays in the FP32
@@ -278,7 +278,7 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bo
     const R *cu = u, *cv = v, *cw = w, *cP = P;
     ST_TRY(dfd_pair<R>(c, 0, pr_mul(q4r, cu), Qcx + 3 * n3, 1, 0, -1.0, pr_addmul(q5r, cP, cu), Qcx + 4 * n3, 1, 0,
                        -1.0));
-    ST_TRY(dfd(c, 0, 0, pr_hmuladd(q1r, cu, cP), Qcx, 0, -1.0));
+    ST_TRY(dfd(c, 0, 0, pr_mulplus(q1r, cu, cP), Qcx, 0, -1.0));
     ST_TRY(dfd_pair<R>(c, 0, pr_mul(q2r, cu), Qcx + n3, 1, 0, -5.0e-1, pr_mul(q3r, cu), Qcx + 2 * n3, 1, 0,
                        -5.0e-1));
     ST_TRY(dfd(c, 0, 1, q1r, FF, 0, 1.0));
@@ -298,12 +298,12 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bo
     // d(rho v)/dy and d(rho w)/dz with iadd=0, cadd=-1: Qconv(4) = 0 - d(.) exactly
     ST_TRY(dfd(c, 1, 1, q2r, Qcy + 3 * n3, 0, -1.0));
     ST_TRY(dfd(c, 1, 1, pr_mul(q1r, v), Qcy, 0, -5.0e-1));
-    ST_TRY(dfd(c, 1, 0, pr_hmuladd(q2r, cv, cP), Qcy + n3, 0, -1.0));
+    ST_TRY(dfd(c, 1, 0, pr_mulplus(q2r, cv, cP), Qcy + n3, 0, -1.0));
     ST_TRY(dfd_pair<R>(c, 1, pr_mul(q3r, cv), Qcy + 2 * n3, 1, 0, -5.0e-1, pr_addmul(q5r, cP, cv), Qcy + 4 * n3, 1,
                        0, -1.0));
     ST_TRY(dfd(c, 2, 1, q3r, Qcz + 3 * n3, 0, -1.0));
     ST_TRY(dfd_pair<R>(c, 2, pr_mul(q1r, cw), Qcz, 1, 0, -5.0e-1, pr_mul(q2r, cw), Qcz + n3, 1, 0, -5.0e-1));
-    ST_TRY(dfd(c, 2, 0, pr_hmuladd(q3r, cw, cP), Qcz + 2 * n3, 0, -1.0));
+    ST_TRY(dfd(c, 2, 0, pr_mulplus(q3r, cw, cP), Qcz + 2 * n3, 0, -1.0));
     ST_TRY(dfd(c, 2, 1, pr_addmul(q5r, P, w), Qcz + 4 * n3, 0, -1.0));
     R *d2Ty = dd[0], *d2Tz = dd[1], *d2uy = dd[2], *d2vy = dd[3], *d2wy = dd[4], *d2wz = dd[5];
     R *dGzz_y = dd[6], *d2uz = dd[7], *d2vz = dd[8], *dGxx_y = dd[9], *dGxx_z = dd[10], *dGyx_y = dd[11];
