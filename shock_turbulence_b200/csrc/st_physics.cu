@@ -151,18 +151,22 @@ __device__ __forceinline__ void thermo(const Phys &f, double g, double Y, double
     P = fac1 * (q5 - 5.0e-1 * Vs * (q1 * q1 + q2 * q2 + q3 * q3));
     T = fac3 * Vs * P;
 }
-// viscosity law, src/rhsv_sym_mf.f:253-263
+// viscosity law, src/rhsv_sym_mf.f:253-263, for results stored as R.  Of x^(e-1)
+// the FP32 mode takes x^e / x where that is defined: a power costs some hundred
+// FP64 operations, which bound its pass (256^3 step 106.0 ms, 106.9 with both
+// powers), and the float that is stored does not see the quotient's rounding.
+// In double it would (rms error 0.47 against 0.30 units in the last place,
+// x from 0.5 to 3), and the pass has room for the second power (384^3 step
+// 437.9 and 440.1 ms).
+template <class R>
 __device__ __forceinline__ void viscosity(const Phys &f, double T, double Y, double &mu, double &dmu) {
     double fac1 = f.g1 - 1.0;
     double fac2 = f.vis_exp - 1.0;
     double se = sqrt(f.eps);
     double num = f.Re1_inv * Y + f.Re2_inv * se * (1.0 - Y);
     double den = Y + se * (1.0 - Y);
-    // x^(e-1) = x^e / x: a power costs some hundred FP64 operations, which
-    // bound the pass in the FP32 mode; taken directly where the quotient is
-    // not defined
     const double x = fac1 * T, pw = pow(x, f.vis_exp);
-    const double pd = (pw > 0.0 && pw < INFINITY) ? pw / x : pow(x, fac2);
+    const double pd = sizeof(R) == 4 && pw > 0.0 && pw < INFINITY ? pw / x : pow(x, fac2);
     mu = pw * num / den;
     dmu = pd * num / den * f.vis_exp * fac1;
 }
@@ -264,7 +268,7 @@ static int rhs_t(st_ctx *c, double *Q, const R *Qr, R *Qrhs, const double *Y, bo
         const double ge = gamma_from_Y ? gamma_of(f, y) : g[p];
         double vs, pp, tt, m, dm;
         thermo(f, ge, y, q1, q2, q3, q4, q5, vs, pp, tt);
-        viscosity(f, (R)tt, y, m, dm);
+        viscosity<R>(f, (R)tt, y, m, dm);
         if (gamma_from_Y) g[p] = ge;
         P[p] = pp; T[p] = tt;
         u[p] = q1 * vs;
