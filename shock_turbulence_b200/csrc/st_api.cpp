@@ -948,10 +948,12 @@ static int step_graph(st_ctx *c, int step) {
     return ST_OK;
 }
 
-// A step that the caller waits for takes the graph on grids whose launches
-// cost the host about as much as their kernels cost the GPU (64^3: 8.6 ms
-// enqueued launch by launch, 6.3 ms replayed); larger grids gain nothing and
-// are spared the capture.
+// A step that the caller waits for takes the graph on grids of up to 128^3,
+// where the launches weigh most.  Launch by launch / replayed, ms, periodic FP64
+// and octant FP32: 64^3 6.2 / 5.8 and 11.7 / 10.6, 128^3 20.6 / 19.3 and 29.5 /
+// 25.8, 192^3 56.7 / 55.6 and 50.2 / 47.4.  Beyond, the gain falls (2 to 6 %)
+// and a run of a few steps is spared the capture; st_step_async replays at
+// every size.
 constexpr size_t kGraphCells = (size_t)128 * 128 * 128;
 int st_step(st_ctx *c, double *time, int *step) {
     SINGLE_CASE(c);

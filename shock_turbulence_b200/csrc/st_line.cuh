@@ -544,8 +544,9 @@ __device__ __forceinline__ void pen_scan(double *buf, const double *mat, const d
 // - E_i x_{i+2}) / (C'_i + tiny).  Carries are 2-vectors that reach over most
 // of the line (the system is nearly singular), so one warp runs the carry
 // recurrence over the segments, one thread per column, between two barriers,
-// and every segment then picks up its carry.  Measured against a scan by all
-// threads (five steps of two fmas with a barrier each): see k_lines.
+// and every segment then picks up its carry.  (The FP32 mode's filter keeps a
+// scan by all threads, log2(P) steps with a barrier each: 384^3 runs at 0.45 of
+// a plain copy with either.)
 // Buffer: cb.a is [2][segment][L] and serves both directions (a thread reads
 // and writes its own segment's entry; only the scanning warp touches others,
 // between barriers).

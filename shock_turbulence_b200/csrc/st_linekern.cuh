@@ -9,7 +9,8 @@
 // fills a slot while the CTA's threads solve the slot before it in registers;
 // the results overwrite input tiles that no later operation reads and leave
 // by TMA stores, or by TMA reductions (cp.reduce, add) where the operation
-// accumulates, so the old value never comes to the SM.  Where only one slot
+// accumulates, so the old value never comes to the SM (the reduction keeps
+// subnormal floats; measured).  Where only one slot
 // fits, its tiles are filled for the next lines one by one, as the operations
 // are done with them.
 //
@@ -18,9 +19,9 @@
 // accumulation 5.8 to 6.3 TB/s of its 24 bytes per cell.  With the solve, FP64,
 // 384^3, against kernels that read the rows from global memory thread by
 // thread (about 85 instructions per cell, 512 threads of 64 registers):
-//   first derivative x, y, z   193, 172, 189 us (230, 290, 222)
-//   filter                     322, 309, 317 us (410, 437, 402)
-//   second with first          316, 300, 309 us (490)
+//   first derivative x, y, z   187, 166, 178 us (230, 290, 222)
+//   filter                     316, 299, 310 us (410, 437, 402)
+//   second with first          295, 288, 289 us (490)
 //   two first derivatives of Compute_Laplacian in one pass, accumulated
 //                              285, 258 us (480 as two passes)
 // The solve's latency is what is left: a solve costs about 130 us of a 384^3

@@ -12,10 +12,9 @@
 namespace st {
 
 // ---- launch helpers ----------------------------------------------------------
-// Four 256-thread CTAs per SM (at most 64 registers a thread): the two
-// largest passes (the fused RHS flux passes, 80 registers uncapped) spill
-// about 100 bytes but gain the occupancy; measured 10 % faster on the FP32
-// mode's pointwise family and 2 % on the FP64 one.
+// Four 256-thread CTAs per SM (at most 64 registers a thread) where a pass does
+// not ask for fewer (RHS: two, of up to 122 registers).  Of all passes only the
+// FP32 mode's outflow faces spill (16 bytes).
 template <int CTAS, class Fn>
 __global__ void __launch_bounds__(256, CTAS) k_pfor(size_t n, Fn fn) {
     pdl_wait();
@@ -69,7 +68,7 @@ static ProdT<R> pr_mulplus(const R *a, const R *b, const R *c) {
 }
 
 // Line operators by field type: double arrays, or float arrays in the FP32
-// mode (the kernels compute in double either way; only storage differs).
+// mode (whose line kernels compute in float).
 static int dfd(st_ctx *c, int dir, int asym, const double *F, double *dF, int iadd, double cadd) {
     return dev_dfd(c, dir, asym, F, dF, iadd, cadd);
 }
@@ -810,8 +809,8 @@ __device__ __forceinline__ void bc_cell(const BcArgs &b, int face, size_t q, dou
 
 // One outflow face in FP64.  Of the pressure's normal derivative only the last
 // row of each line is wanted, which the elimination gives without the back
-// substitution, and which the rows more than 48 before it do not reach (0.38
-// per row: 2e-20).  A block takes 32 lines: its threads form the pressure of
+// substitution, and which the finite rows more than 48 before it do not reach
+// (0.38 per row: 2e-20).  A block takes 32 lines: its threads form the pressure of
 // their last rows, one warp runs the elimination and the conditions.  Latency
 // of that serial elimination bounds it: 384^3, three faces at 0.10 ms a stage,
 // where the pressure as a field and its three whole derivatives (120 bytes per

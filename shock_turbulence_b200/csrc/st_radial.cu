@@ -19,7 +19,7 @@
 // the last few, so the factors of the first rows are one universal table, the
 // interior is at their fixed point (constants) and only rows n-4..n-1 come
 // from a small per-length tail table; a CTA keeps all of them in shared memory.
-// Measured, 512 problems of 128 to 4096 points, 4 steps: 18.5 ms; with scans of
+// Measured, 512 problems of 128 to 4096 points, 4 steps: 19.0 ms; with scans of
 // maps for every system, factors from global memory and the lanes' segments
 // 64 bytes apart in shared memory 31.4 ms.  What is left is instructions (3000
 // per point and stage, a tenth of the FP64 rate) and the barriers of 16 warps.
@@ -192,7 +192,7 @@ __device__ __forceinline__ M block_scan_excl(M m, M *sh) {
 // r'_i = r_i - l_i r'_{i-1}, backward x_i = (r'_i - u_i x_{i+1}) / pivot_i.
 // Each thread runs its rows with zero carries and publishes its end value and
 // the factor it passes a carry on with; the carry is then summed over the
-// threads whose rows reach (56 rows: 0.38^56 < 1e-23), one barrier per
+// threads whose rows reach (56 finite rows: 0.38^56 < 1e-23), one barrier per
 // direction.
 constexpr int kReach = 56;
 template <int SMAX>

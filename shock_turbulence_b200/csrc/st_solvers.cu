@@ -8,14 +8,15 @@
 //
 // One thread per line, in blocks of one warp so that few lines still spread
 // over all SMs, each step's arithmetic and order the reference's.  The chain
-// of a line is a division per row, some 100 cycles; what a thread must not do
-// besides is wait for its rows, so every sweep fetches the next U rows into
-// registers while it works on the U before them (at 16384 lines an SM has
-// about four warps: 32 rows of 32 bytes in flight per thread are what keeps
-// HBM busy).  Measured, 384 rows x 16384 lines, tridiagonal / periodic /
-// pentadiagonal / periodic: 325 / 528 / 415 / 588 us (199 / 296 / 288 / 438 us
-// at 2048 lines: the chain alone); row by row in blocks of 128 lines, with a
-// copy of every array and an allocation per call, the four took 22.9 ms.
+// of a line is a division and the products that depend on it per row; what a
+// thread must not do besides is wait for its rows, so every sweep fetches the
+// next U rows (4 to 8) into registers while it works on the U before them.
+// Measured, 384 rows x 16384 lines, tridiagonal / periodic / pentadiagonal /
+// periodic: 325 / 528 / 415 / 588 us.  At 2048 lines, 64 warps on the chip, it is
+// 199 / 296 / 288 / 438 us: 260 ns, about 490 cycles, per row step of the
+// first, which the chain's latency does not explain alone.  Row by row in
+// blocks of 128 lines, with a copy of every array and an allocation per call,
+// the four took 20.7 to 29.8 ms, as the allocations went.
 #include <cfloat>
 #include "st_internal.h"
 

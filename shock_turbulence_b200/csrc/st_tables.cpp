@@ -28,9 +28,15 @@ static const double kTiny = (double)FLT_MIN;   // tiny(1.0), src/tridiagonal.f90
 int choose_seg(int n) {
     if (n < 2 * 8 || n % 16 != 0 || n > kMaxSeg * kMaxRows) return 0;
     // Longer segments mean fewer halo rows and carries per row, shorter ones
-    // more threads and shorter chains.  Measured (256^3 and 64^3, filter /
-    // first / second derivative, us): 16 rows 102 / 76 / 131 and 22.8 / 23.6 /
-    // 26.8, 8 rows 192 / 87 / 136 and 23.1 / 22.9 / 25.2; they cross at 96.
+    // more threads and shorter chains.  Measured, z lines of n rows on n x 256 x
+    // 256 (calls, us: first / second with first derivative / filter):
+    //   n      64               80               96               128              256
+    //   16   30 / 46 / 35     31 / 57 / 42     36 / 61 / 48     43 / 77 / 56     64 / 114 / 95
+    //   8    30 / 46 / 37     39 / 56 / 56     38 / 60 / 53     44 / 73 / 70     75 / 115 / 184
+    // The filter and the first derivative gain from 16 rows at every length,
+    // the second derivative with the first along y loses up to 128 rows (128:
+    // 76 and 68).  16 rows would serve 80 too; the results' rounding goes with
+    // the segments.
     return n < 96 ? 8 : 16;
 }
 
@@ -536,7 +542,7 @@ int build_tables(st_ctx *c) {
         for (int kind = 0; kind < 2; kind++) {
             std::vector<double> M[5];
             filter_lhs(n, kind, M);
-                PenTab &t = c->pen[d][kind];
+            PenTab &t = c->pen[d][kind];
             upload_pen(c, t, M, nullptr, n, d, &err);
         }
     }
