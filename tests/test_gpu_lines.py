@@ -120,3 +120,35 @@ def test_unaligned_fields():
         getattr(s, f"Compact_Filter_{d}_asym")(G, G)
         assert torch.equal(a, G)
     s.close()
+
+
+@pytest.mark.parametrize("n", [16, 64, 112, 400, 512])
+@pytest.mark.parametrize("d", [0, 1, 2])
+def test_derivatives_in_place(d, n):
+    """An output that is the operand's array: the bits of separate arrays (each
+    tile is read before it is written, whatever the number of slots)."""
+    import torch
+    from shock_turbulence_b200 import Solver
+    grid = [32, 32, 32]
+    grid[d] = n
+    s = Solver(default_params(*grid))
+    F = torch.from_numpy(np.random.default_rng(n).standard_normal(s.shape)).cuda()
+    d1, d2 = getattr(s, f"DFD{DIRS[d]}_asym"), getattr(s, f"D2FD{DIRS[d]}2_sym")
+
+    def run(op, x, *rest):
+        torch.cuda.synchronize()
+        op(x, *rest)
+
+    for iadd in (0, 1):
+        own, same = F.clone(), F.clone()
+        run(d1, F, own, iadd, 0.7)
+        run(d1, same, same, iadd, 0.7)
+        assert torch.equal(own, same), iadd
+    a, a2, b2 = torch.zeros_like(F), torch.zeros_like(F), torch.zeros_like(F)
+    run(d2, F, a, a2, 1)
+    b = F.clone()
+    run(d2, b, b, b2, 1)
+    assert torch.equal(a, b) and torch.equal(a2, b2)
+    b, b1 = F.clone(), torch.zeros_like(F)
+    run(d2, b, b1, b, 1)
+    assert torch.equal(a, b1) and torch.equal(a2, b)
